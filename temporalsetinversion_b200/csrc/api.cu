@@ -249,7 +249,7 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
   }
   bm_words = std::max(1u, (mm_max + 15u) / 16u);
   fp.rcap = (rmax + 3u) & ~3u;
-  const size_t regfile = (size_t)kWarpsPerBlock * fp.rcap * 32u * sizeof(float2);
+  const size_t regfile = (size_t)kWarpsPerBlock * (fp.rcap * 32u * sizeof(float2) + kNarrowChunkBytes);
   // A wide cell keeps its working set in shared memory when it fits the
   // budget: by default what leaves the narrow path's blocks per SM as the
   // register files alone allow; larger working sets use the global scratch.
@@ -892,7 +892,7 @@ TSI_API tsi_status tsi_create(const tsi_device_opts *opts, tsi_ctx **out) {
   c->slice_len = 1024;
   // resident warps at the smallest register file
   {
-    const size_t smem_min = (size_t)kWarpsPerBlock * 4u * 32u * sizeof(float2);
+    const size_t smem_min = (size_t)kWarpsPerBlock * (4u * 32u * sizeof(float2) + kNarrowChunkBytes);
     CKC(refine_set_smem(smem_min));
     int bps = 0;
     CKC(refine_occupancy(kBlock, smem_min, &bps));

@@ -26,6 +26,11 @@
 #define TSI_PRUNE_MAX_REGS 64u  // pruning tracks liveness in one 64-bit mask
 #define TSI_PRUNE_MIN_LEN 8u    // shorter tapes are not worth pruning
 
+// What a narrow warp keeps in shared memory after its register file: a row
+// that is never read and 32 decoded tape instructions of 16 bytes
+// (narrow_interp.cuh).
+constexpr unsigned kNarrowChunkBytes = 256u + 32u * 16u;
+
 enum tsi_scene_flags {
   SF_POINTSAMPLE = 1u << 0,
   SF_FASTENABLED = 1u << 1,

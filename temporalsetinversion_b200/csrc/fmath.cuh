@@ -41,8 +41,39 @@ TSI_DEV float fm_nan() { return __int_as_float(0x7fc00000); }
 TSI_DEV float fm_min(float a, float b) { return fminf(a, b); }
 TSI_DEV float fm_max(float a, float b) { return fmaxf(a, b); }
 
+// Two f32 sums, or fused products and sums, in one instruction (sm_100's
+// packed f32x2 forms): each half rounds like the scalar operation.
+struct F2 {
+  unsigned long long v;
+};
+TSI_DEV F2 f2_pack(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+TSI_DEV void f2_unpack(F2 p, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+TSI_DEV F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+// Products half by half: ptxas contracts a packed product and sum into one
+// fused operation whatever their .rn says (measured: another last bit in one
+// result of sixty), a scalar product and a packed sum it leaves alone.
+TSI_DEV F2 f2_mul(F2 a, F2 b) {
+  float a0, a1, b0, b1;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a.v));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(b.v));
+  return f2_pack(__fmul_rn(a0, b0), __fmul_rn(a1, b1));
+}
+TSI_DEV F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+TSI_DEV F2 f2_dup(float a) { return f2_pack(a, a); }
+
 TSI_DEV float fm_sin(float x) {
-  if (!(fabsf(x) <= 3.0e38f)) return fm_sub(x, x);
   const float two_over_pi = 0.6366197466850281f;
   const float p1 = 1.5703125f, p2 = 0.0004838705062866211f, p3 = -4.371138828673793e-08f;
   float k = rintf(fm_mul(x, two_over_pi));
@@ -65,16 +96,51 @@ TSI_DEV float fm_sin(float x) {
   pc = fm_add(0.0416666679084301f, fm_mul(r2, pc));
   pc = fm_add(-0.5f, fm_mul(r2, pc));
   float c = fm_add(1.0f, fm_mul(r2, pc));
-  switch (q) {
-    case 0: return s;
-    case 1: return c;
-    case 2: return -s;
-    default: return -c;
-  }
+  // quadrants 0..3: s, c, -s, -c (selects: a four-way jump costs more than
+  // both polynomials)
+  const float v = (q & 1) ? c : s;
+  const float y = (q & 2) ? -v : v;
+  return fabsf(x) <= 3.0e38f ? y : fm_sub(x, x);  // infinities and NaN: NaN
+}
+
+// fm_sin of two arguments, operation for operation, two at a time.
+TSI_DEV void fm_sin2(float x0, float x1, float &y0, float &y1) {
+  const float p1 = 1.5703125f, p2 = 0.0004838705062866211f, p3 = -4.371138828673793e-08f;
+  const F2 x = f2_pack(x0, x1);
+  float k0, k1;
+  f2_unpack(f2_mul(x, f2_dup(0.6366197466850281f)), k0, k1);
+  k0 = rintf(k0);
+  k1 = rintf(k1);
+  const F2 k = f2_pack(k0, k1);
+  F2 r = f2_add(x, f2_mul(k, f2_dup(-p1)));
+  r = f2_add(r, f2_mul(k, f2_dup(-p2)));
+  r = f2_add(r, f2_mul(k, f2_dup(-p3)));
+  const int q0 = (int)fm_sub(k0, fm_mul(4.0f, floorf(fm_mul(k0, 0.25f))));
+  const int q1 = (int)fm_sub(k1, fm_mul(4.0f, floorf(fm_mul(k1, 0.25f))));
+  const F2 r2 = f2_mul(r, r);
+  F2 ps = f2_dup(-2.5052107943679403e-08f);
+  ps = f2_add(f2_dup(2.7557318844628753e-06f), f2_mul(r2, ps));
+  ps = f2_add(f2_dup(-0.00019841270113829523f), f2_mul(r2, ps));
+  ps = f2_add(f2_dup(0.008333333767950535f), f2_mul(r2, ps));
+  ps = f2_add(f2_dup(-0.1666666716337204f), f2_mul(r2, ps));
+  const F2 s = f2_add(r, f2_mul(r, f2_mul(r2, ps)));
+  F2 pc = f2_dup(2.0876755879584152e-09f);
+  pc = f2_add(f2_dup(-2.755731998149713e-07f), f2_mul(r2, pc));
+  pc = f2_add(f2_dup(2.4801587642286904e-05f), f2_mul(r2, pc));
+  pc = f2_add(f2_dup(-0.0013888889225199819f), f2_mul(r2, pc));
+  pc = f2_add(f2_dup(0.0416666679084301f), f2_mul(r2, pc));
+  pc = f2_add(f2_dup(-0.5f), f2_mul(r2, pc));
+  const F2 c = f2_add(f2_dup(1.0f), f2_mul(r2, pc));
+  float s0, s1, c0, c1;
+  f2_unpack(s, s0, s1);
+  f2_unpack(c, c0, c1);
+  const float v0 = (q0 & 1) ? c0 : s0, v1 = (q1 & 1) ? c1 : s1;
+  const float w0 = (q0 & 2) ? -v0 : v0, w1 = (q1 & 2) ? -v1 : v1;
+  y0 = fabsf(x0) <= 3.0e38f ? w0 : fm_sub(x0, x0);
+  y1 = fabsf(x1) <= 3.0e38f ? w1 : fm_sub(x1, x1);
 }
 
 TSI_DEV float fm_cos(float x) {
-  if (!(fabsf(x) <= 3.0e38f)) return fm_sub(x, x);
   const float two_over_pi = 0.6366197466850281f;
   const float p1 = 1.5703125f, p2 = 0.0004838705062866211f, p3 = -4.371138828673793e-08f;
   float k = rintf(fm_mul(x, two_over_pi));
@@ -97,12 +163,10 @@ TSI_DEV float fm_cos(float x) {
   pc = fm_add(0.0416666679084301f, fm_mul(r2, pc));
   pc = fm_add(-0.5f, fm_mul(r2, pc));
   float c = fm_add(1.0f, fm_mul(r2, pc));
-  switch (q) {
-    case 0: return c;
-    case 1: return -s;
-    case 2: return -c;
-    default: return s;
-  }
+  // quadrants 0..3: c, -s, -c, s
+  const float v = (q & 1) ? s : c;
+  const float y = (q == 1 || q == 2) ? -v : v;
+  return fabsf(x) <= 3.0e38f ? y : fm_sub(x, x);  // infinities and NaN: NaN
 }
 
 TSI_DEV float fm_pow2i(int e) { return __int_as_float((e + 127) << 23); }

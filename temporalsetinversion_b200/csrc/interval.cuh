@@ -104,8 +104,8 @@ struct IA {
   }
   static TSI_DEV Iv mul_f(Iv a, float b) {
     if (!D) {
-      if (b >= 0.0f) return Iv{__fmul_rn(a.lo, b), __fmul_rn(a.hi, b)};
-      return Iv{__fmul_rn(a.hi, b), __fmul_rn(a.lo, b)};
+      const float x = __fmul_rn(a.lo, b), y = __fmul_rn(a.hi, b);
+      return b >= 0.0f ? Iv{x, y} : Iv{y, x};
     }
     return mul(a, iv(b));
   }
@@ -135,15 +135,16 @@ struct IA {
   static TSI_DEV Iv neg(Iv a) { return Iv{-a.hi, -a.lo}; }
   static TSI_DEV Iv min_(Iv a, Iv b) { return Iv{fm_min(a.lo, b.lo), fm_min(a.hi, b.hi)}; }
   static TSI_DEV Iv max_(Iv a, Iv b) { return Iv{fm_max(a.lo, b.lo), fm_max(a.hi, b.hi)}; }
+  // (selects: the compiler makes a divergent branch of every early return)
   static TSI_DEV Iv abs_(Iv a) {
-    if (contains_zero(a)) return Iv{0.0f, fm_max(-a.lo, a.hi)};
-    if (a.hi < 0.0f) return Iv{-a.hi, -a.lo};
-    return a;
+    const bool z = contains_zero(a), n = a.hi < 0.0f;
+    const float lo = n ? -a.hi : a.lo, hi = n ? -a.lo : a.hi;
+    return Iv{z ? 0.0f : lo, z ? fm_max(-a.lo, a.hi) : hi};
   }
   static TSI_DEV Iv abs_rr(Iv a) {
-    if (contains_zero(a)) return Iv{-1.0f, 1.0f};
-    if (a.hi < 0.0f) return iv(-1.0f);
-    return iv(1.0f);
+    const bool z = contains_zero(a);
+    const float s = a.hi < 0.0f ? -1.0f : 1.0f;
+    return Iv{z ? -1.0f : s, z ? 1.0f : s};
   }
   static TSI_DEV Iv empty() { return Iv{fm_inf(), -fm_inf()}; }
   static TSI_DEV Iv cap(Iv a, Iv b) {
@@ -341,28 +342,48 @@ struct IA {
     o0 = div(iv(1.0f), r);
     o1 = neg(div(l, sqr(r)));
   }
-  static TSI_DEV float mymod(float x, float y) { return __fsub_rn(x, __fmul_rn(y, floorf(__fdiv_rn(x, y)))); }
-  // SIN_I, compute.wgsl:2926-2957 (quadrant method)
+  // floor(x / (pi/2 as f32)) for |x| < 1e7, as floor(__fdiv_rn(x, kHALFPI))
+  // gives it: the quotient by the reciprocal, corrected once by its exact
+  // residual, equals the correctly rounded one for every f32 from 0.5 to 2^25
+  // (checked exhaustively); below 0.5 the floor is that of x itself.
+  static TSI_DEV float quadrant(float x) {
+    const float rc = 0.6366197466850281f;  // 1 / kHALFPI rounded to f32
+    const float q = __fmul_rn(x, rc);
+    const float q2 = __fmaf_rn(__fmaf_rn(-q, kHALFPI, x), rc, q);
+    return floorf(fabsf(x) < 0.5f ? x : q2);
+  }
+  static TSI_DEV float mod4(float x) { return __fsub_rn(x, __fmul_rn(4.0f, floorf(__fmul_rn(x, 0.25f)))); }
+  // SIN_I, compute.wgsl:2926-2957 (quadrant method).  Both sines are taken
+  // side by side and the quadrant cases are selects: 1000 cycles an
+  // instruction as calls, divisions and branches, a quarter of that so.
   static TSI_DEV Iv sin_(Iv a) {
     const Iv whole = Iv{-1.0f, 1.0f};
     if (!D) {
-      if (__fsub_rn(a.hi, a.lo) > kTWOPI) return whole;
-      float lo_q = floorf(__fdiv_rn(a.lo, kHALFPI));
-      float hi_q = floorf(__fdiv_rn(a.hi, kHALFPI));
-      if (__fsub_rn(hi_q, lo_q) > 4.0f) return whole;
-      lo_q = mymod(lo_q, 4.0f);
-      hi_q = mymod(hi_q, 4.0f);
-      if (lo_q == hi_q) {
-        if (__fsub_rn(a.hi, a.lo) > kPI) return whole;
-        return unordered(fm_sin(a.lo), fm_sin(a.hi));
-      } else if ((lo_q == 3.0f && hi_q == 0.0f) || (lo_q == 1.0f && hi_q == 2.0f)) {
-        return unordered(fm_sin(a.lo), fm_sin(a.hi));
-      } else if ((lo_q == 0.0f || lo_q == 3.0f) && (hi_q == 1.0f || hi_q == 2.0f)) {
-        return Iv{fm_min(fm_sin(a.lo), fm_sin(a.hi)), 1.0f};
-      } else if ((lo_q == 1.0f || lo_q == 2.0f) && (hi_q == 3.0f || hi_q == 0.0f)) {
-        return Iv{-1.0f, fm_max(fm_sin(a.lo), fm_sin(a.hi))};
+      float lo_q, hi_q;
+      if (fabsf(a.lo) < 1e7f && fabsf(a.hi) < 1e7f) {
+        lo_q = quadrant(a.lo);
+        hi_q = quadrant(a.hi);
+      } else {
+        lo_q = floorf(__fdiv_rn(a.lo, kHALFPI));
+        hi_q = floorf(__fdiv_rn(a.hi, kHALFPI));
       }
-      return whole;
+      float slo, shi;
+      fm_sin2(a.lo, a.hi, slo, shi);
+      const float width = __fsub_rn(a.hi, a.lo);
+      const bool wide_iv = width > kTWOPI || __fsub_rn(hi_q, lo_q) > 4.0f;
+      lo_q = mod4(lo_q);
+      hi_q = mod4(hi_q);
+      const float mn = fm_min(slo, shi), mx = fm_max(slo, shi);
+      const bool same = lo_q == hi_q;
+      const bool mono = (lo_q == 3.0f && hi_q == 0.0f) || (lo_q == 1.0f && hi_q == 2.0f);
+      const bool top = (lo_q == 0.0f || lo_q == 3.0f) && (hi_q == 1.0f || hi_q == 2.0f);
+      const bool bot = (lo_q == 1.0f || lo_q == 2.0f) && (hi_q == 3.0f || hi_q == 0.0f);
+      Iv v = whole;
+      if (bot) v = Iv{-1.0f, mx};
+      if (top) v = Iv{mn, 1.0f};
+      if (mono || same) v = Iv{mn, mx};
+      if (wide_iv || (same && width > kPI)) v = whole;
+      return v;
     }
     // directed: quadrants of a slightly widened interval decide which
     // extrema (+-1 at pi/2 + k pi) the interval may contain

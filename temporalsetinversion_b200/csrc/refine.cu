@@ -35,6 +35,7 @@
 
 #include "device_types.h"
 #include "interp.cuh"
+#include "narrow_interp.cuh"
 #include "wide_interp.cuh"
 #include "interval.cuh"
 #include "opcost.h"
@@ -58,76 +59,81 @@ extern __shared__ __align__(16) unsigned char tsi_dyn_smem[];
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Backward liveness scan of one sibling group, run by the whole warp with the
-// group leaders (lane 8g, `active`) doing the work: decided min/max become
-// copies/constants, dead instructions vanish.  The kept instructions are
-// written in reverse order to `tmp`; returns their count.  The tape and the
-// branch ballots arrive 32 per coalesced load.
-__device__ uint32_t prune_scan(const uint2 *__restrict__ code, uint32_t len, uint32_t n_minmax, uint32_t out_reg,
-                               const uint2 *dg, uint32_t g, uint32_t E, uint2 *tmp, bool active, uint32_t lane,
-                               uint32_t &mm_kept, uint32_t &fwd_cost, uint32_t &rev_cost) {
-  unsigned long long live = 1ull << out_reg;
-  uint32_t cnt = 0;
-  mm_kept = 0;
-  fwd_cost = 0;
-  rev_cost = 0;
+// Backward liveness scan of one sibling group (g, enqueued siblings E) by the
+// whole warp: decided min/max become copies/constants, dead instructions
+// vanish.  The kept instructions are written in reverse order to `tmp`;
+// returns their count.  A chunk of 32 instructions is decoded one per lane
+// (decision, operand and destination masks); what is left of the serial scan
+// is three logic operations an instruction on the 64-bit mask of live
+// registers, on masks read back by broadcast loads.  (One lane decoding and
+// scanning took 300 cycles an instruction, this takes 35.)
+__device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, uint32_t len_, uint32_t n_minmax_,
+                                                uint32_t out_reg, const uint2 *dg, uint32_t g, uint32_t E, uint2 *tmp,
+                                                const NarrowRows &R, uint32_t lane, uint32_t &mm_kept, uint32_t &fwd_cost,
+                                                uint32_t &rev_cost) {
+  const uint32_t len = uniform_u32(len_);
+  uint32_t live_lo = out_reg < 32u ? 1u << out_reg : 0u, live_hi = out_reg >= 32u ? 1u << (out_reg - 32u) : 0u;
+  uint32_t cnt = 0, kept_mm = 0, fc = 0, rc = 0;
   const int nch = (int)((len + 31u) / 32u);
-  uint2 cur = load_chunk(code, len, nch - 1, lane), nxt = load_chunk(code, len, nch - 2, lane);
-  // ballots: chunk km holds min/max ordinals [32 km, 32 km + 32)
-  int m = (int)n_minmax;
-  int km = (m - 1) / 32;
-  uint2 dcur = load_chunk(dg, n_minmax, m > 0 ? km : -1, lane);
+  int m = (int)uniform_u32(n_minmax_);  // min/max ordinals from the end
+  uint2 nxt = load_chunk(code, len, nch - 1, lane);
   for (int k = nch - 1; k >= 0; --k) {
-    const int c0 = 32 * k;
-    for (int j = min(32, (int)len - c0) - 1; j >= 0; --j) {
-      const uint2 w = chunk_word(cur, (uint32_t)j);
-      const uint32_t h = TSI_W0_H(w.x);
-      const uint32_t d = TSI_W0_DST(w.x), a = TSI_W0_A(w.x), b = w.y & 255u;
-      const bool mmx = TSI_H_IS_MINMAX(h);
-      uint2 dd = make_uint2(0u, 0u);
-      if (mmx) {  // uniform across the warp
-        --m;
-        if (m < 32 * km) {
-          km = m / 32;
-          dcur = load_chunk(dg, n_minmax, km, lane);
-        }
-        dd = chunk_word(dcur, (uint32_t)(m - 32 * km));
-      }
-      if (!active || !((live >> d) & 1ull)) continue;
-      live &= ~(1ull << d);
-      uint2 out = w;
-      uint32_t hk = h;
-      if (mmx) {
-        const uint32_t ga = (dd.x >> (g * 8u)) & 0xffu, gb = (dd.y >> (g * 8u)) & 0xffu;
-        if ((ga & E) == E) {
-          out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, d, a), 0u);
+    const uint2 w = nxt;
+    nxt = load_chunk(code, len, k - 1, lane);
+    const bool valid = 32u * (uint32_t)k + lane < len;
+    const uint32_t h = TSI_W0_H(w.x), d = TSI_W0_DST(w.x), a = TSI_W0_A(w.x), b = w.y & 255u;
+    const bool mmx = valid && TSI_H_IS_MINMAX(h);
+    const uint32_t mmb = __ballot_sync(FULL_MASK, mmx);
+    m -= __popc(mmb);
+    uint2 out = w;
+    uint32_t hk = h;
+    bool use_a = h != H_CONST, use_b = TSI_H_IS_II(h);
+    if (mmx) {
+      const uint2 dd = dg[m + __popc(mmb & ((1u << lane) - 1u))];
+      const uint32_t ga = (dd.x >> (g * 8u)) & 0xffu, gb = (dd.y >> (g * 8u)) & 0xffu;
+      if ((ga & E) == E) {
+        out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, d, a) | (w.x & TSI_W0_ODD), 0u);
+        hk = H_COPY;
+        use_b = false;
+      } else if ((gb & E) == E) {
+        use_a = false;
+        if (TSI_H_IS_II(h)) {
+          out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, d, b) | (w.x & TSI_W0_ODD), 0u);
           hk = H_COPY;
-          live |= 1ull << a;
-        } else if ((gb & E) == E) {
-          if (TSI_H_IS_II(h)) {
-            out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, d, b), 0u);
-            hk = H_COPY;
-            live |= 1ull << b;
-          } else {
-            out = make_uint2(TSI_W0(H_CONST, 0u, 0u, d, 0u), w.y);
-            hk = H_CONST;
-          }
         } else {
-          live |= 1ull << a;
-          if (TSI_H_IS_II(h)) live |= 1ull << b;
-          ++mm_kept;
+          out = make_uint2(TSI_W0(H_CONST, 0u, 0u, d, 0u), w.y);
+          hk = H_CONST;
         }
-      } else {
-        if (h != H_CONST) live |= 1ull << a;
-        if (TSI_H_IS_II(h)) live |= 1ull << b;
       }
-      fwd_cost += c_cost_fwd[hk] + TSI_FIX_COST;
-      rev_cost += c_cost_rr[hk] + TSI_REV_OPERAND_COST * TSI_H_NREG(hk);
-      tmp[cnt++] = out;
     }
-    cur = nxt;
-    nxt = load_chunk(code, len, k - 2, lane);
+    // registers written and read, as 64-bit masks
+    unsigned long long def = valid ? 1ull << d : 0ull, src = 0ull;
+    if (use_a) src |= 1ull << a;
+    if (use_b) src |= 1ull << b;
+    __syncwarp();
+    prog_st(R, lane, make_uint4((uint32_t)def, (uint32_t)(def >> 32), (uint32_t)src, (uint32_t)(src >> 32)));
+    __syncwarp();
+    uint32_t keep = 0;
+#pragma unroll 8
+    for (int j = 31; j >= 0; --j) {
+      const uint4 q = prog_ld(R, (uint32_t)j);
+      const bool on = ((live_lo & q.x) | (live_hi & q.y)) != 0u;
+      live_lo = (live_lo & ~q.x) | (on ? q.z : 0u);
+      live_hi = (live_hi & ~q.y) | (on ? q.w : 0u);
+      keep |= on ? 1u << j : 0u;
+    }
+    if ((keep >> lane) & 1u) {
+      tmp[cnt + __popc(keep & ~((2u << lane) - 1u))] = out;
+      kept_mm += TSI_H_IS_MINMAX(hk) ? 1u : 0u;
+      fc += c_cost_fwd[hk] + TSI_FIX_COST;
+      rc += c_cost_rr[hk] + TSI_REV_OPERAND_COST * TSI_H_NREG(hk);
+    }
+    cnt += __popc(keep);
   }
+  mm_kept = __reduce_add_sync(FULL_MASK, kept_mm);
+  fwd_cost = __reduce_add_sync(FULL_MASK, fc);
+  rev_cost = __reduce_add_sync(FULL_MASK, rc);
+  __syncwarp();  // tmp is read by other lanes
   return cnt;
 }
 
@@ -352,12 +358,14 @@ __device__ __forceinline__ bool item_scratch(const LaunchParams &P, uint32_t ste
 
 template <bool D>
 __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem &it, uint32_t step,
-                                          uint32_t rf_off, float4 *slice_log, uint2 *slice_dec,
+                                          uint32_t rcap, float4 *slice_log, uint2 *slice_dec,
                                           unsigned long long *ws) {
   const StepIdx si = step_idx(step);
-  float2 *rf = reinterpret_cast<float2 *>(tsi_dyn_smem) + rf_off;  // this warp's register file
   using A = IA<D>;
   const uint32_t lane = threadIdx.x & 31u;
+  // this warp's register file and chunk buffer
+  const NarrowRows R = narrow_rows(tsi_dyn_smem + (threadIdx.x >> 5) * (rcap * 256u + kNarrowChunkBytes), rcap, lane,
+                                   it.n);
   const uint32_t g = lane >> 3, k = lane & 7u;
   const SceneLaunch &S = P.scenes[it.scene];
   const VoxelPoolDev &pool = S.pool;
@@ -463,13 +471,16 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
         uint2 *dgs = nullptr;
         if (!item_scratch(P, step, it.scene, TR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
         lg = lgs;
-        dg = want_prune ? dgs : nullptr;
+        dg = dgs;
       }
       const long long q0 = clock64();
-      field = forward_pass<D>(TR.code, TR.len, TR.out_reg, rf, lane, cx, cy, cz, targ, any_deriv ? lg : nullptr, dg);
+      uint32_t nlog = 0;
+      float4 *opl = any_deriv ? lg : nullptr;
+      field = narrow_forward<D>(TR.code, TR.len, TR.out_reg, R, lane, cx, cy, cz, targ, opl, dg, nlog);
       const long long q1 = clock64();
       bool bad = false;
-      if (any_deriv) reverse_pass<D>(TR.code, TR.len, TR.nregs, TR.out_reg, rf, lane, lg, take_deriv, sens, bad);
+      if (any_deriv)
+        narrow_reverse<D>(TR.code, TR.len, TR.nregs, TR.out_reg, R, lane, opl, nlog, take_deriv, sens, bad);
       if (lane == 0 && attempt == 0) {
         ws[ST_CYC_N_FWD] += (unsigned long long)(q1 - q0);
         ws[ST_N_FWD_INSTR] += TR.len;
@@ -629,7 +640,8 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
         lg = lgs;
         dg = dgs;
         const Iv tw = enq ? Iv{nl, nh} : targ;
-        (void)forward_pass<D>(PR.code, PR.len, PR.out_reg, rf, lane, cx, cy, cz, tw, nullptr, dg);
+        uint32_t nlog = 0;
+        (void)narrow_forward<D>(PR.code, PR.len, PR.out_reg, R, lane, cx, cy, cz, tw, nullptr, dg, nlog);
         if (lane == 0) ws[ST_FP32] += (unsigned long long)PR.fwd_cost * __popc(em);
       }
     }
@@ -652,21 +664,30 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
         (want_prune && !handed && lg != nullptr) ? reinterpret_cast<uint2 *>(lg) + (size_t)g * PR.len : nullptr;
     const uint32_t actm = __ballot_sync(FULL_MASK, k == 0 && E != 0 && tmp != nullptr);
     if (actm) {
-      // every pruning group scans the same tape; lanes of other groups (a
-      // group handed to the wide path holds another record) follow the
-      // scan on that tape, so the warp's shuffles stay uniform
-      const int src = __ffs(actm) - 1;
-      const uint2 *pcode = reinterpret_cast<const uint2 *>(
-          __shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(PR.code), src));
-      const uint32_t plen = __shfl_sync(FULL_MASK, PR.len, src);
-      const uint32_t pmm = __shfl_sync(FULL_MASK, PR.n_minmax, src);
-      const uint32_t pout = __shfl_sync(FULL_MASK, PR.out_reg, src);
-      const bool act = (actm >> lane) & 1u;
       const long long q0 = clock64();
-      cnt = prune_scan(pcode, plen, pmm, pout, dg, g, E, tmp, act, lane, mmk, fcost, rcost);
+      __syncwarp();  // the ballots (lane 0) and the log's last readers
+      // every pruning group scans the same tape, one group after another by
+      // the whole warp (a group handed to the wide path holds another record)
+      for (uint32_t rest = actm; rest; rest &= rest - 1u) {
+        const int src = __ffs(rest) - 1;
+        const uint2 *pcode = reinterpret_cast<const uint2 *>(
+            __shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(PR.code), src));
+        const uint32_t plen = __shfl_sync(FULL_MASK, PR.len, src);
+        const uint32_t pmm = __shfl_sync(FULL_MASK, PR.n_minmax, src);
+        const uint32_t pout = __shfl_sync(FULL_MASK, PR.out_reg, src);
+        const uint32_t pE = __shfl_sync(FULL_MASK, E, src);
+        uint2 *ptmp = reinterpret_cast<uint2 *>(__shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(tmp), src));
+        uint32_t mk, fc, rc;
+        const uint32_t n = prune_group(pcode, plen, pmm, pout, dg, (uint32_t)src >> 3, pE, ptmp, R, lane, mk, fc, rc);
+        if ((int)lane == src) {
+          cnt = n;
+          mmk = mk;
+          fcost = fc;
+          rcost = rc;
+          pruned = n < PR.len;
+        }
+      }
       if (lane == 0) ws[ST_CYC_N_PRUNE] += (unsigned long long)(clock64() - q0);
-      pruned = act && cnt < PR.len;
-      if (!act) cnt = 0;
     }
     // reserve arena space and a record (lane 8g), then copy with the group
     unsigned long long off = 0;
@@ -679,8 +700,18 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
     cnt = __shfl_sync(FULL_MASK, cnt, gl0);
     off = __shfl_sync(FULL_MASK, off, gl0);
     ri = __shfl_sync(FULL_MASK, ri, gl0);
+    {  // the pruned tapes in program order, one group after another by the whole warp
+      uint32_t cm = __ballot_sync(FULL_MASK, k == 0 && ri != TSI_NONE);
+      for (; cm; cm &= cm - 1u) {
+        const int src = __ffs(cm) - 1;
+        const uint32_t n = __shfl_sync(FULL_MASK, cnt, src);
+        uint2 *dst = P.code_arena + __shfl_sync(FULL_MASK, off, src);
+        const uint2 *ptmp = reinterpret_cast<const uint2 *>(
+            __shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(tmp), src));
+        for (uint32_t j = lane; j < n; j += 32u) dst[j] = ptmp[n - 1u - j];
+      }
+    }
     if (ri != TSI_NONE) {
-      for (uint32_t j = k; j < cnt; j += 8u) P.code_arena[off + j] = tmp[cnt - 1u - j];
       if (k == 0) {
         TapeRec nr;
         nr.code = P.code_arena + off;
@@ -1001,11 +1032,11 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
             const uint32_t d = (cb[mm >> 4] >> (2u * (mm & 15u))) & 3u;
             const uint32_t dd = TSI_W0_DST(w.x);
             if (d & 1u) {
-              out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)), 0u);
+              out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD), 0u);
               hk = H_COPY;
             } else if (d & 2u) {
               if (TSI_H_IS_II(h)) {
-                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u), 0u);
+                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD), 0u);
                 hk = H_COPY;
               } else {
                 out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u), w.y);
@@ -1409,7 +1440,6 @@ __global__ void __launch_bounds__(256) refine_kernel(const __grid_constant__ Lau
   // touches them; the next step fills them)
   if (blockIdx.x == 0 && threadIdx.x == 0) clear_step(P, (step + 2u) & TSI_STEP_MASK);
   const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + wib;
-  const uint32_t rf_off = wib * rcap * 32u;  // this warp's register file in tsi_dyn_smem (float2 units)
   float4 *slice_log = P.log_slices + (size_t)gw * P.slice_len * 32u;
   uint2 *slice_dec = P.dec_slices + (size_t)gw * P.slice_len;
   unsigned long long *ws = s_stats[wib];
@@ -1469,8 +1499,8 @@ __global__ void __launch_bounds__(256) refine_kernel(const __grid_constant__ Lau
       const WorkItem &it = items[idx];
       take(it.scene);
       const long long c0 = clock64();
-      if (P.scenes[it.scene].flags & SF_DIRECTED) process_item<true>(P, it, step, rf_off, slice_log, slice_dec, ws);
-      else process_item<false>(P, it, step, rf_off, slice_log, slice_dec, ws);
+      if (P.scenes[it.scene].flags & SF_DIRECTED) process_item<true>(P, it, step, rcap, slice_log, slice_dec, ws);
+      else process_item<false>(P, it, step, rcap, slice_log, slice_dec, ws);
       __syncwarp();
       if (lane == 0) {
         const unsigned long long c = (unsigned long long)(clock64() - c0);

@@ -81,11 +81,14 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
   out.count = n;
   // last use of every slot; the field (slot n-1) stays live to the end
   std::vector<int64_t> last_use(n, -1);
+  std::vector<uint32_t> users(n, 0);  // instructions that read the slot
   for (uint32_t j = 4; j < n; ++j) {
     const IrInstr &in = ins[j];
     uint32_t top = op_top_of(in);
     if (top == 0 || top == 1) last_use[in.larg.reg] = j;
     if (top == 0 || top == 2) last_use[in.rarg.reg] = j;
+    if (top == 0 || top == 1) ++users[in.larg.reg];
+    if (top == 2 || (top == 0 && in.rarg.reg != in.larg.reg)) ++users[in.rarg.reg];
   }
   last_use[n - 1] = int64_t(n);
 
@@ -141,7 +144,8 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
     reg[j] = d;
     used[d] = (last_use[j] >= 0) ? 1 : 0;  // a never-read value frees at once
     if (d > maxreg) maxreg = d;
-    out.code.push_back(TSI_W0(h, fa, fb, d, ra));
+    const bool odd = (fa && users[a_slot] > 1u) || (fb && users[b_slot] > 1u);
+    out.code.push_back(TSI_W0(h, fa, fb, d, ra) | (odd ? TSI_W0_ODD : 0u));
     out.code.push_back(w1);
     if (TSI_H_IS_MINMAX(h)) out.n_minmax++;
     out.fwd_cost += fwd_cost[h] + TSI_FIX_COST;

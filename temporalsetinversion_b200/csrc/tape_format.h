@@ -8,7 +8,9 @@
 //   w0  bits  0..5   handler (op x operand kind, table below)
 //       bit   6      operand A is single-use  (ir.rs uses.len() == 1)
 //       bit   7      operand B is single-use
-//       bits  8..15  reserved
+//       bit   8      a flagged operand has other users after all (an uploaded
+//                    tape's use counts may be wrong): no shortcut applies
+//       bits  9..15  reserved
 //       bits 16..23  destination register
 //       bits 24..31  register A (larg, or rarg for the literal-left kinds)
 //   w1  register B in bits 0..7 (two-register handlers) or the f32 literal
@@ -37,6 +39,7 @@ enum tsi_handler {
 
 #define TSI_W0(h, fa, fb, dst, a) \
   ((uint32_t)(h) | ((uint32_t)(fa) << 6) | ((uint32_t)(fb) << 7) | ((uint32_t)(dst) << 16) | ((uint32_t)(a) << 24))
+#define TSI_W0_ODD (1u << 8)
 #define TSI_W0_H(w) ((w) & 63u)
 #define TSI_W0_FA(w) (((w) >> 6) & 1u)
 #define TSI_W0_FB(w) (((w) >> 7) & 1u)
