@@ -131,6 +131,7 @@ LaunchParams make_params(tsi_ctx *c, uint32_t n_scenes, size_t dyn_smem, bool st
   P.slice_len = c->slice_len;
   P.log_overflow = c->d_log_overflow;
   P.log_overflow_used = c->d_log_used;
+  P.long_count = c->d_long_count;
   P.log_overflow_cap = c->log_overflow_cap;
   P.error = c->d_error;
   P.stats = c->d_stats;
@@ -925,6 +926,7 @@ TSI_API tsi_status tsi_create(const tsi_device_opts *opts, tsi_ctx **out) {
   CKC(dalloc(&c->d_dec, (size_t)c->max_warps * c->slice_len));
   CKC(dalloc(&c->d_log_overflow, c->log_overflow_cap));
   CKC(dalloc(&c->d_log_used, TSI_STEP_RING));
+  CKC(dalloc(&c->d_long_count, TSI_STEP_RING));
   CKC(dalloc(&c->d_error, c->max_scenes));
   CKC(dalloc(&c->d_error_sticky, 1));
   CKC(cudaMemset(c->d_error_sticky, 0, sizeof(uint32_t)));
@@ -989,6 +991,7 @@ TSI_API void tsi_destroy(tsi_ctx *c) {
   cudaFree(c->d_dec);
   cudaFree(c->d_log_overflow);
   cudaFree(c->d_log_used);
+  cudaFree(c->d_long_count);
   cudaFree(c->d_error);
   cudaFree(c->d_error_sticky);
   cudaFree(c->d_stats);

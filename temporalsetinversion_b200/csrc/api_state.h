@@ -115,6 +115,7 @@ struct tsi_ctx {
   uint32_t max_warps = 0;
   float4 *d_log_overflow = nullptr;
   unsigned long long *d_log_used = nullptr;
+  uint32_t *d_long_count = nullptr;  // [TSI_STEP_RING]
   uint64_t log_overflow_cap = 0;
   uint32_t *d_error = nullptr;         // [max_scenes] error bits per scene slot
   uint32_t *d_error_sticky = nullptr;  // error words of asynchronous inversions since the last wait

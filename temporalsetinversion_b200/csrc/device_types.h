@@ -228,6 +228,7 @@ struct LaunchParams {
   // next step starts, so every step fills the arena from its start
   unsigned long long *log_overflow_used;
   unsigned long long log_overflow_cap;
+  uint32_t *long_count;             // [TSI_STEP_RING]: items of tapes at least the wide threshold long
   uint32_t *error;                  // [n_scenes]: error bits of each scene
   unsigned long long *stats;        // [n_scenes][ST_COUNT]: counters of each scene
   unsigned long long *level_stats;  // [TSI_STEP_RING][ST_COUNT], per refine launch, or null

@@ -154,10 +154,25 @@ __device__ uint32_t alloc_brick(const SceneLaunch &S, uint32_t *error) {
   return b * 8u;
 }
 
-// The wide threshold for children at `level`: deep levels hold many cells,
-// where the narrow path's throughput beats the wide path's latency.
+// The wide threshold for children at `level`: deep levels may have one of
+// their own.
 __device__ __forceinline__ uint32_t wide_min_len(const WideDev &W, uint32_t level) {
   return level >= W.deep_level ? W.deep_min_len : W.min_len;
+}
+// The tape length from which children of this step's groups take the wide
+// path: the threshold (where a block per cell and a warp per item take
+// equally long) times the waves of blocks that this step's long items need
+// for their eight cells each; the next step seldom has fewer.  A step of
+// long items finishes a wide item of 8 cells in 8/296 of a cell's time on a
+// B200's 296 blocks, but 2368 narrow items at once: by length alone, levels
+// of thousands of long items ran one block per cell.  Rotating swept scene
+// (64 primitives, localsubdiv 9) 8.0 to 2.7 ms an inversion, 1024 primitives
+// (localsubdiv 9) 3.7 to 3.3 ms, 256 primitives unchanged; half and twice
+// the multiplier measured 3.1 and 2.7 ms, 3.6 and 3.2 ms, and 5% more for a
+// directed scene of 64 primitives.
+__device__ __forceinline__ uint32_t route_len(const LaunchParams &P, const WideDev &W, uint32_t step, uint32_t level) {
+  const uint32_t waves = max(1u, 8u * P.long_count[step & TSI_STEP_MASK] / gridDim.x);
+  return (uint32_t)min((unsigned long long)wide_min_len(W, level) * waves, 0xffffffffull);
 }
 
 __device__ __forceinline__ StepIdx step_idx(uint32_t step) {
@@ -619,7 +634,7 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       uint32_t wrec = rec;
       TapeRec WR;
       find_valid(P, wrec, WR, wl, wh);
-      if (WR.len >= wide_min_len(S.wide, it.level + 1u)) {
+      if (WR.len >= route_len(P, S.wide, step, it.level + 1u)) {
         // A long tape: no pass over it on one warp.  A group with a widened
         // child hands its children, with that tape's record, to the wide
         // path; the other groups prune from the first pass's decisions.
@@ -633,7 +648,7 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
         PR = WR;
         want_prune = (flags & SF_PRUNING) && PR.len >= TSI_PRUNE_MIN_LEN && PR.nregs <= TSI_PRUNE_MAX_REGS;
       }
-      if (want_prune && WR.len < wide_min_len(S.wide, it.level + 1u)) {
+      if (want_prune && WR.len < route_len(P, S.wide, step, it.level + 1u)) {
         float4 *lgs;
         uint2 *dgs;
         if (!item_scratch(P, step, it.scene, PR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
@@ -739,9 +754,11 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
 #pragma unroll
     for (int b2 = 0; b2 < 8; ++b2) cb[b2] = __shfl_sync(FULL_MASK, C, gl0 + b2);
     const uint32_t next_len = (new_rec == prec) ? PR.len : ((new_rec == rec) ? TR.len : cnt);
-    if (k == 0 && E != 0)
-      push_children(P, S, it.scene, new_rec, step, it.level, E, cb, next_len >= wide_min_len(S.wide, it.level + 1u),
+    if (k == 0 && E != 0) {
+      if (next_len >= wide_min_len(S.wide, it.level + 1u)) atomicAdd(&P.long_count[si.next], (uint32_t)__popc(E));
+      push_children(P, S, it.scene, new_rec, step, it.level, E, cb, next_len >= route_len(P, S.wide, step, it.level + 1u),
                     ws);
+    }
   }
 
   // ---- counters
@@ -979,7 +996,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
       // wide path evaluates the full tape), or may: children the full wide
       // list turns away run narrow on this record
       const bool wide_room = *(const volatile uint32_t *)&P.witem_count[si.next] + 8u <= P.witem_cap;
-      if (total < n_narrow && (total < wide_min_len(W, it.level + 1u) || !wide_room)) {
+      if (total < n_narrow && (total < route_len(P, W, step, it.level + 1u) || !wide_room)) {
         const unsigned long long off = code_alloc(P, total);
         if (off != ~0ull) {
           const uint32_t ri = rec_alloc(P);
@@ -1082,8 +1099,9 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
   const long long f2 = clock64();
   if (tid < 32u) {
     const uint32_t len = (new_rec == S.root_rec) ? root.len : sh.cnt;
+    if (tid == 0 && len >= wide_min_len(W, it.level + 1u)) atomicAdd(&P.long_count[si.next], (uint32_t)__popc(E));
     push_children_warp(P, S, it.scene, new_rec, step, it.level, E, it.parent[1], it.parent[2] != 0u,
-                       len >= wide_min_len(W, it.level + 1u), ws, tid);
+                       len >= route_len(P, W, step, it.level + 1u), ws, tid);
   }
   if (tid == 0) {
     const long long f3 = clock64();
@@ -1394,6 +1412,7 @@ __device__ __forceinline__ void clear_step(const LaunchParams &P, uint32_t c) {
   P.dealloc_count[c] = 0;
   P.dealloc_cursor[c] = 0;
   P.log_overflow_used[c] = 0;
+  P.long_count[c] = 0;
 }
 
 // A warp's counters belong to the scene whose items it counted: they are
