@@ -27,6 +27,7 @@
 #include "ir_lower.h"
 #include "tape_compile.h"
 #include "trace_params.h"
+#include "wide_tape.h"
 #include "tsi.h"
 
 namespace tsi {
@@ -186,15 +187,20 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
   L.levels = tree_levels(p);
   L.full_len = s->tape->len;
   L.narrow_parents = s->tape->narrow_parents;
-  L.wide.slots = s->tape->d_wslots;
+  L.wide.fwd = s->tape->d_wfwd;
+  L.wide.rev = s->tape->d_wrev;
+  L.wide.rev16 = s->tape->d_wrev16;
+  L.wide.live = s->tape->d_wlive;
   L.wide.bundles = s->tape->d_wbundles;
   L.wide.narrow_mm = s->tape->d_wmm;
-  L.wide.nslots = s->tape->wslots;
+  L.wide.rev_slots = s->tape->wrev_slots;
+  L.wide.ctl = s->tape->d_wctl;
+  L.wide.streams = s->tape->d_wstreams;
   L.wide.nbundles = s->tape->wbundles;
   L.wide.nvalues = s->tape->wvalues;
   // a tape without a bundled form never sends a cell to the wide path,
   // whatever thresholds were set on it
-  const bool has_wide = s->tape->d_wslots != nullptr && s->tape->wbundles > 0;
+  const bool has_wide = s->tape->d_wfwd != nullptr && s->tape->wbundles > 0;
   L.wide.min_len = has_wide ? s->tape->wmin_len : 0xffffffffu;
   L.wide.deep_level = s->tape->wdeep_level;
   L.wide.deep_min_len = has_wide ? s->tape->wdeep_min_len : 0xffffffffu;
@@ -221,11 +227,11 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
 }
 
 // Shared-memory working set of one wide cell (the device's cell_layout):
-// values and sensitivities (8 bytes per SSA value each), contribution
-// records, decision bits, liveness flags.
+// values and sensitivities (8 bytes per SSA value each, the zero and the
+// dummy among them), contribution records, decision bytes, liveness flags.
 size_t wide_cell_bytes(size_t nvalues, size_t ncontrib, size_t bm_words) {
-  return 16 * nvalues + ((ncontrib * 8 + 15) & ~size_t(15)) + ((bm_words * 4 + 15) & ~size_t(15)) +
-         ((nvalues + 15) & ~size_t(15));
+  const size_t nv = nvalues + 2;
+  return ((16 * nv + ncontrib * 8 + 15) & ~size_t(15)) + (bm_words + 1) * 16 + ((nv + 15) & ~size_t(15));
 }
 // Tapes whose cell working set exceeds this stay on the narrow path (the
 // block also needs its static shared memory and room for a second block's
@@ -246,7 +252,7 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
     const tsi_tape *t = scenes[i]->tape;
     fp.lmax = std::max(fp.lmax, tree_levels(scenes[i]->p));
     rmax = std::max(rmax, t->nregs);
-    if (t->d_wslots) mm_max = std::max(mm_max, t->n_minmax);
+    if (t->d_wfwd) mm_max = std::max(mm_max, t->n_minmax);
   }
   bm_words = std::max(1u, (mm_max + 15u) / 16u);
   fp.rcap = (rmax + 3u) & ~3u;
@@ -270,9 +276,9 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
   fp.global.assign(n, 0);
   for (uint32_t i = 0; i < n; ++i) {
     const tsi_tape *t = scenes[i]->tape;
-    if (!t->d_wslots) continue;
+    if (!t->d_wfwd) continue;
     const size_t b = wide_cell_bytes(t->wvalues, t->wcontrib, bm_words);
-    if (b > budget) {
+    if (b > budget || !t->d_wrev16) {
       fp.global[i] = 1;
       gm_bytes = std::max(gm_bytes, b);
     } else {
@@ -1052,27 +1058,27 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
     WideTape wt;
     if (compile_wide(ins, pt, wt, st, why) && wt.nbundles > 0 &&
         wide_cell_bytes(wt.nvalues, wt.ncontrib, (pt.n_minmax + 15) / 16) <= kWideCellMaxGlobalBytes) {
-      // device layout: the three uint4 of every slot in three arrays
-      const size_t nsl = wt.slots.size() / 12;
-      std::vector<uint32_t> soa(wt.slots.size());
-      for (size_t i = 0; i < nsl; ++i)
-        for (size_t q = 0; q < 3; ++q)
-          for (size_t w = 0; w < 4; ++w) soa[(q * nsl + i) * 4 + w] = wt.slots[i * 12 + q * 4 + w];
-      cudaError_t e = dalloc(&t->d_wslots, wt.slots.size() / 4);
-      if (e == cudaSuccess) e = dalloc(&t->d_wbundles, wt.bundles.size() / 2);
-      if (e == cudaSuccess) e = dalloc(&t->d_wmm, wt.narrow_mm.size());
-      if (e == cudaSuccess)
-        e = cudaMemcpy(t->d_wslots, soa.data(), soa.size() * 4, cudaMemcpyHostToDevice);
-      if (e == cudaSuccess)
-        e = cudaMemcpy(t->d_wbundles, wt.bundles.data(), wt.bundles.size() * 4, cudaMemcpyHostToDevice);
-      if (e == cudaSuccess)
-        e = cudaMemcpy(t->d_wmm, wt.narrow_mm.data(), wt.narrow_mm.size() * 4, cudaMemcpyHostToDevice);
+      WideTapeDev dv;
+      decode_wide(wt, dv);
+      auto up = [](auto **dst, const std::vector<uint32_t> &src) -> cudaError_t {
+        cudaError_t r = dalloc(dst, src.size() * sizeof(uint32_t) / sizeof(**dst));
+        if (r == cudaSuccess && !src.empty()) r = cudaMemcpy(*dst, src.data(), src.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+        return r;
+      };
+      cudaError_t e = up(&t->d_wfwd, dv.fwd);
+      if (e == cudaSuccess) e = up(&t->d_wrev, dv.rev);
+      if (e == cudaSuccess) e = up(&t->d_wrev16, dv.rev16);
+      if (e == cudaSuccess) e = up(&t->d_wlive, dv.live);
+      if (e == cudaSuccess) e = up(&t->d_wctl, dv.ctl);
+      if (e == cudaSuccess) e = up(&t->d_wstreams, dv.streams);
+      if (e == cudaSuccess) e = up(&t->d_wbundles, dv.bundles);
+      if (e == cudaSuccess) e = up(&t->d_wmm, wt.narrow_mm);
       if (e != cudaSuccess) {
         g_last_error = cudaGetErrorString(e);
         tsi_tape_destroy(t);
         return TSI_ERR_CUDA;
       }
-      t->wslots = (uint32_t)nsl;
+      t->wrev_slots = dv.rev_slots;
       t->wbundles = wt.nbundles;
       t->wvalues = wt.nvalues;
       // four bundle steps' worth of instructions: near the fastest of the
@@ -1124,7 +1130,7 @@ TSI_API void tsi_tape_destroy(tsi_tape *t) {
   if (!t) return;
   if (t->ctx) t->ctx->tapes.erase(t);
   cudaFree(t->d_code);
-  cudaFree(t->d_wslots);
+  cudaFree(t->d_wfwd);
   cudaFree(t->d_wbundles);
   cudaFree(t->d_wmm);
   delete t;
@@ -1439,13 +1445,13 @@ TSI_API uint32_t tsi_tape_wide_threshold(const tsi_tape *t) { return t ? t->wmin
 
 TSI_API tsi_status tsi_tape_set_wide_threshold(tsi_tape *t, uint32_t min_len) {
   if (!t) return set_err(TSI_ERR_INVALID_ARGUMENT, "null tape");
-  if (t->d_wslots) t->wmin_len = min_len;
+  if (t->d_wfwd) t->wmin_len = min_len;
   return TSI_OK;
 }
 
 TSI_API tsi_status tsi_tape_set_wide_threshold_deep(tsi_tape *t, uint32_t level, uint32_t min_len) {
   if (!t) return set_err(TSI_ERR_INVALID_ARGUMENT, "null tape");
-  if (!t->d_wslots) return TSI_OK;  // no bundled form: every cell stays on the narrow path
+  if (!t->d_wfwd) return TSI_OK;  // no bundled form: every cell stays on the narrow path
   t->wdeep_level = level;
   t->wdeep_min_len = min_len;
   return TSI_OK;
@@ -1481,7 +1487,7 @@ TSI_API tsi_status tsi_scene_autotune(tsi_scene *s, const float *times, uint32_t
   memset(out, 0, sizeof(*out));
   // the tape belongs to the caller's context; its threshold is the tunable
   tsi_tape *t = const_cast<tsi_tape *>(s->tape);
-  if (!t->d_wslots) {
+  if (!t->d_wfwd) {
     out->wide_threshold = t->wmin_len;
     return tsi_scene_reset(s);
   }
@@ -1999,7 +2005,7 @@ TSI_API tsi_status tsi_batch_autotune(tsi_ctx *c, const tsi_request *reqs, uint3
   for (uint32_t i = 0; i < n; ++i) {
     if (!reqs[i].scene || reqs[i].scene->ctx != c) return set_err(TSI_ERR_INVALID_ARGUMENT, "bad request scene");
     tsi_tape *t = const_cast<tsi_tape *>(reqs[i].scene->tape);
-    if (t->d_wslots && std::find(tapes.begin(), tapes.end(), t) == tapes.end()) {
+    if (t->d_wfwd && std::find(tapes.begin(), tapes.end(), t) == tapes.end()) {
       tapes.push_back(t);
       base.push_back(t->wmin_len);
       base_deep.push_back(t->wdeep_min_len);

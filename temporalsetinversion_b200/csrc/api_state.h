@@ -42,10 +42,12 @@ struct tsi_tape {
   uint32_t count = 0, nregs = 0, out_reg = 0, n_minmax = 0;
   uint64_t fwd_cost = 0, rev_cost = 0;
   // bundled form for the wide path (absent when the tape is short)
-  uint4 *d_wslots = nullptr;
+  uint4 *d_wfwd = nullptr, *d_wrev = nullptr, *d_wlive = nullptr, *d_wrev16 = nullptr;
+  uint2 *d_wstreams = nullptr;
+  uint32_t *d_wctl = nullptr;
   uint2 *d_wbundles = nullptr;
   uint32_t *d_wmm = nullptr;
-  uint32_t wslots = 0, wbundles = 0, wvalues = 0, wmin_len = 0xffffffffu, wcontrib = 0;
+  uint32_t wrev_slots = 0, wbundles = 0, wvalues = 0, wmin_len = 0xffffffffu, wcontrib = 0;
   uint32_t wdeep_level = 0xffffffffu, wdeep_min_len = 0xffffffffu;  // level-dependent threshold (off by default)
   uint32_t narrow_parents = 1;  // parents per narrow item above the leaf level
   uint32_t wprune_level = 0xffffffffu;  // first level whose wide groups prune (0xffffffff: half the levels)

@@ -74,12 +74,16 @@ struct SceneCounters {
 // Bundled form of a scene's full tape (tape_compile.h WideTape), evaluated
 // with one block per cell for items whose tape is long.
 struct WideDev {
-  const uint4 *slots;         // [3][nslots]: words 0-3, 4-7, 8-11 of each slot (tape_compile.h)
-  const uint2 *bundles;       // first slot, slot count (padding included)
+  const uint4 *fwd, *rev;     // the streams' slots (wide_tape.h)
+  const uint4 *rev16;         // null: some index needs more than 16 bits
+  const uint32_t *ctl;        // the streams' step bytes
+  const uint2 *streams;       // [16]
+  const uint4 *live;          // bundle by bundle, for the liveness pass
+  const uint2 *bundles;       // of `live`: first slot, slot count (a multiple of 32)
   const uint32_t *narrow_mm;  // min/max ordinal per narrow instruction
-  uint32_t nslots;
+  uint32_t rev_slots;
   uint32_t nbundles;
-  uint32_t nvalues;           // SSA values (nslots + 4); the field is the last
+  uint32_t nvalues;           // SSA values; the field is the last (the zero and the dummy follow)
   uint32_t min_len;           // tapes at least this long go to the wide path
   uint32_t deep_level;        // children at this level or deeper use deep_min_len (TSI_NONE: never)
   uint32_t deep_min_len;

@@ -829,18 +829,30 @@ __device__ void dealloc_brick(const LaunchParams &P, uint2 item, uint32_t step, 
 // cells of an item run on eight blocks; the last to finish prunes the
 // group's tape and enqueues its children.
 
-// Byte offsets of a cell's working set (values, sensitivities, contribution
-// records, decision bits, liveness flags); the host sizes it the same way.
+// Byte offsets of a cell's working set (values; sensitivities and, behind
+// them, the contribution records; a decision byte per min/max; liveness
+// flags) and its size; the host sizes it the same way.
 struct CellLayout {
-  uint32_t sens, rec, bits, flags;
+  uint32_t sens, dec, flags, size;
 };
 __device__ __forceinline__ CellLayout cell_layout(const WideDev &W, uint32_t bm_words) {
   CellLayout L;
-  L.sens = W.nvalues * 8u;
-  L.rec = L.sens + W.nvalues * 8u;
-  L.bits = L.rec + ((W.ncontrib * 8u + 15u) & ~15u);
-  L.flags = L.bits + ((bm_words * 4u + 15u) & ~15u);
+  const uint32_t nv = W.nvalues + 2u;
+  L.sens = nv * 8u;
+  L.dec = (L.sens + (nv + W.ncontrib) * 8u + 15u) & ~15u;
+  L.flags = L.dec + (bm_words + 1u) * 16u;  // one more for the padding lanes
+  L.size = L.flags + ((nv + 15u) & ~15u);
   return L;
+}
+// Sixteen decision bytes as a word of two bits each (bytes past the tape's
+// last min/max hold anything).
+__device__ __forceinline__ uint32_t pack_decisions(const uint8_t *dec, uint32_t w) {
+  const uint4 b = *reinterpret_cast<const uint4 *>(dec + 16u * w);
+  auto four = [](uint32_t x) {
+    x &= 0x03030303u;
+    return (x | (x >> 6) | (x >> 12) | (x >> 18)) & 255u;
+  };
+  return four(b.x) | (four(b.y) << 8) | (four(b.z) << 16) | (four(b.w) << 24);
 }
 
 constexpr uint32_t kSmemBundles = 512;  // bundle descriptors held in shared memory
@@ -931,7 +943,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
   uint32_t new_rec = S.root_rec;
   if (want_prune) {
     const CellLayout L = cell_layout(W, P.bm_words);
-    uint32_t *cb = reinterpret_cast<uint32_t *>(cell + L.bits);  // decisions shared by the enqueued cells
+    uint32_t *cb = reinterpret_cast<uint32_t *>(cell + L.dec);  // decisions shared by the enqueued cells
     uint8_t *flags = cell + L.flags;
     const uint32_t words = (root.n_minmax + 15u) >> 4;
     const uint32_t *gbits = P.cell_bits[si.buf] + (size_t)unit0 * P.bm_words;
@@ -941,18 +953,17 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
         if ((E >> q) & 1u) acc &= gbits[(size_t)q * P.bm_words + w];
       cb[w] = acc;
     }
-    for (uint32_t i = tid; i < W.nvalues; i += blockDim.x) flags[i] = 0;
+    for (uint32_t i = tid; i < W.nvalues + 2u; i += blockDim.x) flags[i] = 0;
     __syncthreads();
     // liveness from the field backwards, bundle by bundle
     {
       const uint2 *bt_tab = bundle_table(W, sh);
-      const uint4 *__restrict__ slots = W.slots;
-      const uint32_t ns = W.nslots;
+      const uint4 *__restrict__ slots = W.live;
       const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
       auto fetch = [&](int kk) -> uint4 {
         if (kk < 0) return zero4;
         const uint2 b = bt_tab[kk];
-        return tid < b.y ? slots[ns + b.x + tid] : zero4;
+        return tid < b.y ? slots[b.x + tid] : zero4;
       };
       if (tid == 0) flags[W.nvalues - 1u] = 1;
       int kb = (int)W.nbundles - 1;
@@ -1133,15 +1144,13 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
   const uint32_t C = base + k;
   const CellLayout L = cell_layout(W, P.bm_words);
   if constexpr (!GM) {  // the host sized the launch for this cell; never write past it
-    if (L.flags + ((W.nvalues + 15u) & ~15u) > P.dyn_smem) {
+    if (L.size > P.dyn_smem) {
       if (tid == 0) atomicOr(P.error + it.scene, EB_SMEM);
       return;
     }
   }
-  float2 *V = reinterpret_cast<float2 *>(cell);
-  float2 *G = reinterpret_cast<float2 *>(cell + L.sens);
-  float2 *R = reinterpret_cast<float2 *>(cell + L.rec);
-  uint32_t *bits = reinterpret_cast<uint32_t *>(cell + L.bits);
+  const CellArray<GM> V(cell), G(cell + L.sens);
+  uint8_t *dec = cell + L.dec, *dec2 = cell + L.flags;
   // the cell's and its parent's state, loaded before the bundle table's
   // copy and barrier so that the loads overlap
   const float4 pxy = pool.box_xy[Pv];
@@ -1158,7 +1167,6 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
   }
   if (W.nbundles <= kSmemBundles)
     for (uint32_t i = tid; i < W.nbundles; i += blockDim.x) sh.bt[i] = W.bundles[i];
-  const uint2 *bt_tab = bundle_table(W, sh);
   __syncthreads();
 
   // ---- cell setup (compute.wgsl:3582-3626), uniform across the block
@@ -1232,26 +1240,17 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
     }
   }
   const bool dual = evaluate && want_prune && (wl < targ.lo || wh > targ.hi);
-  uint32_t *bits2 = reinterpret_cast<uint32_t *>(cell + L.flags);
 
   // ---- forward and reverse over the full tape, bundle by bundle
   Iv field = iv(0.0f);
   Iv sens[4] = {iv(0.0f), iv(0.0f), iv(0.0f), iv(0.0f)};
   if (evaluate) {
-    if (want_prune)
-      for (uint32_t w = tid; w < words; w += blockDim.x) {
-        bits[w] = 0u;
-        if (dual) bits2[w] = 0u;
-      }
     const long long c0 = clock64();
-    if (dual)
-      field = cell_forward2<D>(W, bt_tab, V, G, bits, bits2, cx, cy, cz, targ, Iv{wl, wh});
-    else
-      field = cell_forward<D>(W, bt_tab, V, want_prune ? bits : nullptr, cx, cy, cz, targ);
+    field = cell_forward<D, GM>(W, V, G, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz, targ, Iv{wl, wh});
     const long long c1 = clock64();
     if (take_deriv) {
-      cell_reverse<D>(W, bt_tab, V, G, R, sh.sens);
-      for (int q = 0; q < 4; ++q) sens[q] = ldv(sh.sens, q);
+      cell_reverse<D, GM>(W, V, G, sh.sens);
+      for (int q = 0; q < 4; ++q) sens[q] = Iv{sh.sens[q].x, sh.sens[q].y};
     }
     if (tid == 0) {
       ws[ST_CYC_WIDE_FWD] += (unsigned long long)(c1 - c0);
@@ -1355,11 +1354,10 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
     __syncthreads();
     if (tid == 0) ws[ST_FP32] += (unsigned long long)root.fwd_cost;
     if (dual && nl == wl && nh == wh) {  // taken in the forward pass
-      for (uint32_t w = tid; w < words; w += blockDim.x) bits[w] = bits2[w];
+      dec = dec2;
     } else {
       const long long r0 = clock64();
-      for (uint32_t w = tid; w < words; w += blockDim.x) bits[w] = 0u;
-      (void)cell_forward<D>(W, bt_tab, V, bits, cx, cy, cz, Iv{nl, nh});
+      (void)cell_forward<D, GM>(W, V, G, false, dec, nullptr, cx, cy, cz, Iv{nl, nh}, targ);
       if (tid == 0) {
         ws[ST_WIDE_REFWD] += 1ull;
         ws[ST_CYC_WIDE_REFWD] += (unsigned long long)(clock64() - r0);
@@ -1370,7 +1368,7 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
   __syncthreads();
   if (want_prune && enq) {
     uint32_t *dst = P.cell_bits[si.buf] + (size_t)unit * P.bm_words;
-    for (uint32_t w = tid; w < words; w += blockDim.x) dst[w] = bits[w];
+    for (uint32_t w = tid; w < words; w += blockDim.x) dst[w] = pack_decisions(dec, w);
   }
   if (tid == 0 && want_prune) {  // the time ranges matter only to a pruning finish
     CellInfo ci;

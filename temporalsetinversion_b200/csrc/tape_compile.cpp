@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "opcost.h"
+#include "wide_tape.h"
 
 namespace tsi {
 namespace {
@@ -362,6 +363,138 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   out.nvalues = n;
   out.nbundles = nb;
   return true;
+}
+
+void decode_wide(const WideTape &wt, WideTapeDev &out) {
+  const uint32_t nv = wt.nvalues, zero = nv, dummy = nv + 1u, nv2 = nv + 2u;
+  out = WideTapeDev{};
+  std::vector<uint8_t> used(nv, 0);  // values some instruction reads
+  uint32_t n_minmax = 0;             // a padding lane's ordinal is one past the last
+  for (size_t i = 0; i < wt.slots.size(); i += 12) {
+    const uint32_t *S = &wt.slots[i];
+    if ((S[0] & 63u) == TSI_H_PAD) continue;
+    if (S[6] != TSI_NONE) used[S[6]] = 1;
+    if (S[7] != TSI_NONE) used[S[7]] = 1;
+    if (S[5] != TSI_NONE) n_minmax = std::max(n_minmax, S[5] + 1u);
+  }
+  std::vector<uint32_t> targets;
+  auto push4 = [](std::vector<uint32_t> &v, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    v.push_back(a);
+    v.push_back(b);
+    v.push_back(c);
+    v.push_back(d);
+  };
+  const uint32_t minus0 = 0x80000000u;
+  const bool small = nv2 + wt.ncontrib <= 65536u;  // (a value's records are as many as its users)
+  // One group (warp g of bundle k) of the forward or reverse streams; its
+  // kind.
+  auto emit = [&](uint32_t k, uint32_t g, bool reverse) -> uint32_t {
+    const uint32_t first = wt.bundles[2 * k] + 32u * g, left = wt.bundles[2 * k + 1] - 32u * g;
+    const uint32_t h = wt.slots[size_t(first) * 12] & 63u;  // the group's handler
+    const bool ii = TSI_H_IS_II(h);
+    if (reverse && h == H_CONST) return WK_NONE;  // nothing to propagate
+    uint32_t kind = WK_OTHER, base = ii ? WC_II : 0u;
+    bool gather = false;
+    switch (h) {
+      case H_ADD_II: case H_ADD_IF: case H_SUB_IF: case H_COPY: case H_SUB_II: case H_SUB_FI: case H_NEG:
+        kind = WK_LIN;
+        break;
+      case H_MUL_IF: kind = WK_SCALE; break;
+      case H_MUL_II: kind = WK_MUL; break;
+      case H_SQR: kind = WK_SQR; break;
+      case H_ABS: kind = WK_ABS; break;
+      case H_SQRT: kind = WK_SQRT; break;
+      case H_SIN: kind = WK_SIN; break;
+      case H_MAX_II: case H_MAX_IF: base |= WC_MAX; kind = WK_MM; break;
+      case H_MIN_II: case H_MIN_IF: kind = WK_MM; break;
+      default: break;
+    }
+    for (uint32_t s = 0; s < 32u; ++s) {
+      const uint32_t *S = s < left ? &wt.slots[size_t(first + s) * 12] : nullptr;
+      const bool pad = !S || (S[0] & 63u) == TSI_H_PAD;
+      const uint32_t a = pad || S[6] == TSI_NONE ? zero : S[6];
+      const uint32_t b = pad || S[7] == TSI_NONE ? zero : S[7];
+      const uint32_t mmo = pad || S[5] == TSI_NONE ? n_minmax : S[5];
+      const uint32_t lit = pad || ii ? 0u : S[3];
+      uint32_t c = base, x = a, y = ii ? b : zero, w = lit;
+      if (kind == WK_OTHER && !reverse) {  // the handler travels where the literal or B does not
+        if (ii) w = h;
+        else y = h;
+      }
+      if (!reverse) {
+        if (kind == WK_MM) {
+          if (ii) w = mmo;
+          else y = mmo;
+        }
+        switch (h) {
+          case H_ADD_II: case H_COPY: c |= WC_ZERO; w = minus0; break;
+          case H_SUB_II: c |= WC_ZERO | WC_NEG | WC_SWAP; x = b; y = a; w = minus0; break;
+          case H_SUB_IF: w = lit ^ minus0; break;
+          case H_SUB_FI: c |= WC_NEG | WC_SWAP; break;
+          case H_NEG: c |= WC_NEG | WC_SWAP | WC_ZERO; w = minus0; break;
+          default: break;
+        }
+        push4(out.fwd, c | ((pad ? dummy : S[4]) << WC_DST_SHIFT), x, y, w);
+        continue;
+      }
+      if (h == H_SUB_II) c |= WC_NEG2;
+      if (h == H_SUB_FI || h == H_NEG) c |= WC_NEG;
+      const uint32_t fa = pad ? 0u : (S[0] >> 6) & 1u, fb = pad ? 0u : (S[0] >> 7) & 1u;
+      if (fa && (!ii || fb)) c |= WC_SKIP;
+      uint32_t ta = dummy, tb = dummy, src = zero, n = 0;
+      if (!pad) {
+        if (S[6] != TSI_NONE) ta = S[8] != TSI_NONE ? nv2 + S[8] : S[6];
+        if (S[7] != TSI_NONE) tb = S[9] != TSI_NONE ? nv2 + S[9] : S[7];
+        // a value nobody reads has sensitivity zero, the field one
+        n = S[11];
+        src = n ? nv2 + S[10] : (used[S[4]] || S[4] == nv - 1u ? S[4] : zero);
+        gather = gather || n != 0u;
+      }
+      push4(out.rev, c | (h << 8), x, y, w);
+      push4(targets, ta, tb, src, n);
+      if (small) push4(out.rev16, x | (src << 16), ta | (tb << 16), ii ? y : w, c | (h << 8) | (n << 16));
+    }
+    return kind | (reverse && gather ? WK_GATHER : 0u);
+  };
+  for (uint32_t dir = 0; dir < 2u; ++dir) {
+    const bool reverse = dir == 1u;
+    for (uint32_t g = 0; g < kWideWarps; ++g) {
+      out.streams.push_back(uint32_t((reverse ? out.rev : out.fwd).size() / 4));
+      out.streams.push_back(uint32_t(out.ctl.size()));
+      std::vector<uint8_t> bytes;
+      for (uint32_t q = 0; q < wt.nbundles; ++q) {
+        const uint32_t k = reverse ? wt.nbundles - 1u - q : q;
+        bytes.push_back(uint8_t(32u * g < wt.bundles[2 * k + 1] ? emit(k, g, reverse) : WK_NONE));
+      }
+      while (bytes.size() % kWideAhead) bytes.push_back(uint8_t(WK_NONE));
+      for (uint32_t q = 0; q < kWideAhead + 4u; ++q) bytes.push_back(uint8_t(WK_NONE));
+      for (size_t i = 0; i < bytes.size(); i += 4)
+        out.ctl.push_back(bytes[i] | (uint32_t(bytes[i + 1]) << 8) | (uint32_t(bytes[i + 2]) << 16) |
+                          (uint32_t(bytes[i + 3]) << 24));
+    }
+  }
+  // a warp reads one slot past its last group's
+  for (uint32_t s = 0; s < 32u; ++s) {
+    push4(out.fwd, dummy << WC_DST_SHIFT, zero, zero, 0u);
+    push4(out.rev, 0u, zero, zero, 0u);
+    push4(targets, dummy, dummy, zero, 0u);
+    if (small) push4(out.rev16, zero | (zero << 16), dummy | (dummy << 16), 0u, 0u);
+  }
+  out.rev_slots = uint32_t(out.rev.size() / 4);
+  out.rev.insert(out.rev.end(), targets.begin(), targets.end());
+  uint32_t nslots = 0;
+  for (uint32_t k = 0; k < wt.nbundles; ++k) {
+    const uint32_t first = wt.bundles[2 * k], count = wt.bundles[2 * k + 1];
+    const uint32_t padded = (count + 31u) & ~31u;
+    out.bundles.push_back(nslots);
+    out.bundles.push_back(padded);
+    nslots += padded;
+    for (uint32_t s = 0; s < padded; ++s) {
+      const uint32_t *S = s < count ? &wt.slots[size_t(first + s) * 12] : nullptr;
+      if (!S || (S[0] & 63u) == TSI_H_PAD) push4(out.live, dummy, TSI_NONE, TSI_NONE, TSI_NONE);
+      else push4(out.live, S[4], S[5], S[6], S[7]);
+    }
+  }
 }
 
 }  // namespace tsi

@@ -6,41 +6,116 @@
 // compute.wgsl:3786-3900 with per-use contribution records for values with
 // several users (their sensitivities are summed in the sequential order).
 //
-// A bundle step is a block barrier apart from the next, and its cost is
-// mostly fixed (the barrier, the dependent shared-memory loads, the
-// handler dispatch), so the schedule packs groups of different handlers
-// into one step, one handler per warp.  Each thread reads its handler from
-// its slot; min/max slots (which also record their decisions) have bodies
-// of their own, every other handler shares one generic body, which keeps
-// the loops small enough for the instruction cache (bodies specialised per
-// handler measured no faster, and slower in the reverse pass).
+// A bundle step is a block barrier apart from the next and a cell is a chain
+// of steps, so a step's latency is the cost: what a warp issues between two
+// barriers, about four cycles an instruction.  The host therefore decodes
+// every slot (wide_tape.h): a kind for the whole warp, operand indices that
+// always name a value (an absent one the zero, a padding lane's result the
+// dummy), sensitivity targets that are a value's or a record's place in one
+// array.  A step then takes no test but those on its group's kind, which
+// comes as a byte of a word made uniform for the compiler once in four
+// steps; linear handlers are one fused form; a value with one user needs no
+// accumulator; and the slots of the next four steps are on their way.  (Eight
+// steps ahead hide a load's 900 cycles from L2 better for a lone cell, but
+// the walk unrolled eight times costs levels that mix cells and items a fifth
+// in instruction fetches; the slots out of line, 5% at every level.)
+// 256-primitive tape (32 steps), levels of 64 cells: 31 thousand cycles
+// forward and 58 thousand reverse with a switch over the handlers and slots
+// found through the bundle table, 25 and 52 thousand with this form;
+// inversions of the 256-primitive animation at localsubdiv 10 0.80 to 0.77
+// ms, rotating swept scene 2.66 to 2.58 ms.
 #pragma once
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "device_types.h"
 #include "interp.cuh"
+#include "narrow_interp.cuh"
+#include "wide_tape.h"
 
 namespace tsi {
 
-__device__ __forceinline__ Iv ldv(const float2 *a, uint32_t i) {
-  const float2 v = a[i];
-  return Iv{v.x, v.y};
-}
-__device__ __forceinline__ void stv(float2 *a, uint32_t i, Iv v) { a[i] = make_float2(v.lo, v.hi); }
-
-// A thread's slot of bundle kk and the bundle's slot count, or a padding
-// slot past the bundle (or past the tape).
-struct WideFetch {
-  const uint2 *bt;
-  const uint4 *__restrict__ slots;
-  uint32_t nb, tid;
-  __device__ __forceinline__ uint4 operator()(int kk, uint32_t word_group, uint32_t ns) const {
-    if (kk < 0 || (uint32_t)kk >= nb) return make_uint4(TSI_H_PAD, 0u, TSI_NONE, TSI_NONE);
-    const uint2 b = bt[kk];
-    return tid < b.y ? slots[word_group * ns + b.x + tid] : make_uint4(TSI_H_PAD, 0u, TSI_NONE, TSI_NONE);
+// A cell's array of intervals: shared memory by its 32-bit address, or (GM)
+// the block's slice of the global scratch.
+template <bool GM>
+struct CellArray;
+template <>
+struct CellArray<false> {
+  uint32_t base;
+  __device__ __forceinline__ explicit CellArray(void *p) : base((uint32_t)__cvta_generic_to_shared(p)) {}
+  __device__ __forceinline__ Iv ld(uint32_t i) const {
+    Iv v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.lo), "=f"(v.hi) : "r"(base + i * 8u) : "memory");
+    return v;
+  }
+  __device__ __forceinline__ void st(uint32_t i, Iv v) const {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(base + i * 8u), "f"(v.lo), "f"(v.hi) : "memory");
   }
 };
+template <>
+struct CellArray<true> {
+  float2 *base;
+  __device__ __forceinline__ explicit CellArray(void *p) : base(reinterpret_cast<float2 *>(p)) {}
+  __device__ __forceinline__ Iv ld(uint32_t i) const {
+    const float2 v = base[i];
+    return Iv{v.x, v.y};
+  }
+  __device__ __forceinline__ void st(uint32_t i, Iv v) const { base[i] = make_float2(v.lo, v.hi); }
+};
+
+// The barrier between two steps.  The warps arrive from different places of
+// their walks (every warp arrives once per step); PTX counts the arrivals at
+// the barrier, whichever instruction they come from.
+__device__ __forceinline__ void step_barrier() { asm volatile("barrier.sync 0;" ::: "memory"); }
+
+// One warp's walk through the steps: `step(q, kind)` runs on its slot of each
+// step it has a group in.  The next kWideAhead steps' slots are on their way
+// in registers, at addresses that depend on nothing loaded but the kinds (a
+// load that waits for a test of a loaded table, or whose result is selected,
+// is waited for at once); a step without a group reads the slot of the next
+// one that has (an L1 hit).
+// Steps are rounded up to a multiple of kWideAhead, for every warp alike.
+template <typename Step>
+__device__ __forceinline__ void walk_steps(const WideDev &W, uint32_t stream, const uint4 *__restrict__ recs,
+                                           Step step) {
+  const uint2 st = W.streams[stream];
+  const uint32_t n = uniform_u32(W.nbundles);
+  const uint32_t *__restrict__ ctl = W.ctl + st.y;
+  const uint4 *ptr = recs + st.x + (threadIdx.x & 31u);
+  constexpr uint32_t kWords = kWideAhead / 4u;
+  const uint32_t last = (n + kWideAhead - 1u) / kWideAhead * kWords + kWords;
+  uint32_t c[kWords], l[kWords];
+  uint4 q[kWideAhead];
+#pragma unroll
+  for (uint32_t i = 0; i < kWords; ++i) c[i] = uniform_u32(ctl[i]);
+#pragma unroll
+  for (uint32_t i = 0; i < kWords; ++i) l[i] = ctl[kWords + i];
+#pragma unroll
+  for (uint32_t u = 0; u < kWideAhead; ++u) {
+    q[u] = *ptr;
+    ptr += ((c[u / 4u] >> (8u * (u & 3u))) & 31u) != WK_NONE ? 32 : 0;
+  }
+  for (uint32_t k = 0; k < n; k += kWideAhead) {
+    uint32_t next[kWords];
+#pragma unroll
+    for (uint32_t i = 0; i < kWords; ++i) {
+      next[i] = uniform_u32(l[i]);
+      l[i] = ctl[min(k / 4u + 2u * kWords + i, last)];
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < kWideAhead; ++u) {
+      const uint32_t kind = (c[u / 4u] >> (8u * (u & 3u))) & 31u;
+      const uint32_t ahead = (next[u / 4u] >> (8u * (u & 3u))) & 31u;
+      if (kind != WK_NONE) step(q[u], kind);
+      q[u] = *ptr;
+      ptr += ahead != WK_NONE ? 32 : 0;
+      step_barrier();
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kWords; ++i) c[i] = next[i];
+  }
+}
 
 // 2-bit decision of a min/max over A and B (compute.wgsl:3660-3700): bit 0
 // the A operand is always chosen, bit 1 the B operand is.
@@ -50,221 +125,205 @@ __device__ __forceinline__ uint32_t minmax_decision(bool amax, Iv A, Iv B) {
 }
 
 // ---------------------------------------------------------------- forward
-template <bool D, uint32_t H>
-__device__ __forceinline__ void fwd_slot(float2 *V, uint32_t *bits, const uint4 &sl) {
-  const float lit = __uint_as_float(sl.w);
-  const Iv A = ldv(V, sl.y);
-  const Iv B = TSI_H_IS_II(H) ? ldv(V, sl.z) : iv(lit);
-  stv(V, sl.x >> 8, op_forward<D>(H, A, B, lit));
-  if (TSI_H_IS_MINMAX(H) && bits) {
-    const uint32_t mm = TSI_H_IS_II(H) ? sl.w : sl.z;
-    const uint32_t d = minmax_decision(H == H_MAX_II || H == H_MAX_IF, A, B);
-    if (d) atomicOr(&bits[mm >> 4], d << (2u * (mm & 15u)));
+// One slot over one of the time intervals: its value to V, a min/max's
+// decision to dec (a byte per min/max) when it is set.
+template <bool D, bool GM>
+__device__ __forceinline__ void wide_forward_slot(uint32_t kind_, uint4 q, CellArray<GM> V, uint8_t *dec) {
+  using I = IA<D>;
+  const Iv X = V.ld(q.y), Y0 = V.ld(q.z);
+  const uint32_t kind = uniform_u32(kind_);
+  const float f = __uint_as_float(q.w);
+  Iv v;
+  if (kind == WK_LIN) {
+    // X or -X, plus the literal or Y (the other is the zero that changes no sum)
+    const float m = (q.x & WC_NEG) ? -1.0f : 1.0f;
+    const Iv S = (q.x & WC_SWAP) ? Iv{X.hi, X.lo} : X;
+    if (!D) {
+      const F2 r = f2_add(f2_fma(f2_dup(m), f2_pack(S.lo, S.hi), f2_dup(f)), f2_pack(Y0.lo, Y0.hi));
+      f2_unpack(r, v.lo, v.hi);
+    } else {
+      const float lo = (q.x & WC_ZERO) ? 0.0f : f, hi = (q.x & WC_ZERO) ? -0.0f : f;
+      v = Iv{__fadd_rd(__fmaf_rd(m, S.lo, lo), Y0.lo), __fadd_ru(__fmaf_ru(m, S.hi, hi), Y0.hi)};
+    }
+  } else if (kind == WK_SCALE) {
+    v = I::mul_f(X, f);
+  } else if (kind == WK_SQR) {
+    v = I::sqr(X);
+  } else if (kind == WK_MM) {
+    const Iv B = (q.x & WC_II) ? Y0 : iv(f);
+    const bool mx = q.x & WC_MAX;
+    const Iv lo = I::min_(X, B), hi = I::max_(X, B);
+    v = mx ? hi : lo;
+    if (dec) dec[(q.x & WC_II) ? q.w : q.z] = (uint8_t)minmax_decision(mx, X, B);
+  } else if (kind == WK_MUL) {
+    v = I::mul(X, Y0);
+  } else if (kind == WK_ABS) {
+    v = I::abs_(X);
+  } else if (kind == WK_SQRT) {
+    v = I::sqrt_(X);
+  } else if (kind == WK_SIN) {
+    v = I::sin_(X);
+  } else {
+    const bool ii = q.x & WC_II;
+    v = cold_forward<D>(ii ? q.w : q.z, X, ii ? Y0 : iv(f), f);
   }
-}
-template <bool D>
-__device__ __forceinline__ void fwd_slot_any(uint32_t h, float2 *V, const uint4 &sl) {
-  const float lit = __uint_as_float(sl.w);
-  const Iv A = ldv(V, sl.y);
-  const Iv B = TSI_H_IS_II(h) ? ldv(V, sl.z) : iv(lit);
-  stv(V, sl.x >> 8, op_forward<D>(h, A, B, lit));
+  V.st(q.x >> WC_DST_SHIFT, I::fix(v));
 }
 
 // Forward pass over the bundles (compute.wgsl:3633-3772); returns the field.
-// `bits`: 2 bits per min/max of this cell (A always chosen, B always chosen).
-template <bool D>
-__device__ __forceinline__ Iv cell_forward(const WideDev &W, const uint2 *bt_tab, float2 *V, uint32_t *bits, Iv x, Iv y, Iv z,
-                           Iv t) {
+// dual: over two time intervals at once, V holding the values over `t` (the
+// field and the reverse pass use them) and V2 those over `t2`, whose min/max
+// decisions go to dec2 (those over `t` to dec); the second evaluation is
+// independent of the first, so a step runs both.  Every min/max writes its
+// decision byte when dec is set.
+template <bool D, bool GM>
+__device__ __forceinline__ Iv cell_forward(const WideDev &W, CellArray<GM> V, CellArray<GM> V2, bool dual, uint8_t *dec,
+                                           uint8_t *dec2, Iv x, Iv y, Iv z, Iv t, Iv t2) {
   const uint32_t tid = threadIdx.x;
-  const int nb = (int)W.nbundles;
-  const WideFetch fetch{bt_tab, W.slots, (uint32_t)nb, tid};
   if (tid == 0) {
-    stv(V, 0, x);
-    stv(V, 1, y);
-    stv(V, 2, z);
-    stv(V, 3, t);
-  }
-  // slots fetched three bundles ahead of their use
-  uint4 q0 = fetch(0, 0, 0), q1 = fetch(1, 0, 0), q2 = fetch(2, 0, 0);
-  __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    const uint4 sl = q0;
-    q0 = q1;
-    q1 = q2;
-    q2 = fetch(k + 3, 0, 0);
-    const uint32_t h = sl.x & 63u;
-    if (TSI_H_IS_MINMAX(h)) {
-      switch (h) {
-        case H_MIN_II: fwd_slot<D, H_MIN_II>(V, bits, sl); break;
-        case H_MAX_II: fwd_slot<D, H_MAX_II>(V, bits, sl); break;
-        case H_MIN_IF: fwd_slot<D, H_MIN_IF>(V, bits, sl); break;
-        default: fwd_slot<D, H_MAX_IF>(V, bits, sl); break;
-      }
-    } else if (h != TSI_H_PAD) {
-      fwd_slot_any<D>(h, V, sl);
+    const Iv zero = Iv{D ? 0.0f : -0.0f, -0.0f};
+    V.st(0, x);
+    V.st(1, y);
+    V.st(2, z);
+    V.st(3, t);
+    V.st(W.nvalues, zero);
+    if (dual) {
+      V2.st(0, x);
+      V2.st(1, y);
+      V2.st(2, z);
+      V2.st(3, t2);
+      V2.st(W.nvalues, zero);
     }
-    __syncthreads();
   }
-  return ldv(V, W.nvalues - 1u);
-}
-
-// cell_forward over two time intervals at once: V holds the values over
-// `t` (the field and the reverse pass use them), V2 those over `t2`, whose
-// min/max decisions go to bits2 (those over `t` to bits).  The second
-// evaluation is independent of the first, so a bundle step runs both.
-template <bool D, uint32_t H>
-__device__ __forceinline__ void fwd2_slot(float2 *V, float2 *V2, uint32_t *bits, uint32_t *bits2, const uint4 &sl) {
-  const float lit = __uint_as_float(sl.w);
-  const Iv A = ldv(V, sl.y), A2 = ldv(V2, sl.y);
-  const Iv B = TSI_H_IS_II(H) ? ldv(V, sl.z) : iv(lit);
-  const Iv B2 = TSI_H_IS_II(H) ? ldv(V2, sl.z) : iv(lit);
-  stv(V, sl.x >> 8, op_forward<D>(H, A, B, lit));
-  stv(V2, sl.x >> 8, op_forward<D>(H, A2, B2, lit));
-  if (TSI_H_IS_MINMAX(H)) {
-    const uint32_t mm = TSI_H_IS_II(H) ? sl.w : sl.z;
-    const uint32_t sh = 2u * (mm & 15u);
-    constexpr bool amax = (H == H_MAX_II || H == H_MAX_IF);
-    const uint32_t d = minmax_decision(amax, A, B), d2 = minmax_decision(amax, A2, B2);
-    if (d) atomicOr(&bits[mm >> 4], d << sh);
-    if (d2) atomicOr(&bits2[mm >> 4], d2 << sh);
-  }
-}
-template <bool D>
-__device__ __forceinline__ void fwd2_slot_any(uint32_t h, float2 *V, float2 *V2, const uint4 &sl) {
-  const float lit = __uint_as_float(sl.w);
-  const bool II = TSI_H_IS_II(h);
-  const Iv A = ldv(V, sl.y), A2 = ldv(V2, sl.y);
-  const Iv B = II ? ldv(V, sl.z) : iv(lit);
-  const Iv B2 = II ? ldv(V2, sl.z) : iv(lit);
-  stv(V, sl.x >> 8, op_forward<D>(h, A, B, lit));
-  stv(V2, sl.x >> 8, op_forward<D>(h, A2, B2, lit));
-}
-
-template <bool D>
-__device__ __forceinline__ Iv cell_forward2(const WideDev &W, const uint2 *bt_tab, float2 *V, float2 *V2,
-                                            uint32_t *bits, uint32_t *bits2, Iv x, Iv y, Iv z, Iv t, Iv t2) {
-  const uint32_t tid = threadIdx.x;
-  const int nb = (int)W.nbundles;
-  const WideFetch fetch{bt_tab, W.slots, (uint32_t)nb, tid};
-  if (tid == 0) {
-    stv(V, 0, x);
-    stv(V, 1, y);
-    stv(V, 2, z);
-    stv(V, 3, t);
-    stv(V2, 0, x);
-    stv(V2, 1, y);
-    stv(V2, 2, z);
-    stv(V2, 3, t2);
-  }
-  uint4 q0 = fetch(0, 0, 0), q1 = fetch(1, 0, 0), q2 = fetch(2, 0, 0);
   __syncthreads();
-  for (int k = 0; k < nb; ++k) {
-    const uint4 sl = q0;
-    q0 = q1;
-    q1 = q2;
-    q2 = fetch(k + 3, 0, 0);
-    const uint32_t h = sl.x & 63u;
-    if (TSI_H_IS_MINMAX(h)) {
-      switch (h) {
-        case H_MIN_II: fwd2_slot<D, H_MIN_II>(V, V2, bits, bits2, sl); break;
-        case H_MAX_II: fwd2_slot<D, H_MAX_II>(V, V2, bits, bits2, sl); break;
-        case H_MIN_IF: fwd2_slot<D, H_MIN_IF>(V, V2, bits, bits2, sl); break;
-        default: fwd2_slot<D, H_MAX_IF>(V, V2, bits, bits2, sl); break;
-      }
-    } else if (h != TSI_H_PAD) {
-      fwd2_slot_any<D>(h, V, V2, sl);
-    }
-    __syncthreads();
-  }
-  return ldv(V, W.nvalues - 1u);
+  const bool both = __any_sync(FULL_MASK, dual);
+  walk_steps(W, tid >> 5, W.fwd, [&](const uint4 &q, uint32_t kind) {
+    wide_forward_slot<D, GM>(kind, q, V, dec);
+    if (both) wide_forward_slot<D, GM>(kind, q, V2, dec2);
+  });
+  return V.ld(W.nvalues - 1u);
 }
 
 // Sum of a value's contribution records, last user first, onto +0: the
-// accumulation order of the sequential reverse pass.
-template <bool D>
-__device__ __forceinline__ Iv gather_sens(const float2 *R, uint32_t base, uint32_t count) {
+// accumulation order of the sequential reverse pass.  The sums are one
+// dependent chain; the loads run ahead of it.
+template <bool D, bool GM>
+__device__ __forceinline__ Iv gather_sens(CellArray<GM> R, uint32_t base, uint32_t count) {
   Iv S = iv(0.0f);
   uint32_t i = 0;
-  for (; i + 4u <= count; i += 4u) {  // loads ahead of the dependent adds
-    const float2 c0 = R[base + i], c1 = R[base + i + 1u], c2 = R[base + i + 2u], c3 = R[base + i + 3u];
-    S = IA<D>::add(Iv{c0.x, c0.y}, S);
-    S = IA<D>::add(Iv{c1.x, c1.y}, S);
-    S = IA<D>::add(Iv{c2.x, c2.y}, S);
-    S = IA<D>::add(Iv{c3.x, c3.y}, S);
+  for (; i + 8u <= count; i += 8u) {
+    Iv c[8];
+#pragma unroll
+    for (uint32_t u = 0; u < 8u; ++u) c[u] = R.ld(base + i + u);
+#pragma unroll
+    for (uint32_t u = 0; u < 8u; ++u) S = IA<D>::add(c[u], S);
   }
-  for (; i < count; ++i) S = IA<D>::add(ldv(R, base + i), S);
+  for (; i < count; ++i) S = IA<D>::add(R.ld(base + i), S);
   return S;
 }
 
 // ---------------------------------------------------------------- reverse
+// A slot of the reverse pass, unpacked (wide_tape.h).
+struct WideRevSlot {
+  uint32_t flags, a, b, lit, ta, tb, src, count;
+};
+
 // One slot of the reverse pass: its sensitivity (its own value's, or the sum
 // of its contribution records), the handler's reverse rule and the
-// operands' sensitivities (a record per use for an operand with several
-// users, else written directly; the skip rule of compute.wgsl:3800-3806).
-template <bool D>
-__device__ __forceinline__ void rev_slot_body(uint32_t h, const float2 *V, float2 *G, float2 *R, const uint4 &sl,
-                                              const uint4 &s2) {
+// operands' shares, each to its target in G: the operand's own place (one
+// user: nothing else is added to it) or this use's record.
+template <bool D, bool GM>
+__device__ __forceinline__ void wide_reverse_slot(uint32_t kind_, WideRevSlot p, CellArray<GM> V, CellArray<GM> G) {
   using I = IA<D>;
-  const bool II = TSI_H_IS_II(h);
-  const uint32_t fa = (sl.x >> 6) & 1u, fb = (sl.x >> 7) & 1u;
-  const uint32_t a = sl.y, b = sl.z;
-  const float lit = __uint_as_float(sl.w);
-  const Iv A = ldv(V, a);
-  const Iv B = II ? ldv(V, b) : iv(lit);
-  const Iv s = s2.w ? gather_sens<D>(R, s2.z, s2.w) : ldv(G, sl.x >> 8);
-  const bool s0 = (s.lo == 0.0f && s.hi == 0.0f);
-  const bool skip = II ? (s0 && fa && fb) : (s0 && fa);
-  Iv c0 = iv(0.0f), c1 = iv(0.0f);
-  if (!skip) {
-    Iv r0, r1;
-    op_reverse_rule<D>(h, A, B, lit, r0, r1);
+  const float f = __uint_as_float(p.lit);
+  const Iv A = V.ld(p.a), B0 = V.ld(p.b);
+  const uint32_t kg = uniform_u32(kind_), kind = kg & 15u;
+  Iv s;
+  if (kg & WK_GATHER) s = p.count ? gather_sens<D, GM>(G, p.src, p.count) : G.ld(p.src);
+  else s = G.ld(p.src);
+  // a point factor's product (exact in the directed form: the factor is 0 or
+  // +-1, so one rounding mode serves both bounds)
+  auto point_mul = [&](float c) -> Iv {
+    const float u = __fmul_rn(c, s.lo), w = __fmul_rn(c, s.hi);
+    const Iv r = Iv{fm_min(u, w), fm_max(u, w)};
+    if (D && (u != u || w != w)) return I::entire();
+    return r;
+  };
+  Iv c0, c1 = iv(0.0f);
+  if (kind == WK_LIN) {
+    c0 = point_mul((p.flags & WC_NEG) ? -1.0f : 1.0f);
+    c1 = point_mul((p.flags & WC_NEG2) ? -1.0f : 1.0f);
+  } else if (kind == WK_SCALE) {
+    c0 = I::mul(I::fix(iv(f)), s);
+  } else if (kind == WK_SQR) {
+    c0 = I::mul(I::fix(I::mul_f(A, 2.0f)), s);
+  } else if (kind == WK_MM) {
+    // a decided min/max passes the sensitivity to one operand, an undecided
+    // one to both (directed: by a factor in [0, 1])
+    const Iv B = (p.flags & WC_II) ? B0 : iv(f);
+    const bool mx = p.flags & WC_MAX, a_below = A.hi < B.lo, b_below = !a_below && B.hi < A.lo;
+    const bool a_out = mx ? a_below : b_below, b_out = mx ? b_below : a_below;
+    c0 = point_mul(a_out ? 0.0f : 1.0f);
+    c1 = point_mul(b_out ? 0.0f : 1.0f);
+    if (D && !a_out && !b_out) c0 = c1 = I::mul(Iv{0.0f, 1.0f}, s);
+  } else if (kind == WK_MUL) {
+    c0 = I::mul(I::fix(B0), s);
+    c1 = I::mul(I::fix(A), s);
+  } else if (kind == WK_ABS) {
+    c0 = I::mul(I::abs_rr(A), s);
+  } else if (kind == WK_SQRT) {
+    c0 = I::mul(I::fix(I::sqrt_rr(A)), s);
+  } else if (kind == WK_SIN) {
+    c0 = I::mul(I::fix(I::cos_(A)), s);
+  } else {
+    const bool ii = p.flags & WC_II;
+    Iv r0 = iv(0.0f), r1 = iv(0.0f);
+    cold_reverse_rule<D>((p.flags >> 8) & 63u, A, ii ? B0 : iv(f), f, r0, r1);
     c0 = I::mul(I::fix(r0), s);
-    if (II) c1 = I::mul(I::fix(r1), s);
+    c1 = I::mul(I::fix(r1), s);
   }
-  // both operands read before either is written (an instruction whose
-  // operands are one value keeps the second write)
-  const Iv pa = (s2.x == TSI_NONE && !skip) ? ldv(G, a) : iv(0.0f);
-  const Iv pb = (II && s2.y == TSI_NONE && !skip) ? ldv(G, b) : iv(0.0f);
-  if (s2.x != TSI_NONE) stv(R, s2.x, c0);
-  else stv(G, a, skip ? iv(0.0f) : I::add(c0, pa));
-  if (II) {
-    if (s2.y != TSI_NONE) stv(R, s2.y, c1);
-    else stv(G, b, skip ? iv(0.0f) : I::add(c1, pb));
-  }
+  c0 = I::add(c0, iv(0.0f));
+  c1 = I::add(c1, iv(0.0f));
+  // the skip rule of compute.wgsl:3800-3806 (flagged operands of a zero
+  // sensitivity receive zero); to nearest a finite factor's product with a
+  // zero adds a zero anyway
+  if (D && (p.flags & WC_SKIP) && s.lo == 0.0f && s.hi == 0.0f) c0 = c1 = iv(0.0f);
+  G.st(p.ta, c0);
+  G.st(p.tb, c1);
 }
 
-// Reverse interval AD over the bundles (compute.wgsl:3786-3900).  A
-// single-use operand's sensitivity is written by its one user; an operand
-// with several users gets a contribution record per user (R), summed when
-// the reverse pass reaches the value.  sens_out: 4 floats x 2 in shared
-// memory for the arguments' sensitivities.
-template <bool D>
-__device__ __forceinline__ void cell_reverse(const WideDev &W, const uint2 *bt_tab, const float2 *V, float2 *G, float2 *R,
-                             float2 *sens_out) {
+// Reverse interval AD over the bundles (compute.wgsl:3786-3900).  G: the
+// values' sensitivities and behind them the contribution records.  sens_out:
+// the four arguments' sensitivities, in shared memory.
+template <bool D, bool GM>
+__device__ __forceinline__ void cell_reverse(const WideDev &W, CellArray<GM> V, CellArray<GM> G, float2 *sens_out) {
   const uint32_t tid = threadIdx.x;
-  const uint32_t ns = W.nslots, nv = W.nvalues;
-  const int nb = (int)W.nbundles;
-  const WideFetch fetch{bt_tab, W.slots, (uint32_t)nb, tid};
-  for (uint32_t v = tid; v < nv; v += blockDim.x) G[v] = make_float2(0.0f, 0.0f);
-  // words 0-3 and 8-11 of this thread's slot, two bundles ahead
-  uint4 a0 = fetch(nb - 1, 0, ns), a2 = fetch(nb - 1, 2, ns);
-  uint4 b0 = fetch(nb - 2, 0, ns), b2 = fetch(nb - 2, 2, ns);
+  if (tid < 4u) G.st(tid, iv(0.0f));
+  if (tid == 4u) G.st(W.nvalues, iv(0.0f));       // the zero
+  if (tid == 5u) G.st(W.nvalues + 1u, iv(0.0f));  // the dummy
+  if (tid == 6u) G.st(W.nvalues - 1u, iv(1.0f));  // the field
   __syncthreads();
-  if (tid == 0) G[nv - 1u] = make_float2(1.0f, 1.0f);
-  __syncthreads();
-  for (int k = nb - 1; k >= 0; --k) {
-    const uint4 sl = a0, s2 = a2;
-    a0 = b0;
-    a2 = b2;
-    b0 = fetch(k - 2, 0, ns);
-    b2 = fetch(k - 2, 2, ns);
-    const uint32_t h = sl.x & 63u;
-    if (h != TSI_H_PAD && h != H_CONST) rev_slot_body<D>(h, V, G, R, sl, s2);
-    __syncthreads();
+  const uint32_t stream = kWideWarps + (tid >> 5), nv = W.nvalues;
+  if (GM) {  // indices of more than 16 bits: the second array's slot is read in the step
+    const uint4 *t = W.rev + W.rev_slots + W.streams[stream].x + (tid & 31u);
+    walk_steps(W, stream, W.rev, [&](const uint4 &p, uint32_t kind) {
+      const uint4 r = *t;
+      t += 32;
+      wide_reverse_slot<D, GM>(kind, WideRevSlot{p.x, p.y, p.z, p.w, r.x, r.y, r.z, r.w}, V, G);
+    });
+  } else {
+    walk_steps(W, stream, W.rev16, [&](const uint4 &p, uint32_t kind) {
+      const bool ii = p.w & WC_II;
+      wide_reverse_slot<D, GM>(kind,
+                               WideRevSlot{p.w & 0xffffu, p.x & 0xffffu, ii ? p.z : nv, p.z, p.y & 0xffffu, p.y >> 16,
+                                           p.x >> 16, p.w >> 16},
+                               V, G);
+    });
   }
   if (tid < 4u) {
     const uint32_t gc = W.arg_gcount[tid];
-    stv(sens_out, tid, gc ? gather_sens<D>(R, W.arg_gbase[tid], gc) : ldv(G, tid));
+    const Iv s = gc ? gather_sens<D, GM>(G, nv + 2u + W.arg_gbase[tid], gc) : G.ld(tid);
+    sens_out[tid] = make_float2(s.lo, s.hi);
   }
   __syncthreads();
 }

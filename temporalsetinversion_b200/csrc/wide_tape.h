@@ -1,0 +1,63 @@
+// wide_tape.h — device form of the bundled tape: the slots of tape_compile.h's
+// WideTape decoded for wide_interp.cuh, written once per tape by the host.
+//
+// The passes read the tape as eight streams, one per warp of the block: a
+// warp's groups of 32 slots one after another, in the order of their bundles
+// (the reverse pass's streams in the reverse order), so that the next slot's
+// address is the last one's plus 512 bytes.  Beside them runs a byte per step
+// (bundle) and warp, four to a word: the kind of the warp's group, or that it
+// has none.
+// A padding lane has its group's kind, reads the zero value and writes the
+// dummy.  Value indices: the SSA values 0 .. nvalues-1, then the zero (the
+// one an addition leaves unchanged) and the dummy.  Sensitivity targets index
+// the values' places and, after the dummy's, the contribution records.
+//   forward  x: flags, destination << 8   y: operand A   z: operand B
+//            w: literal or factor; the min/max ordinal sits in w (two
+//            registers) or z (register and literal), the handler of WK_OTHER
+//            likewise
+//   reverse  x: flags, handler << 8   y: A   z: B   w: literal or factor
+//            second array: targets of A's and of B's share, the slot's own
+//            sensitivity: its place, or its first record and their count
+//   reverse, when every index has 16 bits (cells in shared memory), one array:
+//            x: A, own sensitivity << 16   y: targets of A's, B's << 16
+//            z: B (two registers) or the literal   w: flags, handler << 8,
+//            record count << 16
+// The liveness pass walks bundles, whose slots are padded to whole warps.
+#pragma once
+#include <stdint.h>
+
+#include <vector>
+
+namespace tsi {
+
+constexpr uint32_t WK_LIN = 0, WK_SQR = 1, WK_MM = 2, WK_MUL = 3, WK_ABS = 4, WK_SQRT = 5, WK_SIN = 6, WK_OTHER = 7;
+constexpr uint32_t WK_SCALE = 8;  // a literal's multiple (linear to nearest, a product directed)
+constexpr uint32_t WK_NONE = 9;   // no group
+constexpr uint32_t WK_GATHER = 16;  // (reverse) some slot of the group sums contribution records: + kind
+constexpr uint32_t WC_II = 1u << 0;     // two register operands
+constexpr uint32_t WC_SWAP = 1u << 1;   // (forward linear) A's bounds change places
+constexpr uint32_t WC_NEG = 1u << 2;    // (linear) factor -1 on A
+constexpr uint32_t WC_ZERO = 1u << 3;   // (forward linear) the literal is the zero that changes no sum
+constexpr uint32_t WC_NEG2 = 1u << 4;   // (reverse linear) factor -1 on B
+constexpr uint32_t WC_MAX = 1u << 5;    // (min/max) max
+constexpr uint32_t WC_SKIP = 1u << 6;   // (reverse) every operand is flagged single-use
+constexpr uint32_t WC_DST_SHIFT = 8;
+constexpr uint32_t kWideAhead = 4;  // steps whose slots a warp has on their way (a multiple of 4)
+constexpr uint32_t kWideWarps = 8;
+
+struct WideTape;
+struct PackedTape;
+
+struct WideTapeDev {
+  std::vector<uint32_t> fwd;      // 4 words per slot, stream after stream
+  std::vector<uint32_t> rev;      // 4 words per slot of the first array, then the second array
+  std::vector<uint32_t> rev16;    // 4 words per slot (empty: some index needs more than 16 bits)
+  std::vector<uint32_t> ctl;      // step bytes, four to a word: the forward streams, then the reverse ones,
+                                  // each with kWideAhead steps and a word more at its end
+  std::vector<uint32_t> streams;  // 2 words per stream (8 forward, 8 reverse): first slot, first ctl word
+  std::vector<uint32_t> live;     // 4 words per slot: destination, min/max ordinal, A, B (TSI_NONE: absent)
+  std::vector<uint32_t> bundles;  // of `live`: first slot, slot count (a multiple of 32)
+  uint32_t rev_slots = 0;         // slots of the reverse streams
+};
+void decode_wide(const WideTape &wt, WideTapeDev &out);
+}  // namespace tsi
