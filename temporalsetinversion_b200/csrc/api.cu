@@ -542,6 +542,13 @@ void make_camera(const tsi_params &p, const tsi_uniforms &u, TraceParams &T) {
   T.rendermode = u.rendermode;
   T.normal_viz = p.normal_viz ? 1u : 0u;
   T.darken = p.octree_darken_factor;
+  T.plain_boxes = 1u;
+  for (int a = 0; a < 3; ++a) {  // extents of the root and of the smallest cells
+    const float e = p.root_hi[a] - p.root_lo[a];
+    if (!(e <= 16777216.0f) || !(ldexpf(e, -(int)tree_levels(p) - 1) >= 5.9604645e-08f) ||
+        !(fabsf(p.root_lo[a]) <= 16777216.0f))
+      T.plain_boxes = 0u;
+  }
 }
 
 // Whether the context's stream is being captured into a graph (no host

@@ -73,6 +73,30 @@ TSI_DEV F2 f2_fma(F2 a, F2 b, F2 c) {
 }
 TSI_DEV F2 f2_dup(float a) { return f2_pack(a, a); }
 
+// Correctly rounded reciprocal, quotient and square root without a branch,
+// for operands and results well inside the normal range (the callers check):
+// the hardware's approximation and one residual step each, Markstein's
+// scheme ("Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990).  Compared with __frcp_rn and __fsqrt_rn for every
+// mantissa and exponents -60..60 and -80..80, the quotient with __fdiv_rn for
+// 8.6 thousand million pairs of exponents -20..20: no difference.
+TSI_DEV float fm_rcp_in(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return __fmaf_rn(__fmaf_rn(-d, y, 1.0f), y, y);
+}
+// n / d with y = fm_rcp_in(d)
+TSI_DEV float fm_div_in(float n, float d, float y) {
+  const float q = __fmul_rn(n, y);
+  return __fmaf_rn(__fmaf_rn(-d, q, n), y, q);
+}
+TSI_DEV float fm_sqrt_in(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float s = __fmul_rn(x, r);
+  return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, r), s);
+}
+
 TSI_DEV float fm_sin(float x) {
   const float two_over_pi = 0.6366197466850281f;
   const float p1 = 1.5703125f, p2 = 0.0004838705062866211f, p3 = -4.371138828673793e-08f;

@@ -86,8 +86,9 @@ struct Walk {
   uint32_t visits;
 };
 
+// The walk for any ray and any boxes (parallel rays, infinities, NaN).
 template <bool COLOR>
-__device__ __forceinline__ void walk_octree(const TraceParams &T, F3 ro, F3 rd, F3 inv, Walk &w) {
+__device__ __noinline__ void walk_general(const TraceParams &T, F3 ro, F3 rd, F3 inv, Walk &w) {
   const VoxelPoolDev &pool = T.pool;
   const float TEPS = 0.0001f;
   F3 c = f3(1.0f, 1.0f, 1.0f);
@@ -211,6 +212,168 @@ __device__ __forceinline__ void walk_octree(const TraceParams &T, F3 ro, F3 rd, 
   w.tnorm = hit_t;
   w.hit = intersected;
   w.visits = visits;
+}
+
+// Whether a ray may take the fast walk: its direction's components and, by
+// the caller, the boxes' extents are well inside the normal range.
+__device__ __forceinline__ bool plain_ray(F3 ro, F3 rd) {
+  const float lo = 9.094947e-13f, hi = 4.0f, far = 16777216.0f;  // 2^-40, 2^24
+  const float ax = fabsf(rd.x), ay = fabsf(rd.y), az = fabsf(rd.z);
+  return ax >= lo && ay >= lo && az >= lo && ax <= hi && ay <= hi && az <= hi && fabsf(ro.x) <= far &&
+         fabsf(ro.y) <= far && fabsf(ro.z) <= far;
+}
+
+// walk_general's results for such rays, bit for bit, in half the
+// instructions (the tracer is bound by instruction issue):
+//  - the nine divisions of a node's set-up share a reciprocal per axis and
+//    have no slow path (fm_rcp_in, fm_div_in);
+//  - the signs of the local direction are those of rd;
+//  - the march's mask is three predicates, its child index one integer that
+//    the steps add to; the step length is |sd - dd| of the one axis that
+//    stepped (the root of a square is the absolute value, exactly, without
+//    over- or underflow; Boldo 2015), the root only when axes tie;
+//  - the darkened colour is one number until the walk ends: its channels
+//    start equal and are scaled alike.
+template <bool COLOR>
+__device__ __forceinline__ void walk_plain(const TraceParams &T, F3 ro, F3 rd, F3 inv, Walk &w) {
+  const VoxelPoolDev &pool = T.pool;
+  const float TEPS = 0.0001f;
+  float shade = 1.0f;
+  F3 nrm = f3(0.0f, 0.0f, 0.0f);
+  uint32_t visits = 0;
+  bool intersected = false;
+  float hit_since = 0.0f;  // time since the leaf was evaluated
+  float hit_t = T.time;    // time of the finite-difference normal
+  uint32_t stack[32];
+  uint32_t sp = 0;
+  F3 ro2 = ro;
+  stack[sp++] = 0u;
+  uint32_t region = 0u;
+  F3 p0, p1;
+  node_box(pool, region, p0, p1);
+  F3 hit = slabs(p0, p1, ro2, inv);
+  const F3 sg = f3(rd.x > 0.0f ? 1.0f : -1.0f, rd.y > 0.0f ? 1.0f : -1.0f, rd.z > 0.0f ? 1.0f : -1.0f);
+  const F3 hs = muls(sg, 0.5f);
+  const int st0 = rd.x > 0.0f ? 1 : -1, st1 = rd.y > 0.0f ? 2 : -2, st2 = rd.z > 0.0f ? 4 : -4;
+  bool done = (hit.x == 0.0f);
+  for (uint32_t iter = 0; iter < 5000u && !done; ++iter) {
+    if (intersected) break;
+    if (sp == 0) {
+      done = true;
+      break;
+    }
+    region = stack[--sp];
+    if (hit.x == 0.0f) {
+      if (sp == 0) continue;
+      node_box(pool, stack[sp - 1], p0, p1);
+      hit = slabs(p0, p1, ro2, inv);
+      continue;
+    }
+    const uint32_t cbase = pool.child[region];
+    const F3 ext = p1 - p0;
+    const F3 num = muls((ro2 + muls(rd, hit.y + TEPS)) - p0, 2.0f);
+    float cell0, cell1, cell2, sd0, sd1, sd2, dd0, dd1, dd2;
+    auto axis = [](float n, float e, float d, float s, float h, float &cell, float &sd, float &dd) {
+      const float y = fm_rcp_in(e);
+      const float rol = fm_div_in(n, e, y);
+      dd = fm_rcp_in(fabsf(d * fm_div_in(2.0f, e, y)));
+      cell = floorf(rol);
+      sd = (__fmaf_rn(s, cell - rol, h) + 0.5f) * dd;
+    };
+    axis(num.x, ext.x, rd.x, sg.x, hs.x, cell0, sd0, dd0);
+    axis(num.y, ext.y, rd.y, sg.y, hs.y, cell1, sd1, dd1);
+    axis(num.z, ext.z, rd.z, sg.z, hs.z, cell2, sd2, dd2);
+    int ci = (int)cell0 + 2 * (int)cell1 + 4 * (int)cell2;
+    float len = 0.0f;  // |mask (sd - dd)| of the last step
+    const F3 old_ro2 = ro2;
+    // per node: the darkening of every DDA step and the exit distance
+    const bool darken = COLOR && !T.normal_viz && fm_max(ext.x, fm_max(ext.y, ext.z)) < 1.0f;
+    const float leave = hit.z - TEPS;
+    float t = 0.0f;
+    bool moved = false;
+    for (int i = 0; i < 32; ++i) {
+      if (darken) shade = shade * T.darken;
+      t = (len + hit.y) + TEPS;
+      moved = true;
+      if (t >= leave) {  // left the node (4277-4292)
+        ro2 = old_ro2 + muls(rd, hit.z);
+        moved = false;
+        if (sp == 0) {
+          hit = f3(0.0f, 0.0f, 0.0f);
+          break;
+        }
+        node_box(pool, stack[sp - 1], p0, p1);
+        hit = slabs(p0, p1, ro2, inv);
+        break;
+      }
+      if ((uint32_t)ci >= 8u) break;
+      if (cbase != TSI_NONE) {
+        const uint32_t child = cbase + (uint32_t)ci;
+        ++visits;
+        if (pool.f[child] <= 0.0f) {
+          ro2 = old_ro2 + muls(rd, t);
+          moved = false;
+          F3 q0, q1;
+          node_box(pool, child, q0, q1);
+          const F3 tp0 = f3(q0.x - TEPS, q0.y - TEPS, q0.z - TEPS);
+          const F3 tp1 = f3(q1.x + TEPS, q1.y + TEPS, q1.z + TEPS);
+          const F3 th = slabs(tp0, tp1, ro2, inv);
+          if (th.x == 1.0f) {
+            if (pool.child[child] != TSI_NONE) {
+              if (sp < 32) stack[sp++] = region;
+              if (sp < 32) stack[sp++] = child;
+              p0 = tp0;
+              p1 = tp1;
+              hit = th;
+              break;
+            }
+            // the leaf's colour is set after the walk (the fast normal is
+            // evaluated by the whole warp there)
+            intersected = true;
+            const float4 nv = pool.normal[child];
+            nrm = f3(nv.x, nv.y, nv.z);
+            hit_since = T.time - pool.t[child];
+            if (T.swept) hit_t = pool.t[region];  // compute.wgsl:4339-4341
+            break;
+          }
+        }
+      }
+      // 4389-4391
+      const bool b0 = sd0 <= fm_min(sd1, sd2), b1 = sd1 <= fm_min(sd2, sd0), b2 = sd2 <= fm_min(sd0, sd1);
+      float x0 = 0.0f, x1 = 0.0f, x2 = 0.0f;
+      if (b0) {
+        sd0 = sd0 + dd0;
+        x0 = sd0 - dd0;
+        ci += st0;
+      }
+      if (b1) {
+        sd1 = sd1 + dd1;
+        x1 = sd1 - dd1;
+        ci += st1;
+      }
+      if (b2) {
+        sd2 = sd2 + dd2;
+        x2 = sd2 - dd2;
+        ci += st2;
+      }
+      len = fabsf(b0 ? x0 : (b1 ? x1 : x2));
+      if ((b0 && (b1 || b2)) || (b1 && b2)) len = len3(f3(x0, x1, x2));
+    }
+    if (moved) ro2 = old_ro2 + muls(rd, t);
+  }
+  w.end = ro2;
+  w.c = f3(shade, shade, shade);
+  w.nrm = nrm;
+  w.since = hit_since;
+  w.tnorm = hit_t;
+  w.hit = intersected;
+  w.visits = visits;
+}
+
+template <bool COLOR>
+__device__ __forceinline__ void walk_octree(const TraceParams &T, F3 ro, F3 rd, F3 inv, Walk &w) {
+  if (T.plain_boxes && plain_ray(ro, rd)) walk_plain<COLOR>(T, ro, rd, inv, w);
+  else walk_general<COLOR>(T, ro, rd, inv, w);
 }
 
 // The colour of `trace` at the end of a walk from ro (4322-4401): the age
