@@ -72,6 +72,12 @@ TSI_DEV F2 f2_fma(F2 a, F2 b, F2 c) {
   return r;
 }
 TSI_DEV F2 f2_dup(float a) { return f2_pack(a, a); }
+// A packed product that no sum takes (see f2_mul).
+TSI_DEV F2 f2_mul_alone(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
 
 // Correctly rounded reciprocal, quotient and square root without a branch,
 // for operands and results well inside the normal range (the callers check):
