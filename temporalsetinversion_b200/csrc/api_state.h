@@ -37,6 +37,7 @@ struct TsiReadback {
 
 struct tsi_tape {
   tsi_ctx *ctx = nullptr;
+  void *d_block = nullptr;  // the one allocation that holds the tape's arrays on the device
   uint2 *d_code = nullptr;
   uint32_t len = 0;  // instructions after the 4 ARG slots
   uint32_t count = 0, nregs = 0, out_reg = 0, n_minmax = 0;

@@ -8,7 +8,7 @@ import pytest
 
 import oracle
 from conftest import assert_cells_equal
-from temporalsetinversion_b200 import Device, Scene, Tape, api
+from temporalsetinversion_b200 import Device, Scene, Tape, api, scenes
 from test_gpu_narrow import TIMES, mixed_tape
 
 
@@ -33,3 +33,20 @@ def test_wide_cells_match_oracle(device, scratch_device, length, where):
         gs.invert(time)
         os_.invert(time)
         assert_cells_equal(gs.cells(), os_.cells())
+
+
+@pytest.mark.gpu
+def test_destroyed_tapes_give_their_memory_back(device):
+    import torch
+
+    instr = api.IR.new(scenes.csg(64, 5)).gpu_instructions
+
+    def free_after(n):
+        for _ in range(n):
+            t = Tape.upload(device, instr)
+            del t
+        return torch.cuda.mem_get_info()[0]
+
+    before = free_after(20)
+    # 300 tapes of this scene hold more than 40 MB
+    assert before - free_after(300) < 8 << 20
