@@ -855,8 +855,6 @@ __device__ __forceinline__ uint32_t pack_decisions(const uint8_t *dec, uint32_t 
   return four(b.x) | (four(b.y) << 8) | (four(b.z) << 16) | (four(b.w) << 24);
 }
 
-constexpr uint32_t kSmemBundles = 512;  // bundle descriptors held in shared memory
-
 // Base of the block's cell working set: dynamic shared memory, or for tapes
 // too large for it the block's slice of the global scratch (each block of
 // the persistent grid owns one slice; L2 keeps the active slices).
@@ -866,19 +864,17 @@ __device__ __forceinline__ unsigned char *cell_base(const LaunchParams &P) {
   else return tsi_dyn_smem;
 }
 
+// (The kernel's static shared memory is what the largest register files
+// leave: eight of 108 registers with their buffers take 227328 of the 232448
+// bytes a block may have.)
 struct WideShared {
   uint32_t last, E, cnt, mmk, fcost, rcost, ri;
   unsigned long long off;
   float gl, gh, hl, hh;
   uint32_t scan[kWarps];
   float2 sens[4];
-  uint2 bt[kSmemBundles];  // the tape's bundle descriptors when they fit
+  uint2 cost[H_COUNT];  // (finish_group) a handler's forward and reverse cost
 };
-
-// Bundle descriptors: the shared copy when the tape has few enough bundles.
-__device__ __forceinline__ const uint2 *bundle_table(const WideDev &W, const WideShared &sh) {
-  return W.nbundles <= kSmemBundles ? sh.bt : W.bundles;
-}
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *scratch, uint32_t &total) {
   const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -902,7 +898,12 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 
 
 // The last cell of a wide item to finish: prunes the full tape with the
-// branch decisions shared by all enqueued siblings and enqueues them.
+// branch decisions shared by all enqueued siblings and enqueues them.  One
+// block runs it while the launch's end waits for it, bound by latency: loads
+// under a test waited for one after another, a branch per operand, a barrier
+// per compaction step and constant tables read at 32 indices made it 34k
+// cycles on a 4697-instruction tape and 59k on a 3240-instruction one; as
+// written 24k and 35k.
 template <bool GM>
 __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkItem &it, uint32_t step,
                                              uint32_t unit0, WideShared &sh, unsigned long long *ws) {
@@ -923,13 +924,18 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
     ws[ST_WIDE_FIN] += 1;
     // sh.E: the enqueued siblings, from the count-in
     float gl = -fm_inf(), gh = fm_inf(), hl = fm_inf(), hh = -fm_inf();
-    for (int q = 0; q < 8 && want_prune; ++q) {
-      const CellInfo ci = info[q];
-      gl = fmaxf(gl, ci.nl);
-      gh = fminf(gh, ci.nh);
-      if (ci.enq) {
-        hl = fminf(hl, ci.nl);
-        hh = fmaxf(hh, ci.nh);
+    if (want_prune) {
+      CellInfo ci[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) ci[q] = info[q];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        gl = fmaxf(gl, ci[q].nl);
+        gh = fminf(gh, ci[q].nh);
+        if (ci[q].enq) {
+          hl = fminf(hl, ci[q].nl);
+          hh = fmaxf(hh, ci[q].nh);
+        }
       }
     }
     sh.gl = gl;
@@ -943,59 +949,92 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
   uint32_t new_rec = S.root_rec;
   if (want_prune) {
     const CellLayout L = cell_layout(W, P.bm_words);
+    const uint32_t words = (root.n_minmax + 15u) >> 4;
     uint32_t *cb = reinterpret_cast<uint32_t *>(cell + L.dec);  // decisions shared by the enqueued cells
     uint8_t *flags = cell + L.flags;
-    const uint32_t words = (root.n_minmax + 15u) >> 4;
+    if constexpr (GM) {
+      // the liveness flags and the decisions of a cell in the global scratch
+      // go to shared memory all the same when they fit: the pass below is a
+      // chain of them (1024-primitive tape: 65k -> 25k cycles)
+      const uint32_t fb = (W.nvalues + 2u + 15u) & ~15u;
+      if (fb + (words + 1u) * 4u <= P.dyn_smem) {
+        flags = tsi_dyn_smem;
+        cb = reinterpret_cast<uint32_t *>(tsi_dyn_smem + fb);
+      }
+    }
     const uint32_t *gbits = P.cell_bits[si.buf] + (size_t)unit0 * P.bm_words;
     for (uint32_t w = tid; w < words; w += blockDim.x) {
-      uint32_t acc = 0xffffffffu;
-      for (int q = 0; q < 8; ++q)
-        if ((E >> q) & 1u) acc &= gbits[(size_t)q * P.bm_words + w];
+      uint32_t v[8], acc = 0xffffffffu;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = gbits[(size_t)q * P.bm_words + w];  // (all at once; some unused)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc &= v[q] | (((E >> q) & 1u) ? 0u : 0xffffffffu);
       cb[w] = acc;
     }
+    if (tid == 0) cb[words] = 0;  // (of a value that is no min/max)
+    if (tid < H_COUNT)
+      sh.cost[tid] = make_uint2(c_cost_fwd[tid] + TSI_FIX_COST, c_cost_rr[tid] + TSI_REV_OPERAND_COST * TSI_H_NREG(tid));
     for (uint32_t i = tid; i < W.nvalues + 2u; i += blockDim.x) flags[i] = 0;
+    // the values are done with: their place holds the bundle descriptors (a
+    // bundle has at least one value, of the same eight bytes)
+    uint2 *bt = reinterpret_cast<uint2 *>(cell);
+    for (uint32_t i = tid; i < W.nbundles; i += blockDim.x) bt[i] = W.bundles[i];
     __syncthreads();
-    // liveness from the field backwards, bundle by bundle
+    // Liveness from the field backwards, bundle by bundle; a step is bound by
+    // the latency of its slots, which are on their way four bundles ahead.
+    // Threads past a bundle's end repeat its last slot, and the steps past
+    // the first bundle repeat that: setting a flag twice changes nothing, and
+    // a load under a test or select would be waited for at once.
     {
-      const uint2 *bt_tab = bundle_table(W, sh);
       const uint4 *__restrict__ slots = W.live;
-      const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
       auto fetch = [&](int kk) -> uint4 {
-        if (kk < 0) return zero4;
-        const uint2 b = bt_tab[kk];
-        return tid < b.y ? slots[b.x + tid] : zero4;
+        const uint2 b = bt[max(kk, 0)];
+        return slots[b.x + min(tid, b.y - 1u)];
       };
       if (tid == 0) flags[W.nvalues - 1u] = 1;
-      int kb = (int)W.nbundles - 1;
-      uint4 q0 = fetch(kb), q1 = fetch(kb - 1);
+      uint4 q[4];
+      const int kb0 = (int)W.nbundles - 1;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = fetch(kb0 - i);
       __syncthreads();
-      for (; kb >= 0; --kb) {
-        const uint2 bt = bt_tab[kb];
-        const uint4 s1 = q0;
-        q0 = q1;
-        q1 = fetch(kb - 2);
-        if (tid < bt.y && flags[s1.x]) {
-          bool la = s1.z != TSI_NONE, lb = s1.w != TSI_NONE;
-          if (s1.y != TSI_NONE) {  // a min/max: its ordinal
-            const uint32_t d = (cb[s1.y >> 4] >> (2u * (s1.y & 15u))) & 3u;
-            if (d & 1u) lb = false;
-            else if (d & 2u) la = false;
-          }
-          if (la) flags[s1.z] = 1;
-          if (lb) flags[s1.w] = 1;
+#pragma unroll 1
+      for (int kb = kb0; kb >= 0; kb -= 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 s1 = q[i];
+          q[i] = fetch(kb - i - 4);
+          // a min/max has an ordinal: the decision may rule an operand out
+          const bool mm = s1.y != TSI_NONE, live = flags[s1.x] != 0;
+          const uint32_t d = cb[mm ? s1.y >> 4 : words] >> (2u * (s1.y & 15u));
+          if (live && s1.z != TSI_NONE && (d & 3u) != 2u) flags[s1.z] = 1;
+          if (live && s1.w != TSI_NONE && !(d & 1u)) flags[s1.w] = 1;
+          __syncthreads();
         }
-        __syncthreads();
       }
     }
     const long long f1 = clock64();
     if (tid == 0) ws[ST_CYC_FIN_LIVE] += (unsigned long long)(f1 - f0);
-    // compaction of the narrow full tape in program order, one instruction
-    // per thread a step: live instructions by ballot, output positions from
-    // the warps' counts (coalesced reads of the tape)
-    uint32_t mine = 0;
-    for (uint32_t i = tid; i < n_narrow; i += blockDim.x) mine += flags[i + 4u];
+    // Compaction of the narrow full tape in program order, a warp's 32
+    // consecutive instructions at a time: the groups' live counts, their
+    // prefix sums, and then every group by itself, without a barrier and with
+    // its instructions read four groups ahead.
+    const uint32_t lane = tid & 31u, wib = tid >> 5, nw = blockDim.x >> 5;
+    const uint32_t groups = (n_narrow + 31u) >> 5;
+    uint32_t *first = reinterpret_cast<uint32_t *>(cell);  // (the descriptors are done with)
+    for (uint32_t g = wib; g < groups; g += nw) {
+      const uint32_t i = g * 32u + lane;
+      const uint32_t bal = __ballot_sync(FULL_MASK, i < n_narrow && flags[i + 4u]);
+      if (lane == 0) first[g] = __popc(bal);
+    }
+    __syncthreads();
     uint32_t total = 0;
-    (void)block_exclusive_scan(mine, sh.scan, total);
+    for (uint32_t g0 = 0; g0 < groups; g0 += blockDim.x) {
+      const uint32_t g = g0 + tid;
+      uint32_t sum = 0;
+      const uint32_t ex = block_exclusive_scan(g < groups ? first[g] : 0u, sh.scan, sum);
+      if (g < groups) first[g] = total + ex;
+      total += sum;
+    }
     if (tid == 0) {
       sh.ri = TSI_NONE;
       sh.off = 0;
@@ -1020,65 +1059,58 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
     }
     __syncthreads();
     if (sh.ri != TSI_NONE) {
-      const uint32_t lane = tid & 31u, wib = tid >> 5, nw = blockDim.x >> 5;
       const unsigned long long off = sh.off;
-      uint32_t base = 0, mmk = 0, fc = 0, rc = 0;
-      // this thread's instruction of a step, read one step ahead
-      auto fetch = [&](uint32_t i, uint2 &w, uint32_t &mm) {
-        w = make_uint2(0u, 0u);
-        mm = TSI_NONE;
-        if (i < n_narrow) {
-          w = root.code[i];
-          mm = W.narrow_mm[i];
-        }
+      uint32_t mmk = 0, fc = 0, rc = 0;
+      // a group's instructions (past the tape's end: its last)
+      auto fetch = [&](uint32_t g, uint2 &w, uint32_t &mm) {
+        const uint32_t i = min(g * 32u + lane, n_narrow - 1u);
+        w = root.code[i];
+        mm = W.narrow_mm[i];
       };
-      uint2 wn;
-      uint32_t mmn;
-      fetch(tid, wn, mmn);
-      for (uint32_t c0 = 0; c0 < n_narrow; c0 += blockDim.x) {
-        const uint32_t i = c0 + tid;
-        const uint2 w = wn;
-        const uint32_t mm = mmn;
-        fetch(i + blockDim.x, wn, mmn);
-        const bool live = i < n_narrow && flags[i + 4u];
-        const uint32_t bal = __ballot_sync(FULL_MASK, live);
-        if (lane == 0) sh.scan[wib] = __popc(bal);
-        __syncthreads();
-        uint32_t woff = 0, ctot = 0;
-        for (uint32_t q = 0; q < nw; ++q) {
-          const uint32_t v = sh.scan[q];
-          if (q < wib) woff += v;
-          ctot += v;
-        }
-        __syncthreads();  // the counts are read before the next step writes them
-        if (live) {
-          const uint32_t p = base + woff + __popc(bal & ((1u << lane) - 1u));
-          const uint32_t h = TSI_W0_H(w.x);
-          uint2 out = w;
-          uint32_t hk = h;
-          if (TSI_H_IS_MINMAX(h)) {
-            const uint32_t d = (cb[mm >> 4] >> (2u * (mm & 15u))) & 3u;
-            const uint32_t dd = TSI_W0_DST(w.x);
-            if (d & 1u) {
-              out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD), 0u);
-              hk = H_COPY;
-            } else if (d & 2u) {
-              if (TSI_H_IS_II(h)) {
-                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD), 0u);
+      uint2 wq[4];
+      uint32_t mq[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4u; ++u) fetch(wib + u * nw, wq[u], mq[u]);
+#pragma unroll 1
+      for (uint32_t g0 = wib; g0 < groups; g0 += 4u * nw) {
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; ++u) {
+          const uint32_t g = g0 + u * nw;
+          const uint2 w = wq[u];
+          const uint32_t mm = mq[u];
+          fetch(g + 4u * nw, wq[u], mq[u]);
+          const uint32_t i = g * 32u + lane;
+          const bool live = i < n_narrow && flags[i + 4u];
+          const uint32_t bal = __ballot_sync(FULL_MASK, live);
+          if (live) {
+            const uint32_t p = first[g] + __popc(bal & ((1u << lane) - 1u));
+            const uint32_t h = TSI_W0_H(w.x);
+            uint2 out = w;
+            uint32_t hk = h;
+            if (TSI_H_IS_MINMAX(h)) {
+              const uint32_t d = (cb[mm >> 4] >> (2u * (mm & 15u))) & 3u;
+              const uint32_t dd = TSI_W0_DST(w.x);
+              if (d & 1u) {
+                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD), 0u);
                 hk = H_COPY;
+              } else if (d & 2u) {
+                if (TSI_H_IS_II(h)) {
+                  out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD), 0u);
+                  hk = H_COPY;
+                } else {
+                  out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u), w.y);
+                  hk = H_CONST;
+                }
               } else {
-                out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u), w.y);
-                hk = H_CONST;
+                ++mmk;
               }
-            } else {
-              ++mmk;
             }
+            const uint2 cost = sh.cost[hk];
+            fc += cost.x;
+            rc += cost.y;
+            P.code_arena[off + p] = out;
           }
-          fc += c_cost_fwd[hk] + TSI_FIX_COST;
-          rc += c_cost_rr[hk] + TSI_REV_OPERAND_COST * TSI_H_NREG(hk);
-          P.code_arena[off + p] = out;
         }
-        base += ctot;
       }
       atomicAdd(&sh.mmk, mmk);
       atomicAdd(&sh.fcost, fc);
@@ -1151,8 +1183,6 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
   }
   const CellArray<GM> V(cell), G(cell + L.sens);
   uint8_t *dec = cell + L.dec, *dec2 = cell + L.flags;
-  // the cell's and its parent's state, loaded before the bundle table's
-  // copy and barrier so that the loads overlap
   const float4 pxy = pool.box_xy[Pv];
   const float2 pz = pool.box_z[Pv];
   const float pfast = pool.fast[Pv];
@@ -1165,9 +1195,7 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
     c_fast = pool.fast[C];
     c_child = pool.child[C];
   }
-  if (W.nbundles <= kSmemBundles)
-    for (uint32_t i = tid; i < W.nbundles; i += blockDim.x) sh.bt[i] = W.bundles[i];
-  __syncthreads();
+  __syncthreads();  // every thread has read the cell before thread 0 writes it
 
   // ---- cell setup (compute.wgsl:3582-3626), uniform across the block
   const float dx = __fdiv_rn(__fsub_rn(pxy.y, pxy.x), 2.0f);

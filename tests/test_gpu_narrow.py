@@ -111,3 +111,25 @@ def test_directed_narrow_equals_wide(device, parents):
         else:
             for a, b in zip(cells, ref):
                 assert_cells_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("live", [103, 104, 107])
+def test_widest_register_files_run(device, live):
+    """Tapes of 104, 105 and 108 registers: the largest register files that eight
+    warps of a block hold beside their instruction buffers."""
+    b = scenes.IRBuilder()
+    r = b.sub(b.sqrt(b.add(b.add(b.mul(b.X, b.X), b.mul(b.Y, b.Y)), b.mul(b.Z, b.Z))), 1.5)
+    v = [b.add(b.mul(b.X if i % 2 else b.Y, 0.01 * i), 2.0) for i in range(live - 1)]
+    acc = r
+    for x in reversed(v):
+        acc = b.min(acc, b.add(x, b.T))
+    tape = api.IR.new(b.text(acc)).gpu_instructions
+    t = Tape.upload(device, tape)
+    assert t.registers == live + 1
+    p = api.default_params(localsubdiv=4, pruning=0)
+    gs, os_ = Scene(device, t, p), oracle.Scene(tape, p)
+    for time in TIMES[:2]:
+        gs.invert(time)
+        os_.invert(time)
+        assert_cells_equal(gs.cells(), os_.cells())
