@@ -531,9 +531,8 @@ TSI_API void tsi_server_destroy(tsi_server *s);
  * per device (held by every GPU that loads the library until the process
  * exits), and n x (8 x registers + 16 x tape length) bytes must fit in it,
  * else TSI_ERR_BUFFER_TOO_SMALL (split the call).  Nothing in the array needs
- * to start at zero: each launch writes every register and log entry before
- * reading it.  The first call on a device looks up the array's device
- * address (cudaGetSymbolAddress) and loads the evaluation kernel, so make it
+ * to start at zero: each launch writes every log entry before reading it.  The first call on a device looks up the array's device
+ * address (cudaGetSymbolAddress) and loads the evaluation kernels, so make it
  * before any stream capture.  The call makes the tape's device current and
  * puts the caller's current device back before it returns.  All calls share
  * the one array per device: calls that can overlap on the GPU (different

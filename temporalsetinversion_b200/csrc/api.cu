@@ -31,9 +31,6 @@
 #include "tsi.h"
 
 namespace tsi {
-cudaError_t launch_evalbox(bool directed, const uint2 *code, uint32_t len, uint32_t nregs, uint32_t out_reg,
-                           uint32_t n, const float *boxes, int reverse, float *out, float2 *regs, float4 *log,
-                           cudaStream_t st);
 cudaError_t launch_math(int which, uint32_t n, const float *a, const float *b, float *out, cudaStream_t st);
 }  // namespace tsi
 
@@ -164,6 +161,34 @@ uint32_t tree_levels(const tsi_params &p) {
   return std::max(1u, l);
 }
 
+// The tape's bundled form (its members without a tape's part: zero).
+WideDev wide_dev(const tsi_tape *t) {
+  WideDev W{};
+  W.fwd = t->d_wfwd;
+  W.rev = t->d_wrev;
+  W.rev16 = t->d_wrev16;
+  W.live = t->d_wlive;
+  W.bundles = t->d_wbundles;
+  W.narrow_mm = t->d_wmm;
+  W.rev_slots = t->wrev_slots;
+  W.ctl = t->d_wctl;
+  W.streams = t->d_wstreams;
+  W.nbundles = t->wbundles;
+  W.nvalues = t->wvalues;
+  // a tape without a bundled form never sends a cell to the wide path,
+  // whatever thresholds were set on it
+  const bool has_wide = t->d_wfwd != nullptr && t->wbundles > 0;
+  W.min_len = has_wide ? t->wmin_len : 0xffffffffu;
+  W.deep_level = t->wdeep_level;
+  W.deep_min_len = has_wide ? t->wdeep_min_len : 0xffffffffu;
+  W.ncontrib = t->wcontrib;
+  for (int q = 0; q < 4; ++q) {
+    W.arg_gbase[q] = t->warg_gbase[q];
+    W.arg_gcount[q] = t->warg_gcount[q];
+  }
+  return W;
+}
+
 void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool wide_global, SceneLaunch &L,
                  TapeRec &R) {
   const tsi_params &p = s->p;
@@ -187,30 +212,9 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
   L.levels = tree_levels(p);
   L.full_len = s->tape->len;
   L.narrow_parents = s->tape->narrow_parents;
-  L.wide.fwd = s->tape->d_wfwd;
-  L.wide.rev = s->tape->d_wrev;
-  L.wide.rev16 = s->tape->d_wrev16;
-  L.wide.live = s->tape->d_wlive;
-  L.wide.bundles = s->tape->d_wbundles;
-  L.wide.narrow_mm = s->tape->d_wmm;
-  L.wide.rev_slots = s->tape->wrev_slots;
-  L.wide.ctl = s->tape->d_wctl;
-  L.wide.streams = s->tape->d_wstreams;
-  L.wide.nbundles = s->tape->wbundles;
-  L.wide.nvalues = s->tape->wvalues;
-  // a tape without a bundled form never sends a cell to the wide path,
-  // whatever thresholds were set on it
-  const bool has_wide = s->tape->d_wfwd != nullptr && s->tape->wbundles > 0;
-  L.wide.min_len = has_wide ? s->tape->wmin_len : 0xffffffffu;
-  L.wide.deep_level = s->tape->wdeep_level;
-  L.wide.deep_min_len = has_wide ? s->tape->wdeep_min_len : 0xffffffffu;
-  L.wide.ncontrib = s->tape->wcontrib;
+  L.wide = wide_dev(s->tape);
   L.wide.prune_level = s->tape->wprune_level != 0xffffffffu ? s->tape->wprune_level : tree_levels(p) / 2u;
   L.wide.global = wide_global ? 1u : 0u;
-  for (int q = 0; q < 4; ++q) {
-    L.wide.arg_gbase[q] = s->tape->warg_gbase[q];
-    L.wide.arg_gcount[q] = s->tape->warg_gcount[q];
-  }
   R.code = s->tape->d_code;
   R.len = s->tape->len;
   R.nregs = s->tape->nregs;
@@ -1149,9 +1153,8 @@ TSI_API tsi_status tsi_tape_eval_boxes(tsi_ctx *c, const tsi_tape *t, uint32_t n
   if (!c || !t || (!boxes && n) || (!out && n)) return set_err(TSI_ERR_INVALID_ARGUMENT, "null argument");
   if (n == 0) return TSI_OK;
   CK(cudaSetDevice(c->device));
-  const size_t nb = (size_t)n * 8 * 4, no = (size_t)n * 10 * 4;
-  const size_t nr = (size_t)n * t->nregs * 8, nl = (size_t)n * std::max<uint32_t>(t->len, 1u) * 16;
-  const size_t need = nb + no + nr + nl + 1024;
+  const size_t nb = ((size_t)n * 8 * 4 + 255) & ~(size_t)255, no = ((size_t)n * 10 * 4 + 255) & ~(size_t)255;
+  const size_t need = nb + no + (reverse ? evalbox_log_bytes(n, t->len) : 0);
   if (need > c->scratch_bytes) {
     cudaFree(c->d_scratch);
     c->d_scratch = nullptr;
@@ -1161,13 +1164,14 @@ TSI_API tsi_status tsi_tape_eval_boxes(tsi_ctx *c, const tsi_tape *t, uint32_t n
   }
   char *base = (char *)c->d_scratch;
   float *d_boxes = (float *)base;
-  float *d_out = (float *)(base + ((nb + 255) & ~(size_t)255));
-  float2 *d_regs = (float2 *)(base + ((nb + 255) & ~(size_t)255) + ((no + 255) & ~(size_t)255));
-  float4 *d_log = (float4 *)((char *)d_regs + ((nr + 255) & ~(size_t)255));
-  CK(cudaMemcpyAsync(d_boxes, boxes, nb, cudaMemcpyHostToDevice, c->stream));
-  CK(launch_evalbox(rounding_mode == TSI_ROUND_DIRECTED, t->d_code, t->len, t->nregs, t->out_reg, n, d_boxes, reverse,
-                    d_out, d_regs, d_log, c->stream));
-  CK(cudaMemcpyAsync(out, d_out, no, cudaMemcpyDeviceToHost, c->stream));
+  float *d_out = (float *)(base + nb);
+  float4 *d_log = (float4 *)(base + nb + no);
+  TsiTapeView v;
+  tsi_internal_tape_view(t, &v);
+  CK(evalbox_preload());
+  CK(cudaMemcpyAsync(d_boxes, boxes, (size_t)n * 8 * 4, cudaMemcpyHostToDevice, c->stream));
+  CK(launch_evalbox(rounding_mode == TSI_ROUND_DIRECTED, v.tape, n, d_boxes, reverse != 0, d_out, d_log, c->stream));
+  CK(cudaMemcpyAsync(out, d_out, (size_t)n * 10 * 4, cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return TSI_OK;
 }
@@ -1177,10 +1181,12 @@ TSI_API tsi_status tsi_tape_eval_boxes(tsi_ctx *c, const tsi_tape *t, uint32_t n
 // Internal view of a tape for the library's other translation units.
 tsi_status tsi_internal_tape_view(const tsi_tape *t, TsiTapeView *v) {
   if (!t || !v || !t->ctx) return set_err(TSI_ERR_INVALID_ARGUMENT, "null argument");
-  v->code = t->d_code;
-  v->len = t->len;
-  v->nregs = t->nregs;
-  v->out_reg = t->out_reg;
+  v->tape.code = t->d_code;
+  v->tape.len = t->len;
+  v->tape.nregs = t->nregs;
+  v->tape.out_reg = t->out_reg;
+  v->tape.wide = wide_dev(t);
+  v->tape.sm_count = t->ctx->sm_count;
   v->device = t->ctx->device;
   v->stream = t->ctx->stream;
   return TSI_OK;

@@ -4,11 +4,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "evalbox.h"
 #include "tsi.h"
 
 struct TsiTapeView {
-  const uint2 *code;
-  uint32_t len, nregs, out_reg;
+  tsi::EvalTape tape;
   int device;
   cudaStream_t stream;
 };

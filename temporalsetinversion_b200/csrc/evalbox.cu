@@ -2,91 +2,95 @@
 //
 // The body of compute.wgsl:3632-3970 without the octree: forward tape,
 // reverse interval AD seeded with 1 at the output, sensitivities of the four
-// arguments.  One thread per box, registers and the operand log in global
-// scratch.  Used by tsi_tape_eval_boxes (op-level parity tests).
+// arguments, by the interpreters of the refinement kernel.  With one thread
+// per box, registers and log in global memory, every tape instruction waited
+// for its operands from L2.
+//
+// Many boxes: a warp per 32 of them (narrow_interp.cuh), bound by the
+// instructions it issues per tape instruction.  Few boxes on a long tape: a
+// block per box (wide_interp.cuh), bound by the latency of a bundle's step.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
+#include "evalbox.h"
 #include "interval.cuh"
+#include "narrow_interp.cuh"
+#include "wide_interp.cuh"
 
 namespace tsi {
 
-template <bool D>
-__global__ void evalbox_kernel(const uint2 *code, uint32_t len, uint32_t nregs, uint32_t out_reg, uint32_t n,
-                               const float *boxes, int reverse, float *out, float2 *regs, float4 *log) {
-  using A = IA<D>;
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float2 *R = regs + (size_t)i * nregs;
-  float4 *L = log + (size_t)i * len;
-  const float *b = boxes + (size_t)i * 8;
-  for (int q = 0; q < 4; ++q) R[q] = make_float2(b[2 * q], b[2 * q + 1]);
-  for (uint32_t j = 0; j < len; ++j) {
-    const uint2 w = code[j];
-    const uint32_t h = TSI_W0_H(w.x);
-    const float lit = __uint_as_float(w.y);
-    const float2 a = R[TSI_W0_A(w.x)];
-    const Iv Av = Iv{a.x, a.y};
-    Iv Bv = iv(lit);
-    if (TSI_H_IS_II(h)) {
-      const float2 bb = R[w.y & 255u];
-      Bv = Iv{bb.x, bb.y};
-    }
-    L[j] = make_float4(Av.lo, Av.hi, Bv.lo, Bv.hi);
-    const Iv r = A::forward(h, Av, Bv, lit);
-    R[TSI_W0_DST(w.x)] = make_float2(r.lo, r.hi);
-  }
-  float *o = out + (size_t)i * 10;
-  const float2 f = R[out_reg];
-  o[0] = f.x;
-  o[1] = f.y;
-  for (int q = 2; q < 10; ++q) o[q] = 0.0f;
-  if (!reverse) return;
-  for (uint32_t r = 0; r < nregs; ++r) R[r] = make_float2(0.0f, 0.0f);
-  R[out_reg] = make_float2(1.0f, 1.0f);
-  for (int j = (int)len - 1; j >= 0; --j) {
-    const uint2 w = code[j];
-    const uint32_t h = TSI_W0_H(w.x);
-    const uint32_t d = TSI_W0_DST(w.x), a = TSI_W0_A(w.x), bq = w.y & 255u;
-    const float lit = __uint_as_float(w.y);
-    const float4 lg = L[j];
-    const Iv Av = Iv{lg.x, lg.y}, Bv = Iv{lg.z, lg.w};
-    const float2 sv = R[d];
-    const Iv s = Iv{sv.x, sv.y};
-    R[d] = make_float2(0.0f, 0.0f);
-    if (h == H_CONST) continue;
-    const bool s0 = (s.lo == 0.0f && s.hi == 0.0f);
-    if (TSI_H_IS_II(h)) {
-      if (s0 && TSI_W0_FA(w.x) && TSI_W0_FB(w.x)) {
-        R[a] = make_float2(0.0f, 0.0f);
-        R[bq] = make_float2(0.0f, 0.0f);
-      } else {
-        Iv r0, r1;
-        A::reverse_rule(h, Av, Bv, lit, r0, r1);
-        r0 = A::mul(A::fix(r0), s);
-        r1 = A::mul(A::fix(r1), s);
-        const float2 pa = R[a], pb = R[bq];
-        const Iv n0 = A::add(r0, Iv{pa.x, pa.y});
-        const Iv n1 = A::add(r1, Iv{pb.x, pb.y});
-        R[a] = make_float2(n0.lo, n0.hi);
-        R[bq] = make_float2(n1.lo, n1.hi);
-      }
-    } else {
-      if (s0 && TSI_W0_FA(w.x)) {
-        R[a] = make_float2(0.0f, 0.0f);
-      } else {
-        Iv r0, r1;
-        A::reverse_rule(h, Av, Bv, lit, r0, r1);
-        r0 = A::mul(A::fix(r0), s);
-        const float2 pa = R[a];
-        const Iv n0 = A::add(r0, Iv{pa.x, pa.y});
-        R[a] = make_float2(n0.lo, n0.hi);
-      }
-    }
-  }
+// Shared memory of a block: the boxes' register rows and the instruction
+// buffer, or a cell's values and sensitivities.
+extern __shared__ __align__(16) unsigned char evalbox_smem[];
+
+__device__ __forceinline__ void load_box(const float *b, Iv v[4]) {
+  for (int q = 0; q < 4; ++q) v[q] = Iv{b[2 * q], b[2 * q + 1]};
+}
+__device__ __forceinline__ void store_box(float *o, Iv f, const Iv sens[4]) {
+  o[0] = f.lo;
+  o[1] = f.hi;
   for (int q = 0; q < 4; ++q) {
-    o[2 + 2 * q] = R[q].x;
-    o[3 + 2 * q] = R[q].y;
+    o[2 + 2 * q] = sens[q].lo;
+    o[3 + 2 * q] = sens[q].hi;
+  }
+}
+
+// Boxes a warp takes: a row's offset has 16 bits, the sink's included.
+inline __host__ __device__ uint32_t narrow_boxes(uint32_t nregs) { return nregs < 256u ? 32u : 16u; }
+inline size_t narrow_bytes(uint32_t nregs) {
+  return ((size_t)(nregs + 1u) * narrow_boxes(nregs) * 8u + 15u & ~size_t(15)) + 32u * 16u;
+}
+
+// One warp, up to 32 boxes; the rows have exactly as many columns, and the
+// lanes without a box repeat the last one (they write what its lane writes).
+// 60000 boxes on a 4697-instruction tape with sensitivities: a call takes
+// 12.8 ms with a thread per box, 2.5 ms so.
+template <bool D>
+__global__ void __launch_bounds__(32) evalbox_narrow(EvalTape T, uint32_t n, const float *__restrict__ boxes,
+                                                     int reverse, float *__restrict__ out, float4 *log) {
+  const uint32_t lane = threadIdx.x, per = narrow_boxes(T.nregs);
+  const size_t first = (size_t)blockIdx.x * per;
+  const uint32_t cols = (uint32_t)min((size_t)per, (size_t)n - first);
+  NarrowRows R;
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(evalbox_smem);
+  R.stride = cols * 8u;
+  R.col = min(lane, cols - 1u);
+  R.rf = base + R.col * 8u;
+  R.sink = T.nregs * R.stride;
+  R.prog = base + ((R.sink + R.stride + 15u) & ~15u);
+  const size_t box = first + R.col;
+  Iv v[4], sens[4] = {iv(0.0f), iv(0.0f), iv(0.0f), iv(0.0f)};
+  load_box(boxes + box * 8u, v);
+  float4 *lg = reverse ? log + first * max(T.len, 1u) : nullptr;  // `cols` columns of at most len entries
+  uint32_t nlog = 0;
+  const Iv f = narrow_forward<D>(T.code, T.len, T.out_reg, R, lane, v[0], v[1], v[2], v[3], lg, nullptr, nlog);
+  if (reverse) {
+    bool bad = false;
+    narrow_reverse<D>(T.code, T.len, T.nregs, T.out_reg, R, lane, lg, nlog, true, sens, bad);
+  }
+  if (lane < cols) store_box(out + box * 10u, f, sens);
+}
+
+// One block per box at a time, on the bundled form.  511 boxes on a
+// 1177-instruction tape, without sensitivities: a call takes 371 us with a
+// thread per box, 164 with a warp per 32, 53 so (39 of them with one box).
+template <bool D>
+__global__ void __launch_bounds__(256) evalbox_wide(EvalTape T, uint32_t n, const float *__restrict__ boxes,
+                                                    int reverse, float *__restrict__ out) {
+  __shared__ float2 s_sens[4];
+  const CellArray<false> V(evalbox_smem), G(evalbox_smem + (T.wide.nvalues + 2u) * 8u);
+  for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
+    Iv v[4], sens[4] = {iv(0.0f), iv(0.0f), iv(0.0f), iv(0.0f)};
+    load_box(boxes + (size_t)i * 8u, v);
+    const Iv f = cell_forward<D, false>(T.wide, V, G, false, nullptr, nullptr, v[0], v[1], v[2], v[3], v[3]);
+    if (reverse) {
+      cell_reverse<D, false>(T.wide, V, G, s_sens);
+      for (int q = 0; q < 4; ++q) sens[q] = Iv{s_sens[q].x, s_sens[q].y};
+    }
+    if (threadIdx.x == 0) store_box(out + (size_t)i * 10u, f, sens);
+    __syncthreads();  // the field and the sensitivities are read before the next box writes its values
   }
 }
 
@@ -110,24 +114,55 @@ __global__ void math_kernel(int which, uint32_t n, const float *a, const float *
   out[i] = r;
 }
 
-cudaError_t launch_evalbox(bool directed, const uint2 *code, uint32_t len, uint32_t nregs, uint32_t out_reg,
-                           uint32_t n, const float *boxes, int reverse, float *out, float2 *regs, float4 *log,
-                           cudaStream_t st) {
-  const int block = 128;
-  const int grid = (int)((n + block - 1) / block);
-  if (directed)
-    evalbox_kernel<true><<<grid, block, 0, st>>>(code, len, nregs, out_reg, n, boxes, reverse, out, regs, log);
-  else
-    evalbox_kernel<false><<<grid, block, 0, st>>>(code, len, nregs, out_reg, n, boxes, reverse, out, regs, log);
+// Most dynamic shared memory the kernels are launched with.
+constexpr size_t kNarrowMax = 66u << 10, kWideMax = 200u << 10;
+
+template <bool D>
+static cudaError_t launch(const EvalTape &t, uint32_t n, const float *boxes, bool reverse, float *out, float4 *log,
+                          cudaStream_t st) {
+  const WideDev &W = t.wide;
+  const size_t wide = ((size_t)W.nvalues + 2u) * 8u * (reverse ? 2u : 1u) + (reverse ? (size_t)W.ncontrib * 8u : 0u);
+  if (W.nbundles && wide <= kWideMax && (!reverse || W.rev16)) {
+    int bps = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, evalbox_wide<D>, 256, wide);
+    if (e != cudaSuccess) return e;
+    const uint64_t grid = (uint64_t)bps * t.sm_count, waves = grid ? (n + grid - 1) / grid : 0;
+    // A wave of blocks takes as long as four to five instructions per bundle
+    // of the narrow form.  Both ways in microseconds (forward, reverse): 277
+    // instructions in 27 bundles, 2000 boxes 100, 137 against 112, 148; 20000
+    // boxes 418, 699 against 266, 306.  4697 in 34, 20000 boxes 619, 2080
+    // against 765, 1923; 60000 boxes 1658, 6035 against 1224, 2541.
+    if (waves && t.len >= 4u * (uint64_t)W.nbundles * waves) {
+      evalbox_wide<D><<<(unsigned)(n < grid ? n : grid), 256, wide, st>>>(t, n, boxes, reverse, out);
+      return cudaGetLastError();
+    }
+  }
+  const uint32_t per = narrow_boxes(t.nregs);
+  evalbox_narrow<D><<<(n + per - 1u) / per, 32, narrow_bytes(t.nregs), st>>>(t, n, boxes, reverse, out, log);
   return cudaGetLastError();
 }
 
-// Loads both instances of the box kernel on the current device (module
-// loading is lazy, so without this the first launch of each would load it).
+cudaError_t launch_evalbox(bool directed, const EvalTape &t, uint32_t n, const float *boxes, bool reverse, float *out,
+                           float4 *log, cudaStream_t st) {
+  return directed ? launch<true>(t, n, boxes, reverse, out, log, st) : launch<false>(t, n, boxes, reverse, out, log, st);
+}
+
 cudaError_t evalbox_preload() {
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, evalbox_kernel<true>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, evalbox_kernel<false>);
+  static std::mutex mu;
+  static bool done[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  auto limit = [](auto *kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  e = limit(evalbox_narrow<true>, kNarrowMax);
+  if (e == cudaSuccess) e = limit(evalbox_narrow<false>, kNarrowMax);
+  if (e == cudaSuccess) e = limit(evalbox_wide<true>, kWideMax);
+  if (e == cudaSuccess) e = limit(evalbox_wide<false>, kWideMax);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
   return e;
 }
 

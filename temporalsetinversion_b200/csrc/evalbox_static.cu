@@ -1,8 +1,7 @@
 // evalbox_static.cu — tsi_tape_eval_boxes_static: interval evaluation of a
 // tape on device-resident boxes without allocating anything.
 //
-// tsi_tape_eval_boxes allocates device scratch (one interval register file
-// and one operand log per box) with cudaMalloc on first use and whenever a
+// tsi_tape_eval_boxes allocates device scratch (an operand log per box) with cudaMalloc on first use and whenever a
 // call needs more.  Some callers cannot allocate at call time: a render loop
 // recorded into a CUDA graph, a host with a fixed memory budget that
 // reserves everything at start-up, or an embedding runtime that forbids
@@ -10,26 +9,19 @@
 // for the boxes and the output and keeps its scratch in the file-scope
 // array below, which exists once per device that loads the library and stays
 // allocated until the process exits.  Nothing in it needs to start at zero:
-// the kernel writes every register and log entry before reading it.
+// the kernel writes every log entry before reading it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <mutex>
 
 #include "api_internal.h"
-#include "interval.cuh"
+#include "evalbox.h"
 #include "tsi.h"
 
-namespace tsi {
-cudaError_t launch_evalbox(bool directed, const uint2 *code, uint32_t len, uint32_t nregs, uint32_t out_reg,
-                           uint32_t n, const float *boxes, int reverse, float *out, float2 *regs, float4 *log,
-                           cudaStream_t st);
-cudaError_t evalbox_preload();
-}
-
-
-// Scratch of every call: per box, nregs intervals (8 bytes each) then
-// len operand-log entries (16 bytes each), boxes back to back.
+// Scratch of every call: len operand-log entries (16 bytes each) per box.
+// (The call's limit counts nregs intervals of 8 bytes per box too, as the
+// header states; the registers themselves are in shared memory.)
 static __device__ __align__(256) unsigned char g_static_scratch[TSI_STATIC_SCRATCH_BYTES];
 
 namespace {
@@ -39,7 +31,7 @@ std::mutex g_mu;
 void *g_scratch_addr[kMaxDevices];  // device address of g_static_scratch, per device
 
 // Set-up, once per device, with that device current: the array's device
-// address, and both instances of the box kernel loaded (module loading is
+// address, and the box kernels loaded (module loading is
 // lazy), so that later calls load nothing.
 tsi_status scratch_address(int device, void **out) {
   if (device < 0 || device >= kMaxDevices) return TSI_ERR_INVALID_ARGUMENT;
@@ -74,8 +66,8 @@ extern "C" TSI_API tsi_status tsi_tape_eval_boxes_static(const tsi_tape *tape, u
     tsi_internal_set_error("tsi_tape_eval_boxes_static: null device pointer");
     return TSI_ERR_INVALID_ARGUMENT;
   }
-  const uint64_t regs_bytes = ((uint64_t)n * v.nregs * 8u + 255u) & ~255ull;
-  const uint64_t log_bytes = (uint64_t)n * (v.len ? v.len : 1u) * 16u;
+  const uint64_t regs_bytes = ((uint64_t)n * v.tape.nregs * 8u + 255u) & ~255ull;
+  const uint64_t log_bytes = tsi::evalbox_log_bytes(n, v.tape.len);
   if (regs_bytes + log_bytes > TSI_STATIC_SCRATCH_BYTES) {
     tsi_internal_set_error("tsi_tape_eval_boxes_static: n boxes x (registers + tape length) exceeds the "
                            "static scratch of TSI_STATIC_SCRATCH_BYTES; split the call");
@@ -93,11 +85,9 @@ extern "C" TSI_API tsi_status tsi_tape_eval_boxes_static(const tsi_tape *tape, u
   void *base = nullptr;
   st = scratch_address(v.device, &base);
   if (st == TSI_OK) {
-    float2 *regs = (float2 *)base;
-    float4 *log = (float4 *)((unsigned char *)base + regs_bytes);
     cudaStream_t s = cuda_stream ? (cudaStream_t)cuda_stream : v.stream;
-    const cudaError_t e = tsi::launch_evalbox(rounding_mode == TSI_ROUND_DIRECTED, v.code, v.len, v.nregs, v.out_reg,
-                                              n, boxes_dev, reverse, out_dev, regs, log, s);
+    const cudaError_t e = tsi::launch_evalbox(rounding_mode == TSI_ROUND_DIRECTED, v.tape, n, boxes_dev, reverse != 0,
+                                              out_dev, (float4 *)base, s);
     if (e != cudaSuccess) {
       tsi_internal_set_error(cudaGetErrorString(e));
       st = TSI_ERR_CUDA;
