@@ -33,13 +33,16 @@ __device__ __forceinline__ uint32_t pcg_word(uint32_t s) {
   uint32_t w = ((s >> ((s >> 28u) + 4u)) ^ s) * 277803737u;
   return (w >> 22u) ^ w;
 }
+// the reference divides by 4294967295.0, which is 2^32 as an f32: the product
+// with its reciprocal is the same number
+constexpr float kInv2p32 = 2.3283064365386963e-10f;
 __device__ __forceinline__ float frand(uint32_t &seed) {  // -1 to 1
   seed = seed * 747796405u + 1u;
-  return __fsub_rn(__fmul_rn(__fdiv_rn(__uint2float_rn(pcg_word(seed)), 4294967295.0f), 2.0f), 1.0f);
+  return __fsub_rn(__fmul_rn(__fmul_rn(__uint2float_rn(pcg_word(seed)), kInv2p32), 2.0f), 1.0f);
 }
 __device__ __forceinline__ float frand0to1(uint32_t &seed) {
   seed = seed * 747796405u + 1u;
-  return __fdiv_rn(__uint2float_rn(pcg_word(seed)), 4294967295.0f);
+  return __fmul_rn(__uint2float_rn(pcg_word(seed)), kInv2p32);
 }
 
 __device__ __forceinline__ float dot3(F3 a, F3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
@@ -74,27 +77,46 @@ __device__ F3 sample_biased(F3 d, float power, uint32_t &seed) {  // getSampleBi
   return (muls(o1, fm_cos(rx) * oneminus) + muls(o2, fm_sin(rx) * oneminus)) + muls(dir, ry);
 }
 
-// sunsky (520-677) with turbidity 1, sunSize 1 and the sky's sun intensity
-// 1000 (the private globals of 421-427); it returns 0.01 * sky.  pow with the
-// constant exponent 2.0 is x * x, the rewrite shader compilers apply; it is
-// defined for the negative cosines between view and sun.
-__device__ F3 sunsky(F3 view, float spx, float spy) {
-  const float pi = 3.1415927410125732f;
-  const float sun_cos = fm_cos((1.0f * pi) / 180.0f);
-  const F3 sun_dir = normalize3(from_spherical((spx - 0.0f) * 6.28000020980835f, (spy - 0.5f) * 3.140000104904175f));
-  const float cos_view_sun = dot3(view, sun_dir);
-  const float cos_sun_up = dot3(sun_dir, f3(0.0f, 0.0f, 1.0f));
-  const float cos_up_view = dot3(f3(0.0f, 0.0f, 1.0f), view);
-  if (sun_cos == 1.0f) return f3(1.0f, 0.0f, 0.0f);
-  const float sunE = 1000.0f * fm_max(0.0f, 1.0f - fm_exp(-((1.6110731611233942f - fm_acos(cos_sun_up)) / 1.5f)));
-  const F3 rayleigh = f3(5.176821105123963e-6f, 1.2785348189936485e-5f, 2.8530756026157178e-5f);
+// What sunsky (520-677) and the shadow rays derive from the sun's position
+// alone: the same for every ray, so each block works it out once.
+struct Sky {
+  F3 sun_dir;  // sunsky's sun direction
+  F3 shadow;   // the direction of the shadow rays (4482-4484)
+  F3 mie;
+  float sunE, t;
+};
+
+__device__ Sky sky_of(float spx, float spy) {
+  Sky k;
+  k.sun_dir = normalize3(from_spherical((spx - 0.0f) * 6.28000020980835f, (spy - 0.5f) * 3.140000104904175f));
+  const F3 sd = normalize3(from_spherical((spx - 0.0f) * 6.28f, (spy - 0.5f) * 3.14f));
+  k.shadow = f3(sd.x, sd.z, sd.y);
+  const float cos_sun_up = dot3(k.sun_dir, f3(0.0f, 0.0f, 1.0f));
+  k.sunE = 1000.0f * fm_max(0.0f, 1.0f - fm_exp(-((1.6110731611233942f - fm_acos(cos_sun_up)) / 1.5f)));
   const float c = (0.20000000298023224f * 1.0f) * 9.99999983775159e-18f;  // totalMie 438-456, T = 1
   const F3 lambda = f3(6.800000278417428e-7f, 5.499999815583578e-7f, 4.4999998749517545e-7f);
   const F3 K = f3(0.6859999895095825f, 0.6779999732971191f, 0.6660000085830688f);
   const float two_pi = 2.0f * 3.1415927410125732f;
   const F3 q = f3(two_pi, two_pi, two_pi) / lambda;  // pow(q, vec3(4.0 - 2.0)) = q * q
   const F3 tm = muls(q * q, (0.4339999854564667f * c) * 3.1415927410125732f) * K;
-  const F3 mie = muls(tm, 0.004999999888241291f);
+  k.mie = muls(tm, 0.004999999888241291f);
+  k.t = clampf(fm_powf(1.0f - dot3(f3(0.0f, 0.0f, 1.0f), k.sun_dir), 5.0f), 0.0f, 1.0f);
+  return k;
+}
+
+// sunsky (520-677) with turbidity 1, sunSize 1 and the sky's sun intensity
+// 1000 (the private globals of 421-427); it returns 0.01 * sky.  pow with the
+// constant exponent 2.0 is x * x, the rewrite shader compilers apply; it is
+// defined for the negative cosines between view and sun.
+__device__ F3 sunsky(F3 view, const Sky &k) {
+  const float pi = 3.1415927410125732f;
+  const float sun_cos = fm_cos((1.0f * pi) / 180.0f);
+  const float cos_view_sun = dot3(view, k.sun_dir);
+  const float cos_up_view = dot3(f3(0.0f, 0.0f, 1.0f), view);
+  if (sun_cos == 1.0f) return f3(1.0f, 0.0f, 0.0f);
+  const float sunE = k.sunE;
+  const F3 rayleigh = f3(5.176821105123963e-6f, 1.2785348189936485e-5f, 2.8530756026157178e-5f);
+  const F3 mie = k.mie;
   const float zenith = fm_max(0.0f, cos_up_view);
   const float r_len = 8400.0f / zenith, m_len = 1250.0f / zenith;
   const F3 fex = f3(fm_exp(-(rayleigh.x * r_len + mie.x * m_len)), fm_exp(-(rayleigh.y * r_len + mie.y * m_len)),
@@ -107,7 +129,7 @@ __device__ F3 sunsky(F3 view, float spx, float spy) {
   const F3 total = rayleigh + mie, light = r_eye + m_eye;
   const F3 se = muls(light / total, sunE);
   F3 sky = se * (f3(1.0f, 1.0f, 1.0f) - fex);
-  const float t = clampf(fm_powf(1.0f - dot3(f3(0.0f, 0.0f, 1.0f), sun_dir), 5.0f), 0.0f, 1.0f);
+  const float t = k.t;
   const F3 pw = pow3(se * fex, f3(0.5f, 0.5f, 0.5f));
   const F3 mx = f3(1.0f * (1.0f - t) + pw.x * t, 1.0f * (1.0f - t) + pw.y * t, 1.0f * (1.0f - t) + pw.z * t);
   sky = sky * mx;
@@ -150,16 +172,28 @@ __device__ __forceinline__ Sun scene_sun(int32_t scene) {  // 4449-4471
 
 }  // namespace
 
+// The image takes as long as its slowest warp: one thread works through a
+// pixel's samples, whose random numbers begin where the sample before left
+// off.  Per block of four warps, as in trace.cu; what depends on the sun
+// alone once per block.  640x360, 8 samples, 16 spheres: 6.3 ms with the
+// interval interpreter's normals, 3.4 with point_tape.cuh's, 2.9 with the sky
+// shared; a half warp for the path rays and the other for the shadow rays
+// takes 2.7 at 1.6 times the instructions, 3 or 4 blocks of eight warps per SM
+// 3.5 and 4.4.
 template <bool FAST>
-__global__ void __launch_bounds__(256, 2) cinematic_kernel(const TraceParams *__restrict__ Tp) {
+__global__ void __launch_bounds__(128, 4) cinematic_kernel(const TraceParams *__restrict__ Tp) {
   const TraceParams &T = *Tp;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t px = blockIdx.x * 32u + (warp & 3u) * 8u + (lane & 7u);
-  const uint32_t py = blockIdx.y * 8u + (warp >> 2) * 4u + (lane >> 3);
+  const uint32_t px = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
+  const uint32_t py = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);
   const bool valid = px < T.W && py < T.H;
   const uint64_t pix = (uint64_t)py * T.W + px;
   const F3 eye = f3(T.eye[0], T.eye[1], T.eye[2]);
   const Sun sun = scene_sun(T.scene_id);
+  __shared__ Sky s_sky;
+  if (threadIdx.x == 0) s_sky = sky_of(sun.spx, sun.spy);
+  __syncthreads();
+  const Sky &sky_k = s_sky;
   // seed3 of rt_main (4664)
   uint32_t seed = (uint32_t)pix + (uint32_t)(12345.0f * (fm_sin(T.time * 12345.0f) * 0.5f + 0.5f));
   float acc_r = 0.0f, acc_g = 0.0f, acc_b = 0.0f, acc_a = 0.0f, d0 = -1.0f;
@@ -186,7 +220,7 @@ __global__ void __launch_bounds__(256, 2) cinematic_kernel(const TraceParams *__
       if (active) walk_octree<true>(T, frm, dir, rcp3(dir), w);
       if (FAST) {
         if (__any_sync(0xffffffffu, active && w.hit)) {
-          const F3 n = tape_normal(T, lane, warp, w.end, w.tnorm);
+          const F3 n = tape_normal(T, lane, warp, w.end, w.tnorm, active && w.hit);
           if (active && w.hit) w.nrm = n;
         }
       }
@@ -205,8 +239,7 @@ __global__ void __launch_bounds__(256, 2) cinematic_kernel(const TraceParams *__
         dir = sample_biased(n, 3.0f, seed);
         lum = muls(lum * sc, sun.albedo);
         frm = hitpoint + muls(n, 0.05f);
-        const F3 sd = normalize3(from_spherical((sun.spx - 0.0f) * 6.28f, (sun.spy - 0.5f) * 3.14f));
-        const F3 sundir = f3(sd.x, sd.z, sd.y);
+        const F3 sundir = sky_k.shadow;
         const float jx = frand(seed), jy = frand(seed), jz = frand(seed);
         const F3 sample_dir = normalize3(sundir + muls(f3(jx, jy, jz), sun.size));
         const float sunlight = dot3(n, sample_dir);
@@ -224,7 +257,7 @@ __global__ void __launch_bounds__(256, 2) cinematic_kernel(const TraceParams *__
           out_r = out_g = out_b = 10.0f;
           out_a = 0.0f;
         } else {
-          const F3 sky = sunsky(f3(dir.x, dir.z, dir.y), sun.spx, sun.spy);  // getBackground 4440-4442
+          const F3 sky = sunsky(f3(dir.x, dir.z, dir.y), sky_k);  // getBackground 4440-4442
           const F3 cc = direct + lum * sky;
           out_r = cc.x * sun.bg;
           out_g = cc.y * sun.bg;
@@ -258,7 +291,8 @@ __global__ void __launch_bounds__(256, 2) cinematic_kernel(const TraceParams *__
   }
 }
 
-cudaError_t launch_cinematic(const TraceParams &T, const TraceParams *Tdev, size_t smem, cudaStream_t st) {
+cudaError_t launch_cinematic(const TraceParams &T, const TraceParams *Tdev, cudaStream_t st) {
+  const size_t smem = T.code ? (size_t)4 * normal_bytes(T.nregs) : 0;
   if (smem > (48u << 10)) {  // the attribute is per kernel and device: only ever raise it
     static std::mutex mu;
     static size_t set_bytes[64] = {0};
@@ -272,8 +306,8 @@ cudaError_t launch_cinematic(const TraceParams &T, const TraceParams *Tdev, size
       if (dev >= 0 && dev < 64) set_bytes[dev] = smem;
     }
   }
-  dim3 block(256);
-  dim3 grid((T.W + 31) / 32, (T.H + 7) / 8);
+  dim3 block(128);
+  dim3 grid((T.W + 15) / 16, (T.H + 7) / 8);
   if (T.code) cinematic_kernel<true><<<grid, block, smem, st>>>(Tdev);
   else cinematic_kernel<false><<<grid, block, 0, st>>>(Tdev);
   return cudaGetLastError();

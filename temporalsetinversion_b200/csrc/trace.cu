@@ -19,16 +19,21 @@
 
 namespace tsi {
 
+constexpr uint32_t kTraceWarps = 4;  // of a block
+
 // FAST: normals by finite differences of the tape (a separate instance, so
 // the plain tracer carries no point-evaluation code).
 template <bool FAST>
-__global__ void __launch_bounds__(256, 4) trace_kernel(const TraceParams *__restrict__ Tp) {
+__global__ void __launch_bounds__(32 * kTraceWarps, 32 / kTraceWarps) trace_kernel(const TraceParams *__restrict__ Tp) {
   const TraceParams &T = *Tp;
-  // a block covers a 32x8 pixel tile and each warp a 4x8 column of it, so
+  // a block covers a 16x8 pixel tile and each warp a 4x8 column of it, so
   // the rays of a warp are close together and walk similar nodes (8x4 and
-  // 8x8-per-two-warps tiles measured 1-2% slower on the benchmark frames)
+  // 8x8-per-two-warps tiles measured 1-2% slower on the benchmark frames).
+  // Blocks of four warps leave the SMs more evenly than blocks of eight: a
+  // 640x360 frame 0.168 to 0.162 ms, 1280x720 0.215 to 0.207, 1920x1080 the
+  // same; one or two warps gain nothing more.
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t px = blockIdx.x * 32u + warp * 4u + (lane & 3u);
+  const uint32_t px = blockIdx.x * (4u * kTraceWarps) + warp * 4u + (lane & 3u);
   const uint32_t py = blockIdx.y * 8u + (lane >> 2);
   const bool valid = px < T.W && py < T.H;
   const uint64_t pix = (uint64_t)py * T.W + px;
@@ -49,7 +54,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const TraceParams *__rest
   if (FAST) {  // fast normals (compute.wgsl:4337-4342)
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
     if (__any_sync(0xffffffffu, w.hit)) {
-      const F3 n = tape_normal(T, tid & 31u, tid >> 5, w.end, w.tnorm);
+      const F3 n = tape_normal(T, tid & 31u, tid >> 5, w.end, w.tnorm, w.hit);
       if (w.hit) w.nrm = n;
     }
   }
@@ -82,14 +87,14 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const TraceParams *__rest
   }
 }
 
-// Shared memory of one block with fast normals: 8 warps' register files.
-size_t trace_smem_bytes(const TraceParams &T) { return T.code ? (size_t)8 * T.nregs * 32 * sizeof(float2) : 0; }
+// Shared memory of a block with fast normals.
+static size_t trace_smem_bytes(const TraceParams &T) { return T.code ? (size_t)kTraceWarps * normal_bytes(T.nregs) : 0; }
 
-cudaError_t launch_cinematic(const TraceParams &T, const TraceParams *Tdev, size_t smem, cudaStream_t st);
+cudaError_t launch_cinematic(const TraceParams &T, const TraceParams *Tdev, cudaStream_t st);
 
 cudaError_t launch_trace(const TraceParams &T, const TraceParams *Tdev, cudaStream_t st) {
+  if (T.cinematic) return launch_cinematic(T, Tdev, st);
   const size_t smem = trace_smem_bytes(T);
-  if (T.cinematic) return launch_cinematic(T, Tdev, smem, st);
   if (smem > (48u << 10)) {  // the attribute is per kernel and device: only ever raise it
     static std::mutex mu;
     static size_t set_bytes[64] = {0};
@@ -103,8 +108,8 @@ cudaError_t launch_trace(const TraceParams &T, const TraceParams *Tdev, cudaStre
       if (dev >= 0 && dev < 64) set_bytes[dev] = smem;
     }
   }
-  dim3 block(256);
-  dim3 grid((T.W + 31) / 32, (T.H + 7) / 8);
+  dim3 block(32 * kTraceWarps);
+  dim3 grid((T.W + 4 * kTraceWarps - 1) / (4 * kTraceWarps), (T.H + 7) / 8);
   if (T.code) trace_kernel<true><<<grid, block, smem, st>>>(Tdev);
   else trace_kernel<false><<<grid, block, 0, st>>>(Tdev);
   return cudaGetLastError();

@@ -16,6 +16,7 @@
 #include "device_types.h"
 #include "fmath.cuh"
 #include "interp.cuh"
+#include "point_tape.cuh"
 #include "trace_params.h"
 
 namespace tsi {
@@ -49,27 +50,64 @@ __device__ __forceinline__ void node_box(const VoxelPoolDev &pool, uint32_t v, F
   p1 = f3(a.y, a.w, b.y);
 }
 
-// Dynamic shared memory of trace_kernel: with fast normals, one interval
-// register file per warp for the point evaluations.
+// Dynamic shared memory of the tracers: with fast normals, per warp what
+// point_forward takes (in the general form: a register file of intervals).
 extern __shared__ __align__(16) unsigned char trace_smem[];
+
+// Shared memory of a warp with fast normals: four points per lane while four
+// blocks of four warps fit an SM's shared memory so, else two at a time.
+__host__ __device__ __forceinline__ bool four_points(uint32_t nregs) { return point_bytes<2>(nregs) <= 14u << 10; }
+__host__ __device__ __forceinline__ uint32_t normal_bytes(uint32_t nregs) {
+  return four_points(nregs) ? point_bytes<2>(nregs) : point_bytes<1>(nregs);
+}
 
 // finite_diff_normal (compute.wgsl:4143-4184) for any tape: the tetrahedron
 // of points p + k h (h = 0.01, k in {(1,-1,-1), (-1,-1,1), (-1,1,-1),
 // (1,1,1)}) with f evaluated by the tape on point boxes (round to nearest),
 // normalised as v / |v|.  The reference pastes a per-scene function here;
-// the tape makes it work for every scene.  Called by the whole warp; lanes
-// without a hit evaluate a point too and discard it.
-static __device__ __noinline__ F3 tape_normal(const TraceParams &T, uint32_t lane, uint32_t warp, F3 p, float t) {
-  float2 *rf = reinterpret_cast<float2 *>(trace_smem) + (size_t)warp * T.nregs * 32u;
-  const float h = 0.01f;
-  const float kx[4] = {1.0f, -1.0f, -1.0f, 1.0f}, ky[4] = {-1.0f, -1.0f, 1.0f, 1.0f};
-  const float kz[4] = {-1.0f, 1.0f, -1.0f, 1.0f};
-  float f[4];
+// the tape makes it work for every scene.  Called by the whole warp with at
+// least one lane that hit; the others evaluate that lane's points.
+constexpr float kNormalH = 0.01f;
+
+// The four values by the interval interpreter, point by point: for values
+// beyond fix's range.
+static __device__ __noinline__ void tape_values_general(const TraceParams &T, uint32_t lane, float2 *rf, F3 p, float t,
+                                                        float f[4]) {
+  const float h = kNormalH;
+#pragma unroll 1
   for (int q = 0; q < 4; ++q) {
-    const Iv r = forward_pass<false>(T.code, T.len, T.out_reg, rf, lane, iv(p.x + kx[q] * h), iv(p.y + ky[q] * h),
-                                     iv(p.z + kz[q] * h), iv(t), nullptr, nullptr);
+    const float kx = (q == 0 || q == 3) ? 1.0f : -1.0f, ky = q >= 2 ? 1.0f : -1.0f, kz = (q & 1) ? 1.0f : -1.0f;
+    __syncwarp();
+    const Iv r = forward_pass<false>(T.code, T.len, T.out_reg, rf, lane, iv(p.x + kx * h), iv(p.y + ky * h),
+                                     iv(p.z + kz * h), iv(t), nullptr, nullptr);
     f[q] = r.lo;
   }
+}
+
+static __device__ __forceinline__ F3 tape_normal(const TraceParams &T, uint32_t lane, uint32_t warp, F3 p, float t,
+                                                 bool hit) {
+  const uint32_t hits = __ballot_sync(FULL_MASK, hit);
+  const int src = hit ? (int)lane : __ffs((int)hits) - 1;
+  p = f3(__shfl_sync(FULL_MASK, p.x, src), __shfl_sync(FULL_MASK, p.y, src), __shfl_sync(FULL_MASK, p.z, src));
+  t = __shfl_sync(FULL_MASK, t, src);
+  unsigned char *mem = trace_smem + (size_t)warp * normal_bytes(T.nregs);
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(mem);
+  const float h = kNormalH;
+  const float xp = p.x + h, xm = p.x - h, yp = p.y + h, ym = p.y - h, zp = p.z + h, zm = p.z - h;
+  const F2 x0 = f2_pack(xp, xm), x1 = f2_pack(xm, xp), y0 = f2_pack(ym, ym), y1 = f2_pack(yp, yp), z = f2_pack(zm, zp);
+  float f[4];
+  bool good;
+  if (four_points(T.nregs)) {
+    good = point_forward<2>(T.code, T.len, T.nregs, T.out_reg, smem, lane, Pts<2>{x0, x1}, Pts<2>{y0, y1}, Pts<2>{z, z},
+                            t, f);
+  } else {
+    good = point_forward<1>(T.code, T.len, T.nregs, T.out_reg, smem, lane, Pts<1>{x0}, Pts<1>{y0}, Pts<1>{z}, t, f);
+    __syncwarp();
+    good &= point_forward<1>(T.code, T.len, T.nregs, T.out_reg, smem, lane, Pts<1>{x1}, Pts<1>{y1}, Pts<1>{z}, t, f + 2);
+  }
+  if (!__all_sync(FULL_MASK, good)) tape_values_general(T, lane, reinterpret_cast<float2 *>(mem), p, t, f);
+  const float kx[4] = {1.0f, -1.0f, -1.0f, 1.0f}, ky[4] = {-1.0f, -1.0f, 1.0f, 1.0f};
+  const float kz[4] = {-1.0f, 1.0f, -1.0f, 1.0f};
   F3 v = f3(kx[0] * f[0], ky[0] * f[0], kz[0] * f[0]);
   for (int q = 1; q < 4; ++q) v = v + f3(kx[q] * f[q], ky[q] * f[q], kz[q] * f[q]);
   const float l = len3(v);
