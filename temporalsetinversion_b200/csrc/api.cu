@@ -1073,7 +1073,7 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
     if (compile_wide(ins, pt, wt, st, why) && wt.nbundles > 0 &&
         wide_cell_bytes(wt.nvalues, wt.ncontrib, (pt.n_minmax + 15) / 16) <= kWideCellMaxGlobalBytes) {
       WideTapeDev dv;
-      decode_wide(wt, dv);
+      decode_wide(wt, pt, dv);
       auto up = [&](auto **dst, const std::vector<uint32_t> &src) { part(dst, src.data(), src.size() * 4u); };
       up(&t->d_wfwd, dv.fwd);
       up(&t->d_wrev, dv.rev);

@@ -122,6 +122,8 @@ __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, 
       live_hi = (live_hi & ~q.y) | (on ? q.w : 0u);
       keep |= on ? 1u << j : 0u;
     }
+    // a copy of a register to itself does nothing, forward or reverse
+    keep &= ~__ballot_sync(FULL_MASK, hk == H_COPY && TSI_W0_A(out.x) == d);
     if ((keep >> lane) & 1u) {
       tmp[cnt + __popc(keep & ~((2u << lane) - 1u))] = out;
       kept_mm += TSI_H_IS_MINMAX(hk) ? 1u : 0u;
@@ -1005,9 +1007,13 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
           q[i] = fetch(kb - i - 4);
           // a min/max has an ordinal: the decision may rule an operand out
           const bool mm = s1.y != TSI_NONE, live = flags[s1.x] != 0;
-          const uint32_t d = cb[mm ? s1.y >> 4 : words] >> (2u * (s1.y & 15u));
-          if (live && s1.z != TSI_NONE && (d & 3u) != 2u) flags[s1.z] = 1;
+          const uint32_t ord = s1.y & ~(WL_SAME_A | WL_SAME_B);
+          const uint32_t d = (cb[mm ? ord >> 4 : words] >> (2u * (ord & 15u))) & 3u;
+          if (live && s1.z != TSI_NONE && d != 2u) flags[s1.z] = 1;
           if (live && s1.w != TSI_NONE && !(d & 1u)) flags[s1.w] = 1;
+          // a copy of a register to itself is not kept (nothing reads this
+          // flag again but a thread that repeats the slot)
+          if (live && mm && ((d & 1u) ? s1.y & WL_SAME_A : d != 0u ? s1.y & WL_SAME_B : 0u)) flags[s1.x] = 0;
           __syncthreads();
         }
       }

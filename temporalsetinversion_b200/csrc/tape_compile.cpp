@@ -365,7 +365,7 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   return true;
 }
 
-void decode_wide(const WideTape &wt, WideTapeDev &out) {
+void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
   const uint32_t nv = wt.nvalues, zero = nv, dummy = nv + 1u, nv2 = nv + 2u;
   out = WideTapeDev{};
   std::vector<uint8_t> used(nv, 0);  // values some instruction reads
@@ -377,6 +377,12 @@ void decode_wide(const WideTape &wt, WideTapeDev &out) {
     if (S[7] != TSI_NONE) used[S[7]] = 1;
     if (S[5] != TSI_NONE) n_minmax = std::max(n_minmax, S[5] + 1u);
   }
+  // value v is the narrow tape's instruction v - 4
+  auto same = [&](uint32_t v) -> uint32_t {
+    const uint32_t w0 = pt.code[2 * size_t(v - 4u)], w1 = pt.code[2 * size_t(v - 4u) + 1];
+    const bool a = TSI_W0_DST(w0) == TSI_W0_A(w0), b = TSI_H_IS_II(TSI_W0_H(w0)) && TSI_W0_DST(w0) == (w1 & 255u);
+    return (a ? WL_SAME_A : 0u) | (b ? WL_SAME_B : 0u);
+  };
   std::vector<uint32_t> targets;
   auto push4 = [](std::vector<uint32_t> &v, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     v.push_back(a);
@@ -492,7 +498,7 @@ void decode_wide(const WideTape &wt, WideTapeDev &out) {
     for (uint32_t s = 0; s < padded; ++s) {
       const uint32_t *S = s < count ? &wt.slots[size_t(first + s) * 12] : nullptr;
       if (!S || (S[0] & 63u) == TSI_H_PAD) push4(out.live, dummy, TSI_NONE, TSI_NONE, TSI_NONE);
-      else push4(out.live, S[4], S[5], S[6], S[7]);
+      else push4(out.live, S[4], S[5] == TSI_NONE ? TSI_NONE : S[5] | same(S[4]), S[6], S[7]);
     }
   }
 }

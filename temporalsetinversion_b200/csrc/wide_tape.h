@@ -48,6 +48,10 @@ constexpr uint32_t kWideWarps = 8;
 struct WideTape;
 struct PackedTape;
 
+// Of a min/max in the liveness slots: its register is the operand's, so the
+// copy that it becomes when that operand is always chosen does nothing.
+constexpr uint32_t WL_SAME_A = 1u << 30, WL_SAME_B = 1u << 31;
+
 struct WideTapeDev {
   std::vector<uint32_t> fwd;      // 4 words per slot, stream after stream
   std::vector<uint32_t> rev;      // 4 words per slot of the first array, then the second array
@@ -55,9 +59,9 @@ struct WideTapeDev {
   std::vector<uint32_t> ctl;      // step bytes, four to a word: the forward streams, then the reverse ones,
                                   // each with kWideAhead steps and a word more at its end
   std::vector<uint32_t> streams;  // 2 words per stream (8 forward, 8 reverse): first slot, first ctl word
-  std::vector<uint32_t> live;     // 4 words per slot: destination, min/max ordinal, A, B (TSI_NONE: absent)
+  std::vector<uint32_t> live;     // 4 words per slot: destination, min/max ordinal and WL bits, A, B (TSI_NONE: absent)
   std::vector<uint32_t> bundles;  // of `live`: first slot, slot count (a multiple of 32)
   uint32_t rev_slots = 0;         // slots of the reverse streams
 };
-void decode_wide(const WideTape &wt, WideTapeDev &out);
+void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out);
 }  // namespace tsi
