@@ -68,3 +68,23 @@ def test_directed_boxes_do_not_depend_on_the_route(device, name):
     all_ = t.eval_boxes(boxes, rounding_mode=1)
     for n in (1, 33, 70):
         assert same(t.eval_boxes(boxes[:n], rounding_mode=1), all_[:n])
+
+
+@pytest.mark.gpu
+def test_sqrt_at_the_edges_of_its_short_form(device):
+    """Zeros of both signs, negative lower bounds, the ends of the range of
+    the branch-free root and beyond them, denormals, infinities and NaN."""
+    b = scenes.IRBuilder()
+    tape = api.IR.new(b.text(b.sqrt("%0"))).gpu_instructions
+    f = np.float32
+    edge = [0.0, -0.0, -1.0, 1e-45, 1e-38, np.nextafter(f(1e-23), f(0)), 1e-23, np.nextafter(f(1e-23), f(1)), 1e-9,
+            0.25, 2.0, 3.0, np.nextafter(f(1e23), f(0)), 1e23, np.nextafter(f(1e23), f(np.inf)), 3e38, np.inf, -np.inf,
+            np.nan]
+    pairs = np.array([(x, y) for x in edge for y in edge], np.float32)
+    rng = np.random.default_rng(1)
+    more = np.sort((rng.uniform(1, 4, (4000, 2)) * 2.0 ** rng.integers(-84, 84, (4000, 1))).astype(np.float32), axis=1)
+    pairs = np.concatenate([pairs, more])
+    boxes = np.zeros((len(pairs), 8), np.float32)
+    boxes[:, 0:2] = pairs
+    t = Tape.upload(device, tape)
+    assert same(t.eval_boxes(boxes), oracle.eval_boxes(tape, boxes))
