@@ -207,6 +207,9 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
   if (!p.fast_normals && p.normal_viz) f |= SF_ALWAYS_DERIV;
   if (p.pruning) f |= SF_PRUNING;
   if (p.rounding_mode == TSI_ROUND_DIRECTED) f |= SF_DIRECTED;
+  bool plain = !s->tape->strict && fabsf(time) <= 1048576.0f && !(fabsf(L.t0) > 1048576.0f);
+  for (int q = 0; q < 3; ++q) plain = plain && fabsf(p.root_lo[q]) <= 1048576.0f && fabsf(p.root_hi[q]) <= 1048576.0f;
+  if (!plain) f |= SF_STRICT;
   L.flags = f;
   L.root_rec = slot;
   L.levels = tree_levels(p);
@@ -1051,6 +1054,7 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
   t->n_minmax = pt.n_minmax;
   t->fwd_cost = pt.fwd_cost;
   t->rev_cost = pt.rev_cost;
+  t->strict = pt.strict;
   c->tapes.insert(t);
   // The tape's arrays on the device are parts of one allocation, filled by
   // one copy (each allocation and each copy cost more than the bytes: the
@@ -1064,7 +1068,14 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
     memcpy(image.data() + off, src, bytes);
     parts.emplace_back((void **)dst, off);
   };
-  part(&t->d_code, pt.code.data(), (size_t)t->len * sizeof(uint2));
+  std::vector<uint32_t> code = pt.code;
+  for (uint32_t i = 0; i < t->len; ++i) {
+    const uint32_t h = TSI_W0_H(code[2 * i]);
+    if (!TSI_H_IS_MINMAX(h)) continue;
+    code[2 * i] |= TSI_W0_WITH_DEPS(pt.deps[i] & 15u);
+    if (TSI_H_IS_II(h)) code[2 * i + 1] |= (uint32_t)(pt.deps[i] >> 4) << 8;
+  }
+  part(&t->d_code, code.data(), (size_t)t->len * sizeof(uint2));
   // bundled form for long tapes (the wide path pays off once a tape has
   // several times more instructions than bundles); a working set beyond
   // shared memory lives in the per-block global scratch

@@ -42,6 +42,7 @@ struct tsi_tape {
   uint32_t len = 0;  // instructions after the 4 ARG slots
   uint32_t count = 0, nregs = 0, out_reg = 0, n_minmax = 0;
   uint64_t fwd_cost = 0, rev_cost = 0;
+  bool strict = false;  // PackedTape::strict
   // bundled form for the wide path (absent when the tape is short)
   uint4 *d_wfwd = nullptr, *d_wrev = nullptr, *d_wlive = nullptr, *d_wrev16 = nullptr;
   uint2 *d_wstreams = nullptr;

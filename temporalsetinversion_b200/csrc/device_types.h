@@ -39,6 +39,7 @@ enum tsi_scene_flags {
   SF_ALWAYS_DERIV = 1u << 4,  // !fast_normals && normal_viz (compute.wgsl:3780)
   SF_PRUNING = 1u << 5,
   SF_DIRECTED = 1u << 6,  // outward rounding (tsi_rounding TSI_ROUND_DIRECTED)
+  SF_STRICT = 1u << 7,    // an infinite reverse rule may meet a pruned branch's zero (see narrow_reverse)
 };
 
 enum tsi_error_bits {

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(32) evalbox_narrow(EvalTape T, uint32_t n, con
   const Iv f = narrow_forward<D>(T.code, T.len, T.out_reg, R, lane, v[0], v[1], v[2], v[3], lg, nullptr, nlog);
   if (reverse) {
     bool bad = false;
-    narrow_reverse<D>(T.code, T.len, T.nregs, T.out_reg, R, lane, lg, nlog, true, sens, bad);
+    narrow_reverse<D>(T.code, T.len, T.nregs, T.out_reg, R, lane, lg, nlog, true, false, sens, bad);
   }
   if (lane < cols) store_box(out + box * 10u, f, sens);
 }

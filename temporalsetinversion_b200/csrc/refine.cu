@@ -19,7 +19,8 @@
 // dropped.  Pruning never changes a result: a decided MIN/MAX returns its
 // chosen operand bit for bit, and the reverse pass falls back to the full
 // tape when a sensitivity overflows (the only case where the dead branch of
-// the full tape would contribute, through 0 * inf).
+// the full tape would contribute, through 0 * inf; narrow_reverse tells
+// where).
 //
 // A pruned tape is valid for cells inside its group's boxes whose time
 // interval lies inside the interval the decisions were taken on.  The
@@ -67,6 +68,7 @@ __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddep
 // is three logic operations an instruction on the 64-bit mask of live
 // registers, on masks read back by broadcast loads.  (One lane decoding and
 // scanning took 300 cycles an instruction, this takes 35.)
+template <bool D>
 __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, uint32_t len_, uint32_t n_minmax_,
                                                 uint32_t out_reg, const uint2 *dg, uint32_t g, uint32_t E, uint2 *tmp,
                                                 const NarrowRows &R, uint32_t lane, uint32_t &mm_kept, uint32_t &fwd_cost,
@@ -89,19 +91,21 @@ __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, 
     uint32_t hk = h;
     bool use_a = h != H_CONST, use_b = TSI_H_IS_II(h);
     if (mmx) {
+      const uint32_t deps_a = TSI_W0_WITH_DEPS(TSI_W0_DEPS(w.x));
+      const uint32_t deps_b = TSI_H_IS_II(h) ? TSI_W0_WITH_DEPS(TSI_W1_DEPS(w.y)) : 0u;
       const uint2 dd = dg[m + __popc(mmb & ((1u << lane) - 1u))];
       const uint32_t ga = (dd.x >> (g * 8u)) & 0xffu, gb = (dd.y >> (g * 8u)) & 0xffu;
       if ((ga & E) == E) {
-        out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, d, a) | (w.x & TSI_W0_ODD), 0u);
+        out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, d, a) | (w.x & TSI_W0_ODD) | deps_b, 0u);
         hk = H_COPY;
         use_b = false;
       } else if ((gb & E) == E) {
         use_a = false;
         if (TSI_H_IS_II(h)) {
-          out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, d, b) | (w.x & TSI_W0_ODD), 0u);
+          out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, d, b) | (w.x & TSI_W0_ODD) | deps_a, 0u);
           hk = H_COPY;
         } else {
-          out = make_uint2(TSI_W0(H_CONST, 0u, 0u, d, 0u), w.y);
+          out = make_uint2(TSI_W0(H_CONST, 0u, 0u, d, 0u) | deps_a, w.y);
           hk = H_CONST;
         }
       }
@@ -122,8 +126,9 @@ __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, 
       live_hi = (live_hi & ~q.y) | (on ? q.w : 0u);
       keep |= on ? 1u << j : 0u;
     }
-    // a copy of a register to itself does nothing, forward or reverse
-    keep &= ~__ballot_sync(FULL_MASK, hk == H_COPY && TSI_W0_A(out.x) == d);
+    // a copy of a register to itself does nothing, forward or reverse, but
+    // carry a directed reverse pass's test
+    if (!D) keep &= ~__ballot_sync(FULL_MASK, hk == H_COPY && TSI_W0_A(out.x) == d);
     if ((keep >> lane) & 1u) {
       tmp[cnt + __popc(keep & ~((2u << lane) - 1u))] = out;
       kept_mm += TSI_H_IS_MINMAX(hk) ? 1u : 0u;
@@ -497,7 +502,8 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       const long long q1 = clock64();
       bool bad = false;
       if (any_deriv)
-        narrow_reverse<D>(TR.code, TR.len, TR.nregs, TR.out_reg, R, lane, opl, nlog, take_deriv, sens, bad);
+        narrow_reverse<D>(TR.code, TR.len, TR.nregs, TR.out_reg, R, lane, opl, nlog, take_deriv, (flags & SF_STRICT) != 0, sens,
+                          bad);
       if (lane == 0 && attempt == 0) {
         ws[ST_CYC_N_FWD] += (unsigned long long)(q1 - q0);
         ws[ST_N_FWD_INSTR] += TR.len;
@@ -695,7 +701,7 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
         const uint32_t pE = __shfl_sync(FULL_MASK, E, src);
         uint2 *ptmp = reinterpret_cast<uint2 *>(__shfl_sync(FULL_MASK, reinterpret_cast<unsigned long long>(tmp), src));
         uint32_t mk, fc, rc;
-        const uint32_t n = prune_group(pcode, plen, pmm, pout, dg, (uint32_t)src >> 3, pE, ptmp, R, lane, mk, fc, rc);
+        const uint32_t n = prune_group<D>(pcode, plen, pmm, pout, dg, (uint32_t)src >> 3, pE, ptmp, R, lane, mk, fc, rc);
         if ((int)lane == src) {
           cnt = n;
           mmk = mk;
@@ -989,6 +995,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
     // a load under a test or select would be waited for at once.
     {
       const uint4 *__restrict__ slots = W.live;
+      const bool same = !(S.flags & SF_DIRECTED);  // (prune_group's rule)
       auto fetch = [&](int kk) -> uint4 {
         const uint2 b = bt[max(kk, 0)];
         return slots[b.x + min(tid, b.y - 1u)];
@@ -1013,7 +1020,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
           if (live && s1.w != TSI_NONE && !(d & 1u)) flags[s1.w] = 1;
           // a copy of a register to itself is not kept (nothing reads this
           // flag again but a thread that repeats the slot)
-          if (live && mm && ((d & 1u) ? s1.y & WL_SAME_A : d != 0u ? s1.y & WL_SAME_B : 0u)) flags[s1.x] = 0;
+          if (same && live && mm && ((d & 1u) ? s1.y & WL_SAME_A : d != 0u ? s1.y & WL_SAME_B : 0u)) flags[s1.x] = 0;
           __syncthreads();
         }
       }
@@ -1096,15 +1103,17 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
             if (TSI_H_IS_MINMAX(h)) {
               const uint32_t d = (cb[mm >> 4] >> (2u * (mm & 15u))) & 3u;
               const uint32_t dd = TSI_W0_DST(w.x);
+              const uint32_t deps_a = TSI_W0_WITH_DEPS(TSI_W0_DEPS(w.x));
+              const uint32_t deps_b = TSI_H_IS_II(h) ? TSI_W0_WITH_DEPS(TSI_W1_DEPS(w.y)) : 0u;
               if (d & 1u) {
-                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD), 0u);
+                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD) | deps_b, 0u);
                 hk = H_COPY;
               } else if (d & 2u) {
                 if (TSI_H_IS_II(h)) {
-                  out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD), 0u);
+                  out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD) | deps_a, 0u);
                   hk = H_COPY;
                 } else {
-                  out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u), w.y);
+                  out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u) | deps_a, w.y);
                   hk = H_CONST;
                 }
               } else {

@@ -2,6 +2,8 @@
 #include "tape_compile.h"
 
 #include <algorithm>
+#include <cmath>
+#include <limits>
 #include <set>
 #include <utility>
 #include <cstring>
@@ -70,6 +72,24 @@ uint32_t handler_of(uint32_t op, uint32_t top) {
 
 }  // namespace
 
+// A bound of log2 |value| from those of the operands; NaN for handlers whose
+// value or reverse rule is infinite on ordinary operands.
+static double magnitude(uint32_t h, double a, double b, float lit) {
+  const double l = lit == 0.0f ? -150.0 : std::log2(std::fabs(double(lit)));
+  switch (h) {
+    case H_CONST: return l;
+    case H_COPY: case H_NEG: case H_ABS: case H_SQRT: return std::max(a, 0.0);
+    case H_ADD_II: case H_SUB_II: case H_MIN_II: case H_MAX_II: return std::max(a, b) + 1.0;
+    case H_ADD_IF: case H_SUB_IF: case H_SUB_FI: case H_MIN_IF: case H_MAX_IF: return std::max(a, l) + 1.0;
+    case H_MUL_II: return std::max(a, 0.0) + std::max(b, 0.0) + 1.0;
+    case H_MUL_IF: return a + l + 1.0;
+    case H_SQR: return std::max(2.0 * a, 0.0) + 1.0;
+    case H_FLOOR: return std::max(a, 0.0) + 1.0;
+    case H_SIN: case H_COS: return 1.0;
+    default: return std::numeric_limits<double>::quiet_NaN();
+  }
+}
+
 bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &status,
                   std::string &why) {
   const uint32_t n = uint32_t(ins.size());
@@ -104,6 +124,10 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
   static const uint32_t fwd_cost[H_COUNT] = TSI_OPCOST_FWD_INIT;
   static const uint32_t rr_cost[H_COUNT] = TSI_OPCOST_RR_INIT;
   out.code.reserve(size_t(n - 4) * 2);
+  std::vector<double> mag(n, 20.0);  // every slot's bound of log2 |value|
+  std::vector<uint8_t> deps(n, 0);   // every slot's arguments
+  for (uint32_t a = 0; a < 4 && a < n; ++a) deps[a] = uint8_t(1u << a);
+  out.deps.reserve(n - 4);
   for (uint32_t j = 4; j < n; ++j) {
     const IrInstr &in = ins[j];
     const uint32_t top = op_top_of(in);
@@ -149,6 +173,11 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
     out.code.push_back(TSI_W0(h, fa, fb, d, ra) | (odd ? TSI_W0_ODD : 0u));
     out.code.push_back(w1);
     if (TSI_H_IS_MINMAX(h)) out.n_minmax++;
+    const uint32_t da = has_a ? deps[a_slot] : 0u, db = has_b ? deps[b_slot] : 0u;
+    deps[j] = uint8_t(da | db);
+    out.deps.push_back(uint8_t(da | (db << 4)));
+    mag[j] = magnitude(h, has_a ? mag[a_slot] : 0.0, has_b ? mag[b_slot] : 0.0, lit);
+    if (odd || !(mag[j] < 120.0) || (h == H_SQRT && !fa)) out.strict = true;
     out.fwd_cost += fwd_cost[h] + TSI_FIX_COST;
     out.rev_cost += rr_cost[h] + TSI_REV_OPERAND_COST * TSI_H_NREG(h);
   }

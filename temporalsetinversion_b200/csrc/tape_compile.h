@@ -17,6 +17,11 @@ struct PackedTape {
   uint32_t n_minmax = 0;
   uint64_t fwd_cost = 0;       // opcost.h, forward, one cell
   uint64_t rev_cost = 0;       // opcost.h, reverse, one cell
+  // Some instruction may have an infinite reverse rule at a zero sensitivity
+  // that the skip rule (compute.wgsl:3800-3806) does not keep from it, for
+  // arguments up to 2^20.
+  bool strict = false;
+  std::vector<uint8_t> deps;  // per instruction: the arguments A depends on, B's in the upper four bits
   std::vector<uint32_t> slot_reg;  // register of every SSA slot (debug, tests)
 };
 

@@ -10,10 +10,14 @@
 //       bit   7      operand B is single-use
 //       bit   8      a flagged operand has other users after all (an uploaded
 //                    tape's use counts may be wrong): no shortcut applies
-//       bits  9..15  reserved
+//       bits  9..12  uploaded min/max: the arguments that operand A depends on;
+//                    copy or constant of a decided min/max: those that the
+//                    operand which lost depends on (x, y, z, t from bit 9)
+//       bits 13..15  reserved
 //       bits 16..23  destination register
 //       bits 24..31  register A (larg, or rarg for the literal-left kinds)
-//   w1  register B in bits 0..7 (two-register handlers) or the f32 literal
+//   w1  register B in bits 0..7 (two-register handlers; of an uploaded min/max
+//       the arguments that B depends on in bits 8..11) or the f32 literal
 //
 // The handler folds compute.wgsl's two-level switch (op_top at 3642, op at
 // 3647/3714/3753) into one warp-uniform dispatch.  Unsupported (op, op_top)
@@ -40,6 +44,9 @@ enum tsi_handler {
 #define TSI_W0(h, fa, fb, dst, a) \
   ((uint32_t)(h) | ((uint32_t)(fa) << 6) | ((uint32_t)(fb) << 7) | ((uint32_t)(dst) << 16) | ((uint32_t)(a) << 24))
 #define TSI_W0_ODD (1u << 8)
+#define TSI_W0_DEPS(w) (((w) >> 9) & 15u)
+#define TSI_W1_DEPS(w) (((w) >> 8) & 15u)
+#define TSI_W0_WITH_DEPS(deps) ((uint32_t)(deps) << 9)
 #define TSI_W0_H(w) ((w) & 63u)
 #define TSI_W0_FA(w) (((w) >> 6) & 1u)
 #define TSI_W0_FB(w) (((w) >> 7) & 1u)

@@ -133,3 +133,37 @@ def test_widest_register_files_run(device, live):
         gs.invert(time)
         os_.invert(time)
         assert_cells_equal(gs.cells(), os_.cells())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene", ["csg", "division"])
+def test_directed_infinite_sensitivities_match_full_tape(device, scene):
+    """Cells around roots at zero below decided maxima (distances to boxes), on
+    a tape whose rules are finite but for the roots' and on one with
+    quotients: pruned tapes give what the full tape gives, on one warp and
+    block-wide, bit for bit."""
+    if scene == "csg":
+        tape = api.IR.new(scenes.csg(24, 3)).gpu_instructions
+    else:
+        b = scenes.IRBuilder()
+        acc = b.sub(b.sqrt(b.add(b.mul(b.X, b.X), b.mul(b.Y, b.Y))), 0.9)
+        for i in range(14):
+            q = b.max(b.sub(b.abs(b.sub(b.X, 0.2 * i - 1.4)), 0.08), 0.0)
+            r = b.max(b.sub(b.abs(b.add(b.Z, b.mul(b.T, 0.3))), 0.2), 0.0)
+            s = b.sub(b.sqrt(b.add(b.mul(q, q), b.mul(r, r))), 0.03)
+            acc = b.min(acc, b.max(b.div(s, 3.0), b.sub(b.Y, 0.5)))
+        tape = api.IR.new(b.text(acc)).gpu_instructions
+    ref = None
+    for threshold, pruning in ((0xFFFFFFFF, 0), (0xFFFFFFFF, 1), (1, 1)):
+        t = Tape.upload(device, tape)
+        t.wide_threshold = threshold
+        s = Scene(device, t, api.default_params(localsubdiv=6, delta=0.01, rounding_mode=1, normal_viz=1, pruning=pruning))
+        cells = []
+        for time in TIMES:
+            s.invert(time)
+            cells.append(s.cells())
+        if ref is None:
+            ref = cells
+        else:
+            for a, c in zip(cells, ref):
+                assert_cells_equal(a, c)
