@@ -55,13 +55,16 @@ struct CellArray<false> {
 };
 template <>
 struct CellArray<true> {
-  float2 *base;
-  __device__ __forceinline__ explicit CellArray(void *p) : base(reinterpret_cast<float2 *>(p)) {}
+  unsigned long long base;
+  __device__ __forceinline__ explicit CellArray(void *p) : base((unsigned long long)__cvta_generic_to_global(p)) {}
   __device__ __forceinline__ Iv ld(uint32_t i) const {
-    const float2 v = base[i];
-    return Iv{v.x, v.y};
+    Iv v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.lo), "=f"(v.hi) : "l"(base + i * 8ull) : "memory");
+    return v;
   }
-  __device__ __forceinline__ void st(uint32_t i, Iv v) const { base[i] = make_float2(v.lo, v.hi); }
+  __device__ __forceinline__ void st(uint32_t i, Iv v) const {
+    asm volatile("st.global.v2.f32 [%0], {%1, %2};" ::"l"(base + i * 8ull), "f"(v.lo), "f"(v.hi) : "memory");
+  }
 };
 
 // The barrier between two steps.  The warps arrive from different places of
@@ -304,7 +307,7 @@ __device__ __forceinline__ void cell_reverse(const WideDev &W, CellArray<GM> V, 
   if (tid == 6u) G.st(W.nvalues - 1u, iv(1.0f));  // the field
   __syncthreads();
   const uint32_t stream = kWideWarps + (tid >> 5), nv = W.nvalues;
-  if (GM) {  // indices of more than 16 bits: the second array's slot is read in the step
+  if (GM && !W.rev16) {  // indices of more than 16 bits: the second array's slot is read in the step
     const uint4 *t = W.rev + W.rev_slots + W.streams[stream].x + (tid & 31u);
     walk_steps(W, stream, W.rev, [&](const uint4 &p, uint32_t kind) {
       const uint4 r = *t;
