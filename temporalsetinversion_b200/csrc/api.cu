@@ -185,7 +185,10 @@ WideDev wide_dev(const tsi_tape *t) {
   for (int q = 0; q < 4; ++q) {
     W.arg_gbase[q] = t->warg_gbase[q];
     W.arg_gcount[q] = t->warg_gcount[q];
+    W.g_arg[q] = t->wg_arg[q];
   }
+  W.gslots = t->wgslots;
+  W.g_field = t->wg_field;
   return W;
 }
 
@@ -234,11 +237,12 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
 }
 
 // Shared-memory working set of one wide cell (the device's cell_layout):
-// values and sensitivities (8 bytes per SSA value each, the zero and the
-// dummy among them), contribution records, decision bytes, liveness flags.
-size_t wide_cell_bytes(size_t nvalues, size_t ncontrib, size_t bm_words) {
+// values (8 bytes per SSA value, the zero and the dummy among them), the
+// second time interval's values or the sensitivities (`rows` of 8 bytes),
+// decision bytes, liveness flags.
+size_t wide_cell_bytes(size_t nvalues, size_t rows, size_t bm_words) {
   const size_t nv = nvalues + 2;
-  return ((16 * nv + ncontrib * 8 + 15) & ~size_t(15)) + (bm_words + 1) * 16 + ((nv + 15) & ~size_t(15));
+  return ((8 * nv + 8 * rows + 15) & ~size_t(15)) + (bm_words + 1) * 16 + ((nv + 15) & ~size_t(15));
 }
 // Tapes whose cell working set exceeds this stay on the narrow path (the
 // block also needs its static shared memory and room for a second block's
@@ -284,10 +288,14 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
   for (uint32_t i = 0; i < n; ++i) {
     const tsi_tape *t = scenes[i]->tape;
     if (!t->d_wfwd) continue;
-    const size_t b = wide_cell_bytes(t->wvalues, t->wcontrib, bm_words);
+    const size_t nv2 = (size_t)t->wvalues + 2;
+    const size_t b = wide_cell_bytes(t->wvalues, std::max<size_t>(nv2, t->wgslots), bm_words);
     if (b > budget || !t->d_wrev16) {
       fp.global[i] = 1;
-      gm_bytes = std::max(gm_bytes, b);
+      gm_bytes = std::max(gm_bytes, wide_cell_bytes(t->wvalues, nv2 + t->wcontrib, bm_words));
+      // the sensitivities' slots in shared memory all the same, if they fit
+      const size_t g = (size_t)t->wgslots * 8;
+      if (t->d_wrev16 && g <= budget) cell_bytes = std::max(cell_bytes, g);
     } else {
       cell_bytes = std::max(cell_bytes, b);
     }
@@ -1082,7 +1090,7 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
   if (t->len >= 256) {
     WideTape wt;
     if (compile_wide(ins, pt, wt, st, why) && wt.nbundles > 0 &&
-        wide_cell_bytes(wt.nvalues, wt.ncontrib, (pt.n_minmax + 15) / 16) <= kWideCellMaxGlobalBytes) {
+        wide_cell_bytes(wt.nvalues, wt.nvalues + 2 + wt.ncontrib, (pt.n_minmax + 15) / 16) <= kWideCellMaxGlobalBytes) {
       WideTapeDev dv;
       decode_wide(wt, pt, dv);
       auto up = [&](auto **dst, const std::vector<uint32_t> &src) { part(dst, src.data(), src.size() * 4u); };
@@ -1105,7 +1113,10 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
       for (int q = 0; q < 4; ++q) {
         t->warg_gbase[q] = wt.arg_gbase[q];
         t->warg_gcount[q] = wt.arg_gcount[q];
+        t->wg_arg[q] = dv.g_arg[q];
       }
+      t->wgslots = dv.gslots;
+      t->wg_field = dv.g_field;
     }
   }
   if (!image.empty()) {

@@ -54,6 +54,7 @@ struct tsi_tape {
   uint32_t narrow_parents = 1;  // parents per narrow item above the leaf level
   uint32_t wprune_level = 0xffffffffu;  // first level whose wide groups prune (0xffffffff: half the levels)
   uint32_t warg_gbase[4] = {TSI_NONE, TSI_NONE, TSI_NONE, TSI_NONE}, warg_gcount[4] = {0, 0, 0, 0};
+  uint32_t wgslots = 0, wg_arg[4] = {0, 0, 0, 0}, wg_field = 0;
 };
 
 struct tsi_scene {

@@ -94,6 +94,7 @@ struct WideDev {
                               // LaunchParams::wscratch (too large for shared memory)
   uint32_t arg_gbase[4];      // records of x, y, z, t (TSI_NONE: one user)
   uint32_t arg_gcount[4];
+  uint32_t gslots, g_arg[4], g_field;  // the sensitivities' slots of rev16
 };
 
 struct SceneLaunch {

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) evalbox_wide(EvalTape T, uint32_t n, cons
     load_box(boxes + (size_t)i * 8u, v);
     const Iv f = cell_forward<D, false>(T.wide, V, G, false, nullptr, nullptr, v[0], v[1], v[2], v[3], v[3]);
     if (reverse) {
-      cell_reverse<D, false>(T.wide, V, G, s_sens);
+      cell_reverse16<D>(T.wide, V, G, s_sens);
       for (int q = 0; q < 4; ++q) sens[q] = Iv{s_sens[q].x, s_sens[q].y};
     }
     if (threadIdx.x == 0) store_box(out + (size_t)i * 10u, f, sens);
@@ -121,7 +121,7 @@ template <bool D>
 static cudaError_t launch(const EvalTape &t, uint32_t n, const float *boxes, bool reverse, float *out, float4 *log,
                           cudaStream_t st) {
   const WideDev &W = t.wide;
-  const size_t wide = ((size_t)W.nvalues + 2u) * 8u * (reverse ? 2u : 1u) + (reverse ? (size_t)W.ncontrib * 8u : 0u);
+  const size_t wide = ((size_t)W.nvalues + 2u) * 8u + (reverse ? (size_t)W.gslots * 8u : 0u);
   if (W.nbundles && wide <= kWideMax && (!reverse || W.rev16)) {
     int bps = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, evalbox_wide<D>, 256, wide);

@@ -847,7 +847,7 @@ __device__ __forceinline__ CellLayout cell_layout(const WideDev &W, uint32_t bm_
   CellLayout L;
   const uint32_t nv = W.nvalues + 2u;
   L.sens = nv * 8u;
-  L.dec = (L.sens + (nv + W.ncontrib) * 8u + 15u) & ~15u;
+  L.dec = (L.sens + (W.global ? nv + W.ncontrib : max(nv, W.gslots)) * 8u + 15u) & ~15u;
   L.flags = L.dec + (bm_words + 1u) * 16u;  // one more for the padding lanes
   L.size = L.flags + ((nv + 15u) & ~15u);
   return L;
@@ -1292,7 +1292,12 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
     field = cell_forward<D, GM>(W, V, G, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz, targ, Iv{wl, wh});
     const long long c1 = clock64();
     if (take_deriv) {
-      cell_reverse<D, GM>(W, V, G, sh.sens);
+      if constexpr (GM) {
+        if (W.rev16 && W.gslots * 8u <= P.dyn_smem) cell_reverse16<D>(W, V, CellArray<false>(tsi_dyn_smem), sh.sens);
+        else cell_reverse<D>(W, V, G, sh.sens);
+      } else {
+        cell_reverse16<D>(W, V, G, sh.sens);
+      }
       for (int q = 0; q < 4; ++q) sens[q] = Iv{sh.sens[q].x, sh.sens[q].y};
     }
     if (tid == 0) {

@@ -3,7 +3,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <iterator>
 #include <limits>
+#include <map>
 #include <set>
 #include <utility>
 #include <cstring>
@@ -75,7 +77,10 @@ uint32_t handler_of(uint32_t op, uint32_t top) {
 // A bound of log2 |value| from those of the operands; NaN for handlers whose
 // value or reverse rule is infinite on ordinary operands.
 static double magnitude(uint32_t h, double a, double b, float lit) {
-  const double l = lit == 0.0f ? -150.0 : std::log2(std::fabs(double(lit)));
+  int e = -150;  // |lit| < 2^e
+  if (lit != lit || std::fabs(lit) > 3.4e38f) e = 1000;
+  else if (lit != 0.0f) std::frexp(lit, &e);
+  const double l = e;
   switch (h) {
     case H_CONST: return l;
     case H_COPY: case H_NEG: case H_ABS: case H_SQRT: return std::max(a, 0.0);
@@ -394,6 +399,47 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   return true;
 }
 
+// Slots of the sensitivities in the order of the reverse pass (wide_tape.h):
+// first fit, but for single slots, which are taken again last in, first out.
+struct SlotPool {
+  std::map<uint32_t, uint32_t> gaps{{0u, 0xffffffffu}};  // first slot, length
+  std::vector<uint32_t> ones;
+  uint32_t top = 0;
+  uint32_t take(uint32_t n) {
+    if (n == 1u && !ones.empty()) {
+      const uint32_t at = ones.back();
+      ones.pop_back();
+      return at;
+    }
+    auto it = gaps.begin();
+    while (it->second < n) ++it;
+    const uint32_t at = it->first, left = it->second - n;
+    gaps.erase(it);
+    if (left) gaps.emplace(at + n, left);
+    top = std::max(top, at + n);
+    return at;
+  }
+  void give(uint32_t at, uint32_t n) {
+    if (n == 1u) {
+      ones.push_back(at);
+      return;
+    }
+    auto next = gaps.lower_bound(at);
+    if (next != gaps.end() && next->first == at + n) {
+      n += next->second;
+      next = gaps.erase(next);
+    }
+    if (next != gaps.begin()) {
+      auto prev = std::prev(next);
+      if (prev->first + prev->second == at) {
+        prev->second += n;
+        return;
+      }
+    }
+    gaps.emplace(at, n);
+  }
+};
+
 void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
   const uint32_t nv = wt.nvalues, zero = nv, dummy = nv + 1u, nv2 = nv + 2u;
   out = WideTapeDev{};
@@ -420,7 +466,40 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
     v.push_back(d);
   };
   const uint32_t minus0 = 0x80000000u;
-  const bool small = nv2 + wt.ncontrib <= 65536u;  // (a value's records are as many as its users)
+  // ---- the sensitivities' slots: per value its place or its records' first
+  std::vector<uint32_t> place(nv, TSI_NONE), count(nv, 0u), first_rec(nv, 0u);
+  {
+    SlotPool pool;
+    pool.take(2);  // the zero, the dummy
+    for (uint32_t q = 0; q < 4u; ++q) {
+      count[q] = wt.arg_gcount[q];
+      first_rec[q] = count[q] ? wt.arg_gbase[q] : 0u;
+      out.g_arg[q] = place[q] = pool.take(std::max(1u, count[q]));
+    }
+    for (size_t i = 0; i < wt.slots.size(); i += 12) {
+      const uint32_t *S = &wt.slots[i];
+      if ((S[0] & 63u) == TSI_H_PAD || !S[11]) continue;
+      count[S[4]] = S[11];
+      first_rec[S[4]] = S[10];
+    }
+    if (place[nv - 1u] == TSI_NONE) place[nv - 1u] = pool.take(1);
+    out.g_field = place[nv - 1u];
+    for (uint32_t k = wt.nbundles; k-- > 0u;) {
+      const uint32_t first = wt.bundles[2 * k], last = first + wt.bundles[2 * k + 1];
+      for (uint32_t s = first; s < last; ++s) {
+        const uint32_t *S = &wt.slots[size_t(s) * 12];
+        if ((S[0] & 63u) == TSI_H_PAD) continue;
+        for (int q = 6; q < 8; ++q)
+          if (S[q] != TSI_NONE && place[S[q]] == TSI_NONE) place[S[q]] = pool.take(std::max(1u, count[S[q]]));
+      }
+      for (uint32_t s = first; s < last; ++s) {  // read in this step: free from the next on
+        const uint32_t *S = &wt.slots[size_t(s) * 12];
+        if ((S[0] & 63u) != TSI_H_PAD && place[S[4]] != TSI_NONE) pool.give(place[S[4]], std::max(1u, count[S[4]]));
+      }
+    }
+    out.gslots = pool.top;
+  }
+  const bool small = nv2 <= 65536u && out.gslots <= 65536u;  // (a value's records are as many as its users)
   // One group (warp g of bundle k) of the forward or reverse streams; its
   // kind.
   auto emit = [&](uint32_t k, uint32_t g, bool reverse) -> uint32_t {
@@ -477,17 +556,21 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
       const uint32_t fa = pad ? 0u : (S[0] >> 6) & 1u, fb = pad ? 0u : (S[0] >> 7) & 1u;
       if (fa && (!ii || fb)) c |= WC_SKIP;
       uint32_t ta = dummy, tb = dummy, src = zero, n = 0;
+      uint32_t ga = 1u, gb = 1u, gs = 0u;  // the same in the 16-bit form's slots
       if (!pad) {
         if (S[6] != TSI_NONE) ta = S[8] != TSI_NONE ? nv2 + S[8] : S[6];
         if (S[7] != TSI_NONE) tb = S[9] != TSI_NONE ? nv2 + S[9] : S[7];
         // a value nobody reads has sensitivity zero, the field one
         n = S[11];
         src = n ? nv2 + S[10] : (used[S[4]] || S[4] == nv - 1u ? S[4] : zero);
+        if (S[6] != TSI_NONE) ga = place[S[6]] + (S[8] != TSI_NONE ? S[8] - first_rec[S[6]] : 0u);
+        if (S[7] != TSI_NONE) gb = place[S[7]] + (S[9] != TSI_NONE ? S[9] - first_rec[S[7]] : 0u);
+        if (src != zero) gs = place[S[4]];
         gather = gather || n != 0u;
       }
       push4(out.rev, c | (h << 8), x, y, w);
       push4(targets, ta, tb, src, n);
-      if (small) push4(out.rev16, x | (src << 16), ta | (tb << 16), ii ? y : w, c | (h << 8) | (n << 16));
+      if (small) push4(out.rev16, x | (gs << 16), ga | (gb << 16), ii ? y : w, c | (h << 8) | (n << 16));
     }
     return kind | (reverse && gather ? WK_GATHER : 0u);
   };
@@ -513,7 +596,7 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
     push4(out.fwd, dummy << WC_DST_SHIFT, zero, zero, 0u);
     push4(out.rev, 0u, zero, zero, 0u);
     push4(targets, dummy, dummy, zero, 0u);
-    if (small) push4(out.rev16, zero | (zero << 16), dummy | (dummy << 16), 0u, 0u);
+    if (small) push4(out.rev16, zero, 1u | (1u << 16), 0u, 0u);
   }
   out.rev_slots = uint32_t(out.rev.size() / 4);
   out.rev.insert(out.rev.end(), targets.begin(), targets.end());

@@ -210,8 +210,8 @@ __device__ __forceinline__ Iv cell_forward(const WideDev &W, CellArray<GM> V, Ce
 // Sum of a value's contribution records, last user first, onto +0: the
 // accumulation order of the sequential reverse pass.  The sums are one
 // dependent chain; the loads run ahead of it.
-template <bool D, bool GM>
-__device__ __forceinline__ Iv gather_sens(CellArray<GM> R, uint32_t base, uint32_t count) {
+template <bool D, typename G>
+__device__ __forceinline__ Iv gather_sens(G R, uint32_t base, uint32_t count) {
   Iv S = iv(0.0f);
   uint32_t i = 0;
   for (; i + 8u <= count; i += 8u) {
@@ -235,14 +235,14 @@ struct WideRevSlot {
 // of its contribution records), the handler's reverse rule and the
 // operands' shares, each to its target in G: the operand's own place (one
 // user: nothing else is added to it) or this use's record.
-template <bool D, bool GM>
-__device__ __forceinline__ void wide_reverse_slot(uint32_t kind_, WideRevSlot p, CellArray<GM> V, CellArray<GM> G) {
+template <bool D, typename VArray, typename GArray>
+__device__ __forceinline__ void wide_reverse_slot(uint32_t kind_, WideRevSlot p, VArray V, GArray G) {
   using I = IA<D>;
   const float f = __uint_as_float(p.lit);
   const Iv A = V.ld(p.a), B0 = V.ld(p.b);
   const uint32_t kg = uniform_u32(kind_), kind = kg & 15u;
   Iv s;
-  if (kg & WK_GATHER) s = p.count ? gather_sens<D, GM>(G, p.src, p.count) : G.ld(p.src);
+  if (kg & WK_GATHER) s = p.count ? gather_sens<D>(G, p.src, p.count) : G.ld(p.src);
   else s = G.ld(p.src);
   // a point factor's product (exact in the directed form: the factor is 0 or
   // +-1, so one rounding mode serves both bounds)
@@ -295,37 +295,59 @@ __device__ __forceinline__ void wide_reverse_slot(uint32_t kind_, WideRevSlot p,
   G.st(p.tb, c1);
 }
 
-// Reverse interval AD over the bundles (compute.wgsl:3786-3900).  G: the
-// values' sensitivities and behind them the contribution records.  sens_out:
-// the four arguments' sensitivities, in shared memory.
-template <bool D, bool GM>
-__device__ __forceinline__ void cell_reverse(const WideDev &W, CellArray<GM> V, CellArray<GM> G, float2 *sens_out) {
+// Reverse interval AD over the bundles (compute.wgsl:3786-3900).  sens_out:
+// the four arguments' sensitivities, in shared memory.  G: the sensitivities'
+// slots, in shared memory also where the values are in the global scratch:
+// a step reads and writes them, so their round trips to L2 are what it then
+// waits for, while the values are only read.  18777-instruction tape, some
+// 5000 slots for as many values and 7850 records: 315 to 125 thousand cycles
+// a cell, inversions of the 1024-primitive animation 2.88 and 4.08 to 2.01
+// and 2.68 ms.
+template <bool D, typename VArray>
+__device__ __forceinline__ void cell_reverse16(const WideDev &W, VArray V, CellArray<false> G, float2 *sens_out) {
+  const uint32_t tid = threadIdx.x;
+  if (tid < 4u && !W.arg_gcount[tid]) G.st(W.g_arg[tid], iv(0.0f));
+  if (tid == 4u) G.st(0u, iv(0.0f));         // the zero
+  if (tid == 5u) G.st(1u, iv(0.0f));         // the dummy
+  if (tid == 6u) G.st(W.g_field, iv(1.0f));  // the field
+  __syncthreads();
+  const uint32_t nv = W.nvalues;
+  walk_steps(W, kWideWarps + (tid >> 5), W.rev16, [&](const uint4 &p, uint32_t kind) {
+    const bool ii = p.w & WC_II;
+    wide_reverse_slot<D>(kind,
+                         WideRevSlot{p.w & 0xffffu, p.x & 0xffffu, ii ? p.z : nv, p.z, p.y & 0xffffu, p.y >> 16,
+                                     p.x >> 16, p.w >> 16},
+                         V, G);
+  });
+  if (tid < 4u) {
+    const uint32_t gc = W.arg_gcount[tid];
+    const Iv s = gc ? gather_sens<D>(G, W.g_arg[tid], gc) : G.ld(W.g_arg[tid]);
+    sens_out[tid] = make_float2(s.lo, s.hi);
+  }
+  __syncthreads();
+}
+
+// The same with everything in the global scratch, by indices of 32 bits (the
+// second array's slot is read in the step).  G: the values' sensitivities and
+// behind them the contribution records.
+template <bool D>
+__device__ __forceinline__ void cell_reverse(const WideDev &W, CellArray<true> V, CellArray<true> G, float2 *sens_out) {
   const uint32_t tid = threadIdx.x;
   if (tid < 4u) G.st(tid, iv(0.0f));
   if (tid == 4u) G.st(W.nvalues, iv(0.0f));       // the zero
   if (tid == 5u) G.st(W.nvalues + 1u, iv(0.0f));  // the dummy
   if (tid == 6u) G.st(W.nvalues - 1u, iv(1.0f));  // the field
   __syncthreads();
-  const uint32_t stream = kWideWarps + (tid >> 5), nv = W.nvalues;
-  if (GM && !W.rev16) {  // indices of more than 16 bits: the second array's slot is read in the step
-    const uint4 *t = W.rev + W.rev_slots + W.streams[stream].x + (tid & 31u);
-    walk_steps(W, stream, W.rev, [&](const uint4 &p, uint32_t kind) {
-      const uint4 r = *t;
-      t += 32;
-      wide_reverse_slot<D, GM>(kind, WideRevSlot{p.x, p.y, p.z, p.w, r.x, r.y, r.z, r.w}, V, G);
-    });
-  } else {
-    walk_steps(W, stream, W.rev16, [&](const uint4 &p, uint32_t kind) {
-      const bool ii = p.w & WC_II;
-      wide_reverse_slot<D, GM>(kind,
-                               WideRevSlot{p.w & 0xffffu, p.x & 0xffffu, ii ? p.z : nv, p.z, p.y & 0xffffu, p.y >> 16,
-                                           p.x >> 16, p.w >> 16},
-                               V, G);
-    });
-  }
+  const uint32_t stream = kWideWarps + (tid >> 5);
+  const uint4 *t = W.rev + W.rev_slots + W.streams[stream].x + (tid & 31u);
+  walk_steps(W, stream, W.rev, [&](const uint4 &p, uint32_t kind) {
+    const uint4 r = *t;
+    t += 32;
+    wide_reverse_slot<D>(kind, WideRevSlot{p.x, p.y, p.z, p.w, r.x, r.y, r.z, r.w}, V, G);
+  });
   if (tid < 4u) {
     const uint32_t gc = W.arg_gcount[tid];
-    const Iv s = gc ? gather_sens<D, GM>(G, nv + 2u + W.arg_gbase[tid], gc) : G.ld(tid);
+    const Iv s = gc ? gather_sens<D>(G, W.nvalues + 2u + W.arg_gbase[tid], gc) : G.ld(tid);
     sens_out[tid] = make_float2(s.lo, s.hi);
   }
   __syncthreads();

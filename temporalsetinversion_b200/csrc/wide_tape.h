@@ -18,10 +18,14 @@
 //   reverse  x: flags, handler << 8   y: A   z: B   w: literal or factor
 //            second array: targets of A's and of B's share, the slot's own
 //            sensitivity: its place, or its first record and their count
-//   reverse, when every index has 16 bits (cells in shared memory), one array:
+//   reverse, when every index has 16 bits, one array:
 //            x: A, own sensitivity << 16   y: targets of A's, B's << 16
 //            z: B (two registers) or the literal   w: flags, handler << 8,
 //            record count << 16
+// In that form the sensitivities have slots of their own, taken when the first
+// share is written and given back after the step that reads their value's, a
+// value's records next to one another: slot 0 holds the zero, slot 1 is the
+// dummy, then come the four arguments (or their records).
 // The liveness pass walks bundles, whose slots are padded to whole warps.
 #pragma once
 #include <stdint.h>
@@ -62,6 +66,8 @@ struct WideTapeDev {
   std::vector<uint32_t> live;     // 4 words per slot: destination, min/max ordinal and WL bits, A, B (TSI_NONE: absent)
   std::vector<uint32_t> bundles;  // of `live`: first slot, slot count (a multiple of 32)
   uint32_t rev_slots = 0;         // slots of the reverse streams
+  // of rev16: the sensitivities' slots, the arguments' (first) ones, the field's
+  uint32_t gslots = 0, g_arg[4] = {0, 0, 0, 0}, g_field = 0;
 };
 void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out);
 }  // namespace tsi

@@ -36,6 +36,23 @@ def test_wide_cells_match_oracle(device, scratch_device, length, where):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("where", ["shared", "scratch"])
+def test_cells_beyond_shared_memory_match_oracle(device, scratch_device, where):
+    """Values in the global scratch: with the sensitivities in shared memory
+    (the default budget), and with them in the scratch too (no budget, more
+    slots than the register files leave room for)."""
+    tape = api.IR.new(scenes.csg(1400, 2)).gpu_instructions
+    p = api.default_params(localsubdiv=3, delta=0.02)
+    t = Tape.upload(device if where == "shared" else scratch_device, tape)
+    t.wide_threshold = 1
+    gs, os_ = Scene(t.device, t, p), oracle.Scene(tape, p)
+    for time in TIMES[:3]:
+        gs.invert(time)
+        os_.invert(time)
+        assert_cells_equal(gs.cells(), os_.cells())
+
+
+@pytest.mark.gpu
 def test_destroyed_tapes_give_their_memory_back(device):
     import torch
 
