@@ -334,27 +334,28 @@ __device__ __forceinline__ void walk_plain(const TraceParams &T, F3 ro, F3 rd, F
     f2_unpack(box.x, x0, x1);
     f2_unpack(box.y, y0, y1);
     f2_unpack(box.z, z0, z1);
-    const F3 ext = f3(x1 - x0, y1 - y0, z1 - z0);
-    const F3 num = muls((ro2 + muls(rd, hy + TEPS)) - f3(x0, y0, z0), 2.0f);
+    const F3 half = f3((x1 - x0) * 0.5f, (y1 - y0) * 0.5f, (z1 - z0) * 0.5f);
+    const F3 num = (ro2 + muls(rd, hy + TEPS)) - f3(x0, y0, z0);
     float cell0, cell1, cell2, sd0, sd1, sd2, dd0, dd1, dd2;
-    auto axis = [](float n, float e, float d, float s, float &cell, float &sd, float &dd) {
-      const float y = fm_rcp_in(e);
-      const float rol = fm_div_in(n, e, y);
-      dd = fm_rcp_in(fabsf(d * fm_div_in(2.0f, e, y)));
+    // by the half extent h: 2 n / e = n / h and 2 / e = 1 / h, exactly
+    auto axis = [](float n, float h, float d, float s, float &cell, float &sd, float &dd) {
+      const float y = fm_rcp_in(h);
+      const float rol = fm_div_in(n, h, y);
+      dd = fm_rcp_in(fabsf(d * y));
       cell = floorf(rol);
       // (s (cell - rol) + s / 2) + 1/2: the sign comes out of the first sum
       sd = __fmaf_rn(s, (cell - rol) + 0.5f, 0.5f) * dd;
     };
-    axis(num.x, ext.x, rd.x, sg.x, cell0, sd0, dd0);
-    axis(num.y, ext.y, rd.y, sg.y, cell1, sd1, dd1);
-    axis(num.z, ext.z, rd.z, sg.z, cell2, sd2, dd2);
+    axis(num.x, half.x, rd.x, sg.x, cell0, sd0, dd0);
+    axis(num.y, half.y, rd.y, sg.y, cell1, sd1, dd1);
+    axis(num.z, half.z, rd.z, sg.z, cell2, sd2, dd2);
     // the cells are small whole numbers: their sum is exact, and adding
     // 1.5 2^23 leaves it in the low bits
     int ci = __float_as_int(__fmaf_rn(4.0f, cell2, __fmaf_rn(2.0f, cell1, cell0)) + 12582912.0f) - 0x4b400000;
     float len = 0.0f;  // |mask (sd - dd)| of the last step
     const F3 old_ro2 = ro2;
     // per node: the darkening of every DDA step and the exit distance
-    const bool darken = COLOR && !T.normal_viz && fm_max(ext.x, fm_max(ext.y, ext.z)) < 1.0f;
+    const bool darken = COLOR && !T.normal_viz && fm_max(half.x, fm_max(half.y, half.z)) < 0.5f;
     const float leave = hz - TEPS;
     const float *cf = pool.f + cbase;
     go = false;
