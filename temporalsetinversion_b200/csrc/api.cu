@@ -369,9 +369,6 @@ tsi_status enqueue_invert(tsi_ctx *c, tsi_scene *const *scenes, const float *tim
     CK(cudaEventRecord(c->launch_up, c->stream));
     c->launch_up_pending = true;
   }
-  CK(cudaMemsetAsync(c->d_error, 0, n * sizeof(uint32_t), c->stream));
-  CK(cudaMemsetAsync(c->d_stats, 0, (size_t)n * ST_COUNT * sizeof(unsigned long long), c->stream));
-  CK(cudaMemsetAsync(c->d_level_stats, 0, TSI_STEP_RING * ST_COUNT * sizeof(unsigned long long), c->stream));
   const LaunchParams P = make_params(c, n, fp.smem, sticky);
   CK(launch_frame_begin(P, c->stream));
   const bool prof = c->profile_levels && c->level_events.size() >= lmax + 1;
@@ -687,22 +684,8 @@ tsi_status copy_image_out(tsi_scene *s, tsi_image *out) { return copy_image_out(
 
 tsi_status reset_scene(tsi_scene *s) {
   tsi_ctx *c = s->ctx;
-  // main.rs:749-766: root voxel 0 = root box, t 0, no children, f 0
-  const float4 xy = make_float4(s->p.root_lo[0], s->p.root_hi[0], s->p.root_lo[1], s->p.root_hi[1]);
-  const float2 z = make_float2(s->p.root_lo[2], s->p.root_hi[2]);
-  const float zero = 0.0f;
-  const uint32_t none = TSI_NONE;
-  const float4 n0 = make_float4(0, 0, 0, 0);
-  CK(cudaMemcpyAsync(s->pool.box_xy, &xy, sizeof(xy), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.box_z, &z, sizeof(z), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.t, &zero, 4, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.time_err, &zero, 4, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.f, &zero, 4, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.fast, &zero, 4, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.child, &none, 4, cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(s->pool.normal, &n0, sizeof(n0), cudaMemcpyHostToDevice, c->stream));
-  SceneCounters ctr{0, 1u, 0u, 1u};
-  CK(cudaMemcpyAsync(s->d_ctr, &ctr, sizeof(ctr), cudaMemcpyHostToDevice, c->stream));
+  // (one launch: a reset takes 12 us, with nine copies of a few bytes each 20 us)
+  CK(launch_scene_reset(s->pool, s->d_ctr, s->p.root_lo, s->p.root_hi, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return TSI_OK;
 }

@@ -20,6 +20,8 @@ namespace tsi {
 cudaError_t launch_refine(const LaunchParams &P, uint32_t step, uint32_t rcap, int grid, int block, size_t smem,
                           cudaStream_t st, bool overlap = false);
 cudaError_t launch_frame_begin(const LaunchParams &P, cudaStream_t st);
+cudaError_t launch_scene_reset(const VoxelPoolDev &pool, SceneCounters *ctr, const float lo[3], const float hi[3],
+                               cudaStream_t st);
 cudaError_t launch_step_begin(const LaunchParams &P, uint32_t step, const StepSeeds &sd, cudaStream_t st);
 cudaError_t launch_frame_end(const LaunchParams &P, uint32_t first, uint32_t count, cudaStream_t st,
                              bool overlap = false);

@@ -1639,8 +1639,10 @@ __device__ void seed_root(const LaunchParams &P, uint32_t s, uint32_t step) {
 
 
 // Per frame of the plain and batched forms (steps 0, 1, ... are the levels):
-// clear every step's lists and the tape arenas, seed the root of every scene
-// at step 0.  With n_scenes = 0 it only clears (the continuous form's start).
+// clear every step's lists, the tape arenas and the scenes' error words and
+// counters (a memset each cost a frame 2 us more), seed the root of every
+// scene at step 0.  With n_scenes = 0 it only clears (the continuous form's
+// start).
 __global__ void frame_begin_kernel(const __grid_constant__ LaunchParams P) {
   const uint32_t t = threadIdx.x;
   grid_dependents_launch();  // the first level's launch may begin
@@ -1651,8 +1653,26 @@ __global__ void frame_begin_kernel(const __grid_constant__ LaunchParams P) {
     *P.rec_low = 0;
     *P.code_low = 0;
   }
+  for (uint32_t i = t; i < P.n_scenes; i += blockDim.x) P.error[i] = 0;
+  for (uint32_t i = t; i < P.n_scenes * ST_COUNT; i += blockDim.x) P.stats[i] = 0;
+  if (P.level_stats)
+    for (uint32_t i = t; i < TSI_STEP_RING * ST_COUNT; i += blockDim.x) P.level_stats[i] = 0;
   __syncthreads();
   for (uint32_t s = t; s < P.n_scenes; s += blockDim.x) seed_root(P, s, 0u);
+}
+
+// An empty octree (main.rs:749-766): root voxel 0 = root box, t 0, no
+// children, f 0; no brick but the root's in use.
+__global__ void scene_reset_kernel(VoxelPoolDev pool, SceneCounters *ctr, float4 xy, float2 z) {
+  pool.box_xy[0] = xy;
+  pool.box_z[0] = z;
+  pool.t[0] = 0.0f;
+  pool.time_err[0] = 0.0f;
+  pool.f[0] = 0.0f;
+  pool.fast[0] = 0.0f;
+  pool.child[0] = TSI_NONE;
+  pool.normal[0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  *ctr = SceneCounters{0, 1u, 0u, 1u};
 }
 
 // Start of a step of the continuous form at which slots join: record the
@@ -1736,7 +1756,12 @@ cudaError_t launch_refine(const LaunchParams &P, uint32_t step, uint32_t rcap, i
   return cudaLaunchKernelEx(&lc.cfg, refine_kernel, P, step, rcap);
 }
 cudaError_t launch_frame_begin(const LaunchParams &P, cudaStream_t st) {
-  frame_begin_kernel<<<1, 64, 0, st>>>(P);
+  frame_begin_kernel<<<1, 256, 0, st>>>(P);
+  return cudaGetLastError();
+}
+cudaError_t launch_scene_reset(const VoxelPoolDev &pool, SceneCounters *ctr, const float lo[3], const float hi[3],
+                               cudaStream_t st) {
+  scene_reset_kernel<<<1, 1, 0, st>>>(pool, ctr, make_float4(lo[0], hi[0], lo[1], hi[1]), make_float2(lo[2], hi[2]));
   return cudaGetLastError();
 }
 cudaError_t launch_step_begin(const LaunchParams &P, uint32_t step, const StepSeeds &sd, cudaStream_t st) {
