@@ -72,7 +72,14 @@ __global__ void __launch_bounds__(32 * kTraceWarps, 32 / kTraceWarps) trace_kern
     cr = cg = cb = 10.0f;
     ca = 0.0f;
   }
-  if (valid && T.rgba) T.rgba[pix] = make_float4(fm_powf(cr, 0.45f), fm_powf(cg, 0.45f), fm_powf(cb, 0.45f), ca);
+  if (T.rgba) {
+    // the channels of a warp without a hit are one number each, the age
+    // colour's green and blue are: a power costs some hundred instructions
+    const float pr = fm_powf(cr, 0.45f);
+    const float pg = __all_sync(FULL_MASK, cg == cr) ? pr : fm_powf(cg, 0.45f);
+    const float pb = __all_sync(FULL_MASK, cb == cg) ? pg : fm_powf(cb, 0.45f);
+    if (valid) T.rgba[pix] = make_float4(pr, pg, pb, ca);
+  }
   if (valid && T.depth) T.depth[pix] = dist;
   if (valid && T.normal) {
     T.normal[pix * 3 + 0] = nrm.x;
