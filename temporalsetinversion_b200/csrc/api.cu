@@ -134,6 +134,7 @@ LaunchParams make_params(tsi_ctx *c, uint32_t n_scenes, size_t dyn_smem, bool st
   P.error = c->d_error;
   P.stats = c->d_stats;
   P.level_stats = c->d_level_stats;
+  P.live = c->d_live;
   return P;
 }
 
@@ -395,12 +396,16 @@ tsi_status ensure_readback_rows(tsi_ctx *c, uint32_t n) {
   CK(cudaStreamSynchronize(c->stream));
   cudaFreeHost(c->h_err);
   cudaFreeHost(c->h_stats);
+  cudaFreeHost(c->h_live);
   c->h_err = nullptr;
   c->h_stats = nullptr;
+  c->h_live = nullptr;
   c->rb_rows = 0;
   const uint32_t rows = std::max(n, 64u);
   CK(cudaMallocHost((void **)&c->h_err, rows * sizeof(uint32_t)));
   CK(cudaMallocHost((void **)&c->h_stats, (size_t)rows * ST_COUNT * sizeof(unsigned long long)));
+  CK(cudaMallocHost((void **)&c->h_live, rows * sizeof(uint32_t)));
+  memset(c->h_live, 0, rows * sizeof(uint32_t));
   memset(c->h_err, 0, rows * sizeof(uint32_t));
   memset(c->h_stats, 0, (size_t)rows * ST_COUNT * sizeof(unsigned long long));
   c->rb_rows = rows;
@@ -414,6 +419,7 @@ tsi_status enqueue_readback(tsi_ctx *c, uint32_t n, uint32_t row0 = 0) {
   CK(cudaMemcpyAsync(c->h_err + row0, c->d_error, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(c->h_stats + (size_t)row0 * ST_COUNT, c->d_stats, (size_t)n * ST_COUNT * sizeof(unsigned long long),
                      cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(c->h_live + row0, c->d_live, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(c->h_rb->item_count, c->d_item_count, sizeof(c->h_rb->item_count), cudaMemcpyDeviceToHost,
                      c->stream));
   return TSI_OK;
@@ -943,6 +949,7 @@ TSI_API tsi_status tsi_create(const tsi_device_opts *opts, tsi_ctx **out) {
   CKC(cudaMemset(c->d_error_sticky, 0, sizeof(uint32_t)));
   CKC(dalloc(&c->d_stats, (size_t)c->max_scenes * ST_COUNT));
   CKC(dalloc(&c->d_level_stats, (size_t)TSI_STEP_RING * ST_COUNT));
+  CKC(dalloc(&c->d_live, c->max_scenes));
   c->fork_events.resize(TSI_STEP_RING);
   for (auto &ev : c->fork_events) CKC(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CKC(cudaEventCreateWithFlags(&c->join_event, cudaEventDisableTiming));
@@ -1007,6 +1014,7 @@ TSI_API void tsi_destroy(tsi_ctx *c) {
   cudaFree(c->d_error_sticky);
   cudaFree(c->d_stats);
   cudaFree(c->d_level_stats);
+  cudaFree(c->d_live);
   for (auto &ev : c->level_events) cudaEventDestroy(ev);
   for (auto &ev : c->fork_events) cudaEventDestroy(ev);
   if (c->join_event) cudaEventDestroy(c->join_event);
@@ -1014,6 +1022,7 @@ TSI_API void tsi_destroy(tsi_ctx *c) {
   cudaFree(c->d_scratch);
   cudaFreeHost(c->h_rb);
   cudaFreeHost(c->h_err);
+  cudaFreeHost(c->h_live);
   cudaFreeHost(c->h_stats);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->launch_up) cudaEventDestroy(c->launch_up);
@@ -1364,10 +1373,7 @@ TSI_API tsi_status tsi_scene_invert(tsi_scene *s, float time, float t0_or_nan, t
   float ms = 0.0f;
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   if (stats) {
-    SceneCounters ctr;
-    st = read_counters(s, ctr);
-    if (st != TSI_OK) return st;
-    fill_stats(c, 0, s, stats, (uint64_t)ctr.live_bricks * 8u);
+    fill_stats(c, 0, s, stats, (uint64_t)c->h_live[0] * 8u);
     stats->device_ms = ms;
   }
   return status_from_error_bits(c->h_err[0]);
@@ -2003,10 +2009,7 @@ TSI_API tsi_status tsi_batch_run(tsi_ctx *c, tsi_request *reqs, uint32_t n) {
   for (uint32_t i = 0; i < n; ++i) {
     err |= c->h_err[i];
     if (reqs[i].stats) {
-      SceneCounters ctr;
-      st = read_counters(reqs[i].scene, ctr);
-      if (st != TSI_OK) return st;
-      fill_stats(c, i, reqs[i].scene, reqs[i].stats, (uint64_t)ctr.live_bricks * 8u);
+      fill_stats(c, i, reqs[i].scene, reqs[i].stats, (uint64_t)c->h_live[i] * 8u);
       reqs[i].stats->device_ms = ms;
     }
   }

@@ -131,6 +131,7 @@ struct tsi_ctx {
   cudaEvent_t launch_up = nullptr;
   bool launch_up_pending = false;
   unsigned long long *d_stats = nullptr;        // [max_scenes][ST_COUNT]
+  uint32_t *d_live = nullptr, *h_live = nullptr;  // [max_scenes], [rb_rows]
   unsigned long long *d_level_stats = nullptr;  // [TSI_STEP_RING][ST_COUNT]
   unsigned long long *d_visits = nullptr;
   TsiReadback *h_rb = nullptr;

@@ -237,6 +237,7 @@ struct LaunchParams {
   uint32_t *long_count;             // [TSI_STEP_RING]: items of tapes at least the wide threshold long
   uint32_t *error;                  // [n_scenes]: error bits of each scene
   unsigned long long *stats;        // [n_scenes][ST_COUNT]: counters of each scene
+  uint32_t *live;                   // [n_scenes]: bricks in use at the end of a frame, or null
   unsigned long long *level_stats;  // [TSI_STEP_RING][ST_COUNT], per refine launch, or null
 };
 

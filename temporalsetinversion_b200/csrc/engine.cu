@@ -184,6 +184,7 @@ tsi_status Engine::step() {
   sd.oldest = (uint32_t)oldest;
   LaunchParams P = make_params(c_, (uint32_t)slots_.size(), plan_.smem, false);
   P.level_stats = nullptr;
+  P.live = nullptr;
   if (sd.n) ECK(tsi::launch_step_begin(P, (uint32_t)s, sd, c_->stream));
   ECK(tsi::launch_refine(P, (uint32_t)s, plan_.rcap, plan_.grid, kBlock, plan_.smem, c_->stream));
   const cudaEvent_t done = step_ev_[s % kStepRing];
@@ -205,7 +206,8 @@ tsi_status Engine::finish_slot(uint32_t i, cudaEvent_t after) {
   tsi_scene *sc = s.req.scene;
   const cudaStream_t ts = c_->trace_stream;
   ECK(cudaStreamWaitEvent(ts, after, 0));
-  const LaunchParams P = make_params(c_, (uint32_t)slots_.size(), plan_.smem, false);
+  LaunchParams P = make_params(c_, (uint32_t)slots_.size(), plan_.smem, false);
+  P.live = nullptr;  // the slots' counters are read back whole
   ECK(tsi::launch_frame_end(P, i, 1, ts));
   s.inverting = false;
   --ninv_;

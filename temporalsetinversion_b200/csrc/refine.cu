@@ -1726,6 +1726,8 @@ __global__ void frame_end_kernel(const __grid_constant__ LaunchParams P, uint32_
     c->pending_count = 0;
     uint32_t used = min(c->bump, S.pool.cap_bricks);
     c->live_bricks = used - (uint32_t)(fc0 + (int32_t)np);
+    // read back with the counters: the host needs no copy of its own for it
+    if (P.live) P.live[s] = c->live_bricks;
   }
 }
 
