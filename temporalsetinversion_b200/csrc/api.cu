@@ -68,6 +68,7 @@ struct tsi_batch_graph {
   cudaGraphExec_t exec = nullptr;
   bool launched = false;
   std::vector<uint8_t> global;  // per request: wide cells in the global scratch
+  std::shared_ptr<unsigned char> wscratch;  // that scratch, which a later plan of the context may replace
 };
 
 namespace tsi_host {
@@ -314,10 +315,11 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
     const size_t stride = (gm_bytes + 255) & ~size_t(255);
     const size_t need = stride * (size_t)fp.grid;
     if (need > c->wscratch_bytes) {
-      cudaFree(c->d_wscratch);
+      c->wscratch.reset();
       c->d_wscratch = nullptr;
       c->wscratch_bytes = 0;
       CK(dalloc(&c->d_wscratch, need));
+      c->wscratch.reset(c->d_wscratch, [](unsigned char *q) { cudaFree(q); });
       c->wscratch_bytes = need;
     }
     c->wscratch_stride = stride;
@@ -1000,7 +1002,7 @@ TSI_API void tsi_destroy(tsi_ctx *c) {
   cudaFree(c->d_witem_count);
   cudaFree(c->d_witem_cursor);
   for (int q = 0; q < 2; ++q) cudaFree(c->d_cell_info[q]);
-  cudaFree(c->d_wscratch);
+  c->wscratch.reset();
   cudaFree(c->d_dealloc[0]);
   cudaFree(c->d_dealloc[1]);
   cudaFree(c->d_dealloc_count);
@@ -2104,6 +2106,7 @@ TSI_API tsi_status tsi_batch_graph_create(tsi_ctx *c, tsi_request *reqs, uint32_
       return pst;
     }
     g->global = fp.global;  // the captured launches' choice, re-applied at every replay
+    g->wscratch = c->wscratch;
   }
   for (uint32_t i = 0; i < n; ++i) {
     const tsi_status dst = drain_copy(reqs[i].scene);  // no outside event inside the capture

@@ -8,6 +8,7 @@
 
 #include <set>
 #include <string>
+#include <memory>
 #include <vector>
 
 #include "device_types.h"
@@ -108,7 +109,8 @@ struct tsi_ctx {
   uint32_t *d_cell_bits[2] = {nullptr, nullptr};
   size_t cell_arena_bytes = 0;  // of each parity's info + bits
   uint32_t witem_cap = 0, bm_words = 0;
-  unsigned char *d_wscratch = nullptr;
+  unsigned char *d_wscratch = nullptr;          // *wscratch
+  std::shared_ptr<unsigned char> wscratch;      // captured graphs keep the one that their launches name
   size_t wscratch_bytes = 0, wscratch_stride = 0;
   size_t wide_smem_bytes = 0;  // shared-memory budget of a wide cell (0: keep the narrow occupancy)
   uint64_t hbm_budget = 0;     // bytes the scenes may hold together (0: no limit)

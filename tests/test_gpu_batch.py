@@ -71,3 +71,28 @@ def test_graph_replays_equal_plain_frames(device):
                 assert np.array_equal(got["rgba"], want["rgba"])
     finally:
         g.close()
+
+
+@pytest.mark.gpu
+def test_graph_survives_a_larger_scratch():
+    """A graph whose cells live in the context's global scratch replays after a
+    scene with larger cells has had that scratch replaced."""
+    from temporalsetinversion_b200 import Device
+
+    dev = Device()
+    try:
+        p = api.default_params(localsubdiv=3, delta=0.02)
+        small = Tape.from_llvm_ir(dev, scenes.csg(700, 2))
+        a, b = Scene(dev, small, p), Scene(dev, small, p)
+        g = api.BatchGraph(dev, [(a, 0.0, float("nan"), None)])
+        big = Tape.from_llvm_ir(dev, scenes.csg(1400, 2))
+        c = Scene(dev, big, p)
+        c.invert(0.0)
+        for t in (0.0, 0.05):
+            g.launch([t])
+            g.wait()
+            b.invert(t)
+            assert_cells_equal(a.cells(), b.cells())
+        g.close()
+    finally:
+        dev.close()
