@@ -35,6 +35,12 @@ struct TraceParams {
 };
 
 // T: the host copy (grid size, variant); Tdev: the same in device memory, read by the kernel.
-cudaError_t launch_trace(const TraceParams &T, const TraceParams *Tdev, cudaStream_t st);
+// The frames of one launch, by device address (one per blockIdx.z).
+constexpr uint32_t kTraceBatch = 64;
+struct TraceBatch {
+  const TraceParams *T[kTraceBatch];
+};
+// Traces n frames, T[i] the host's copy of the one at Tdev[i].
+cudaError_t launch_traces(const TraceParams *const *T, const TraceParams *const *Tdev, uint32_t n, cudaStream_t st);
 
 }  // namespace tsi

@@ -96,3 +96,29 @@ def test_graph_survives_a_larger_scratch():
         g.close()
     finally:
         dev.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 5, 65])
+def test_frames_of_one_launch_equal_their_own(device, n):
+    """Frames traced together: sizes that are no multiple of a block's tile,
+    down to one pixel, field normals and path tracing among them, and one more
+    scene than a launch takes."""
+    sizes = [(96, 64), (33, 17), (1, 1), (17, 9), (64, 8)]
+    kinds = [dict(), dict(fast_normals=1), dict(cinematic=1, samples=2), dict(normal_viz=1), dict()]
+    texts = [scenes.csg(16, 1, 0.9), scenes.spheres16(2)]
+    tapes = [Tape.from_llvm_ir(device, t) for t in texts]
+    cam = scenes.camera_look_at((0.4, 0.8, 2.4))
+    reqs, alone = [], []
+    for i in range(n):
+        p = api.default_params(localsubdiv=4 + i % 2, **kinds[i % 5])
+        u = api.make_uniforms(cam, sizes[i % 5], 0.1)
+        reqs.append((Scene(device, tapes[i % 2], p, 1 << 14), 0.1, math.nan, u))
+        if i < 10 or i == n - 1:
+            s = Scene(device, tapes[i % 2], p, 1 << 14)
+            s.invert(0.1)
+            alone.append((i, s.trace(u)))
+    res = api.run_batch(device, reqs)
+    for i, img in alone:
+        for k in ("depth", "rgba", "normal"):
+            assert np.array_equal(res[i][k], img[k], equal_nan=True)
