@@ -2,10 +2,10 @@
 //
 // One launch per octree level, over every scene of the launch.  A warp takes
 // one work item: up to four sibling parents (children of one grandparent,
-// sharing one tape record) x 8 octants, one child cell per lane.  The tape is
-// warp-uniform, so instruction fetch is a broadcast and the handler switch
-// never diverges.  Interval registers live in shared memory as
-// regs[register][lane] (one column per lane, conflict free).
+// sharing one tape record) x 8 octants, one child cell per lane
+// (narrow_interp.cuh: interval registers in shared memory, a column per
+// cell).  While a level has blocks enough for its cells, items of long tapes
+// go to the wide path instead, one block per cell (wide_interp.cuh).
 //
 // Per child cell the lane runs, as in the reference:
 //   cell setup and temporal interval         compute.wgsl:3582-3626

@@ -79,7 +79,7 @@ static __device__ __noinline__ void tape_values_general(const TraceParams &T, ui
     const float kx = (q == 0 || q == 3) ? 1.0f : -1.0f, ky = q >= 2 ? 1.0f : -1.0f, kz = (q & 1) ? 1.0f : -1.0f;
     __syncwarp();
     const Iv r = forward_pass<false>(T.code, T.len, T.out_reg, rf, lane, iv(p.x + kx * h), iv(p.y + ky * h),
-                                     iv(p.z + kz * h), iv(t), nullptr, nullptr);
+                                     iv(p.z + kz * h), iv(t));
     f[q] = r.lo;
   }
 }
