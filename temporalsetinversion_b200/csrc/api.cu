@@ -169,6 +169,9 @@ WideDev wide_dev(const tsi_tape *t) {
   W.fwd = t->d_wfwd;
   W.rev = t->d_wrev;
   W.rev16 = t->d_wrev16;
+  W.fwd_slots = t->d_wfwd_slots;
+  W.fslots = t->wfslots;
+  W.f_field = t->wf_field;
   W.live = t->d_wlive;
   W.bundles = t->d_wbundles;
   W.narrow_mm = t->d_wmm;
@@ -295,9 +298,11 @@ tsi_status plan_frame(tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, FramePla
     if (b > budget || !t->d_wrev16) {
       fp.global[i] = 1;
       gm_bytes = std::max(gm_bytes, wide_cell_bytes(t->wvalues, nv2 + t->wcontrib, bm_words));
-      // the sensitivities' slots in shared memory all the same, if they fit
-      const size_t g = (size_t)t->wgslots * 8;
+      // the sensitivities' slots in shared memory all the same, and those of
+      // the forward values over two time intervals, if they fit
+      const size_t g = (size_t)t->wgslots * 8, f = (size_t)t->wfslots * 16;
       if (t->d_wrev16 && g <= budget) cell_bytes = std::max(cell_bytes, g);
+      if (t->d_wfwd_slots && f <= budget) cell_bytes = std::max(cell_bytes, f);
     } else {
       cell_bytes = std::max(cell_bytes, b);
     }
@@ -1101,6 +1106,9 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
       up(&t->d_wfwd, dv.fwd);
       up(&t->d_wrev, dv.rev);
       up(&t->d_wrev16, dv.rev16);
+      up(&t->d_wfwd_slots, dv.fwd_slots);
+      t->wfslots = dv.fslots;
+      t->wf_field = dv.f_field;
       up(&t->d_wlive, dv.live);
       up(&t->d_wctl, dv.ctl);
       up(&t->d_wstreams, dv.streams);

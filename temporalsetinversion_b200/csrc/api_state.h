@@ -48,6 +48,7 @@ struct tsi_tape {
   bool strict = false;  // PackedTape::strict
   // bundled form for the wide path (absent when the tape is short)
   uint4 *d_wfwd = nullptr, *d_wrev = nullptr, *d_wlive = nullptr, *d_wrev16 = nullptr;
+  uint4 *d_wfwd_slots = nullptr;
   uint2 *d_wstreams = nullptr;
   uint32_t *d_wctl = nullptr;
   uint2 *d_wbundles = nullptr;
@@ -57,6 +58,7 @@ struct tsi_tape {
   uint32_t narrow_parents = 1;  // parents per narrow item above the leaf level
   uint32_t wprune_level = 0xffffffffu;  // first level whose wide groups prune (0xffffffff: half the levels)
   uint32_t warg_gbase[4] = {TSI_NONE, TSI_NONE, TSI_NONE, TSI_NONE}, warg_gcount[4] = {0, 0, 0, 0};
+  uint32_t wfslots = 0, wf_field = 0;
   uint32_t wgslots = 0, wg_arg[4] = {0, 0, 0, 0}, wg_field = 0;
 };
 

@@ -77,6 +77,7 @@ struct SceneCounters {
 struct WideDev {
   const uint4 *fwd, *rev;     // the streams' slots (wide_tape.h)
   const uint4 *rev16;         // null: some index needs more than 16 bits
+  const uint4 *fwd_slots;     // null: none (wide_tape.h)
   const uint32_t *ctl;        // the streams' step bytes
   const uint2 *streams;       // [16]
   const uint4 *live;          // bundle by bundle, for the liveness pass
@@ -95,6 +96,7 @@ struct WideDev {
   uint32_t arg_gbase[4];      // records of x, y, z, t (TSI_NONE: one user)
   uint32_t arg_gcount[4];
   uint32_t gslots, g_arg[4], g_field;  // the sensitivities' slots of rev16
+  uint32_t fslots, f_field;            // the values' slots of fwd_slots
 };
 
 struct SceneLaunch {

@@ -1197,6 +1197,7 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
     }
   }
   const CellArray<GM> V(cell), G(cell + L.sens);
+  const bool slots = GM && W.fwd_slots && W.fslots * 16u <= P.dyn_smem;  // forward values in shared memory
   uint8_t *dec = cell + L.dec, *dec2 = cell + L.flags;
   const float4 pxy = pool.box_xy[Pv];
   const float2 pz = pool.box_z[Pv];
@@ -1289,7 +1290,14 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
   Iv sens[4] = {iv(0.0f), iv(0.0f), iv(0.0f), iv(0.0f)};
   if (evaluate) {
     const long long c0 = clock64();
-    field = cell_forward<D, GM>(W, V, G, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz, targ, Iv{wl, wh});
+    if constexpr (GM) {
+      if (slots)
+        field = cell_forward_slots<D>(W, tsi_dyn_smem, V, take_deriv, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz,
+                                      targ, Iv{wl, wh});
+      else field = cell_forward<D, GM>(W, V, G, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz, targ, Iv{wl, wh});
+    } else {
+      field = cell_forward<D, GM>(W, V, G, dual, want_prune ? dec : nullptr, dec2, cx, cy, cz, targ, Iv{wl, wh});
+    }
     const long long c1 = clock64();
     if (take_deriv) {
       if constexpr (GM) {
@@ -1405,7 +1413,13 @@ __device__ __noinline__ void process_cell(const LaunchParams &P, WorkItem *itp, 
       dec = dec2;
     } else {
       const long long r0 = clock64();
-      (void)cell_forward<D, GM>(W, V, G, false, dec, nullptr, cx, cy, cz, Iv{nl, nh}, targ);
+      if constexpr (GM) {
+        if (slots)
+          (void)cell_forward_slots<D>(W, tsi_dyn_smem, V, false, false, dec, nullptr, cx, cy, cz, Iv{nl, nh}, targ);
+        else (void)cell_forward<D, GM>(W, V, G, false, dec, nullptr, cx, cy, cz, Iv{nl, nh}, targ);
+      } else {
+        (void)cell_forward<D, GM>(W, V, G, false, dec, nullptr, cx, cy, cz, Iv{nl, nh}, targ);
+      }
       if (tid == 0) {
         ws[ST_WIDE_REFWD] += 1ull;
         ws[ST_CYC_WIDE_REFWD] += (unsigned long long)(clock64() - r0);

@@ -499,6 +499,40 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
     }
     out.gslots = pool.top;
   }
+  // ---- the forward values' slots
+  std::vector<uint32_t> fplace;  // (of the zero and the dummy too)
+  if (nv >= kForwardSlotsMin) {
+    fplace.assign(nv2, 0u);
+    fplace[dummy] = 1u;
+    std::vector<uint32_t> last_use(nv, 0u);
+    for (uint32_t k = 0; k < wt.nbundles; ++k)
+      for (uint32_t s = wt.bundles[2 * k], e = s + wt.bundles[2 * k + 1]; s < e; ++s) {
+        const uint32_t *S = &wt.slots[size_t(s) * 12];
+        if ((S[0] & 63u) == TSI_H_PAD) continue;
+        if (S[6] != TSI_NONE) last_use[S[6]] = k;
+        if (S[7] != TSI_NONE) last_use[S[7]] = k;
+      }
+    SlotPool pool;
+    pool.take(2);
+    for (uint32_t q = 0; q < 4u; ++q) fplace[q] = pool.take(1);
+    std::vector<std::vector<uint32_t>> ends(wt.nbundles);  // the values read for the last time in a bundle
+    for (uint32_t v = 4; v + 1u < nv; ++v)
+      if (used[v]) ends[last_use[v]].push_back(v);
+    for (uint32_t k = 0; k < wt.nbundles; ++k) {
+      std::vector<uint32_t> unread;
+      for (uint32_t s = wt.bundles[2 * k], e = s + wt.bundles[2 * k + 1]; s < e; ++s) {
+        const uint32_t *S = &wt.slots[size_t(s) * 12];
+        if ((S[0] & 63u) == TSI_H_PAD) continue;
+        fplace[S[4]] = pool.take(1);
+        if (!used[S[4]] && S[4] != nv - 1u) unread.push_back(S[4]);
+      }
+      for (uint32_t v : ends[k]) pool.give(fplace[v], 1);
+      for (uint32_t v : unread) pool.give(fplace[v], 1);
+    }
+    out.fslots = pool.top;
+    out.f_field = fplace[nv - 1u];
+    if (out.fslots > 65536u) fplace.clear();
+  }
   const bool small = nv2 <= 65536u && out.gslots <= 65536u;  // (a value's records are as many as its users)
   // One group (warp g of bundle k) of the forward or reverse streams; its
   // kind.
@@ -549,6 +583,9 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
           default: break;
         }
         push4(out.fwd, c | ((pad ? dummy : S[4]) << WC_DST_SHIFT), x, y, w);
+        if (!fplace.empty())
+          push4(out.fwd_slots, c | ((pad ? dummy : S[4]) << WC_DST_SHIFT),
+                fplace[x] | (fplace[pad ? dummy : S[4]] << 16), ii ? fplace[y] : y, w);
         continue;
       }
       if (h == H_SUB_II) c |= WC_NEG2;
@@ -594,6 +631,7 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
   // a warp reads one slot past its last group's
   for (uint32_t s = 0; s < 32u; ++s) {
     push4(out.fwd, dummy << WC_DST_SHIFT, zero, zero, 0u);
+    if (!fplace.empty()) push4(out.fwd_slots, dummy << WC_DST_SHIFT, 1u << 16, zero, 0u);
     push4(out.rev, 0u, zero, zero, 0u);
     push4(targets, dummy, dummy, zero, 0u);
     if (small) push4(out.rev16, zero, 1u | (1u << 16), 0u, 0u);

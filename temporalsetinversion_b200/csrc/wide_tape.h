@@ -26,6 +26,12 @@
 // share is written and given back after the step that reads their value's, a
 // value's records next to one another: slot 0 holds the zero, slot 1 is the
 // dummy, then come the four arguments (or their records).
+// For cells whose values are in the global scratch (long tapes), the forward
+// slots once more with the values in slots of shared memory, taken at their
+// definition and given back after the step of their last use (0 the zero, 1
+// the dummy, 2 to 5 the arguments):
+//            x: as above (the destination for the reverse pass)   y: A's slot,
+//            the result's << 16   z: B's slot, or as above   w: as above
 // The liveness pass walks bundles, whose slots are padded to whole warps.
 #pragma once
 #include <stdint.h>
@@ -66,8 +72,12 @@ struct WideTapeDev {
   std::vector<uint32_t> live;     // 4 words per slot: destination, min/max ordinal and WL bits, A, B (TSI_NONE: absent)
   std::vector<uint32_t> bundles;  // of `live`: first slot, slot count (a multiple of 32)
   uint32_t rev_slots = 0;         // slots of the reverse streams
+  std::vector<uint32_t> fwd_slots;  // the forward slots with shared-memory slots (empty: none)
+  uint32_t fslots = 0, f_field = 0;  // of fwd_slots: the values' slots, the field's
   // of rev16: the sensitivities' slots, the arguments' (first) ones, the field's
   uint32_t gslots = 0, g_arg[4] = {0, 0, 0, 0}, g_field = 0;
 };
+// Tapes of at least this many values get fwd_slots.
+constexpr uint32_t kForwardSlotsMin = 6144;
 void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out);
 }  // namespace tsi
