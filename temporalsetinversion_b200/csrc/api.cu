@@ -226,6 +226,7 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
   L.wide = wide_dev(s->tape);
   L.wide.prune_level = s->tape->wprune_level != 0xffffffffu ? s->tape->wprune_level : tree_levels(p) / 2u;
   L.wide.global = wide_global ? 1u : 0u;
+  L.wide.directed = p.rounding_mode == TSI_ROUND_DIRECTED ? 1u : 0u;
   R.code = s->tape->d_code;
   R.len = s->tape->len;
   R.nregs = s->tape->nregs;

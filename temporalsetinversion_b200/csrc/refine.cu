@@ -175,10 +175,13 @@ __device__ __forceinline__ uint32_t wide_min_len(const WideDev &W, uint32_t leve
 // of thousands of long items ran one block per cell.  Rotating swept scene
 // (64 primitives, localsubdiv 9) 8.0 to 2.7 ms an inversion, 1024 primitives
 // (localsubdiv 9) 3.7 to 3.3 ms, 256 primitives unchanged; half and twice
-// the multiplier measured 3.1 and 2.7 ms, 3.6 and 3.2 ms, and 5% more for a
-// directed scene of 64 primitives.
+// the multiplier measured 3.1 and 2.7 ms, 3.6 and 3.2 ms.  Directed, a
+// one-warp item costs two to four times as much an instruction (outward
+// rounding has no packed form, and its sines no short one) and the length
+// decides alone: rotating swept scenes of 44 and 64 primitives, localsubdiv 8,
+// three inversions 10.6 and 19.8 ms so, 15.3 and 23.0 with the waves.
 __device__ __forceinline__ uint32_t route_len(const LaunchParams &P, const WideDev &W, uint32_t step, uint32_t level) {
-  const uint32_t waves = max(1u, 8u * P.long_count[step & TSI_STEP_MASK] / gridDim.x);
+  const uint32_t waves = W.directed ? 1u : max(1u, 8u * P.long_count[step & TSI_STEP_MASK] / gridDim.x);
   return (uint32_t)min((unsigned long long)wide_min_len(W, level) * waves, 0xffffffffull);
 }
 
