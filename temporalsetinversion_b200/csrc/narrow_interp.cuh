@@ -276,6 +276,7 @@ __device__ __noinline__ Iv narrow_forward(const uint2 *__restrict__ code, uint32
     const uint32_t other = __ballot_sync(FULL_MASK, lane >= n || !(dec.x & NC_LIN));
     const NarrowKinds K = narrow_kinds(dec.x);
     nxt = load_chunk(code, len, (int)(c0 / 32u) + 1, lane);  // a chunk ahead
+    __syncwarp();  // (votes order no memory)
     uint32_t j = 0;
     uint4 w = prog_ld(R, 0);
     while (j < n) {
@@ -430,6 +431,7 @@ __device__ __noinline__ void narrow_reverse(const uint2 *__restrict__ code, uint
     const uint32_t other = __ballot_sync(FULL_MASK, !(dec.x & NC_LIN));
     const NarrowKinds K = narrow_kinds(dec.x);
     nxt = load_chunk(code, len, k - 1, lane);
+    __syncwarp();  // (votes order no memory)
     int j = n - 1;
     uint4 w = prog_ld(R, (uint32_t)j);
     while (j >= 0) {
