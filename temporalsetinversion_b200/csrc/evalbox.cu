@@ -37,33 +37,30 @@ __device__ __forceinline__ void store_box(float *o, Iv f, const Iv sens[4]) {
   }
 }
 
-// Boxes a warp takes: a row's offset has 16 bits, the sink's included.
-inline __host__ __device__ uint32_t narrow_boxes(uint32_t nregs) { return nregs < 256u ? 32u : 16u; }
-inline size_t narrow_bytes(uint32_t nregs) {
-  return ((size_t)(nregs + 1u) * narrow_boxes(nregs) * 8u + 15u & ~size_t(15)) + 32u * 16u;
-}
-
-// One warp, up to 32 boxes; the rows have exactly as many columns, and the
-// lanes without a box repeat the last one (they write what its lane writes).
+// One warp, up to 32 boxes, each in a column of its own (evalbox.h).  The
+// lanes without a box work on the last one in a column that no box has: a
+// lane that ran ahead in a shared one would change what the others still
+// read.  Their operands go to one place behind the log, read as anything.
 // 60000 boxes on a 4697-instruction tape with sensitivities: a call takes
 // 12.8 ms with a thread per box, 2.5 ms so.
 template <bool D>
 __global__ void __launch_bounds__(32) evalbox_narrow(EvalTape T, uint32_t n, const float *__restrict__ boxes,
                                                      int reverse, float *__restrict__ out, float4 *log) {
   const uint32_t lane = threadIdx.x, per = narrow_boxes(T.nregs);
-  const size_t first = (size_t)blockIdx.x * per;
+  const size_t first = (size_t)blockIdx.x * per, len = max(T.len, 1u);
   const uint32_t cols = (uint32_t)min((size_t)per, (size_t)n - first);
   NarrowRows R;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(evalbox_smem);
-  R.stride = cols * 8u;
-  R.col = min(lane, cols - 1u);
-  R.rf = base + R.col * 8u;
+  R.stride = narrow_columns(T.nregs) * 8u;
+  R.rf = base + narrow_column(T.nregs, lane) * 8u;
   R.sink = T.nregs * R.stride;
   R.prog = base + ((R.sink + R.stride + 15u) & ~15u);
-  const size_t box = first + R.col;
+  R.log_step = lane < cols ? cols : 0u;
+  const size_t box = first + min(lane, cols - 1u);
   Iv v[4], sens[4] = {iv(0.0f), iv(0.0f), iv(0.0f), iv(0.0f)};
   load_box(boxes + box * 8u, v);
-  float4 *lg = reverse ? log + first * max(T.len, 1u) : nullptr;  // `cols` columns of at most len entries
+  // `cols` columns of at most len entries
+  float4 *lg = !reverse ? nullptr : lane < cols ? log + first * len + lane : log + n * len;
   uint32_t nlog = 0;
   const Iv f = narrow_forward<D>(T.code, T.len, T.out_reg, R, lane, v[0], v[1], v[2], v[3], lg, nullptr, nlog);
   if (reverse) {
@@ -114,8 +111,7 @@ __global__ void math_kernel(int which, uint32_t n, const float *a, const float *
   out[i] = r;
 }
 
-// Most dynamic shared memory the kernels are launched with.
-constexpr size_t kNarrowMax = 66u << 10, kWideMax = 200u << 10;
+constexpr size_t kWideMax = 200u << 10;  // most dynamic shared memory of a block per box
 
 template <bool D>
 static cudaError_t launch(const EvalTape &t, uint32_t n, const float *boxes, bool reverse, float *out, float4 *log,

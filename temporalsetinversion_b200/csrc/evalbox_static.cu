@@ -19,9 +19,10 @@
 #include "evalbox.h"
 #include "tsi.h"
 
-// Scratch of every call: len operand-log entries (16 bytes each) per box.
-// (The call's limit counts nregs intervals of 8 bytes per box too, as the
-// header states; the registers themselves are in shared memory.)
+// Scratch of every call: len operand-log entries (16 bytes each) per box and
+// one more.  (The call's limit counts nregs intervals of 8 bytes per box too,
+// as the header states, at least 256 bytes; the registers themselves are in
+// shared memory.)
 static __device__ __align__(256) unsigned char g_static_scratch[TSI_STATIC_SCRATCH_BYTES];
 
 namespace {
@@ -67,7 +68,7 @@ extern "C" TSI_API tsi_status tsi_tape_eval_boxes_static(const tsi_tape *tape, u
     return TSI_ERR_INVALID_ARGUMENT;
   }
   const uint64_t regs_bytes = ((uint64_t)n * v.tape.nregs * 8u + 255u) & ~255ull;
-  const uint64_t log_bytes = tsi::evalbox_log_bytes(n, v.tape.len);
+  const uint64_t log_bytes = (uint64_t)n * (v.tape.len ? v.tape.len : 1u) * 16u;
   if (regs_bytes + log_bytes > TSI_STATIC_SCRATCH_BYTES) {
     tsi_internal_set_error("tsi_tape_eval_boxes_static: n boxes x (registers + tape length) exceeds the "
                            "static scratch of TSI_STATIC_SCRATCH_BYTES; split the call");

@@ -58,17 +58,21 @@ struct NarrowRows {
   uint32_t rf;      // shared address of this lane's column of row 0
   uint32_t prog;    // shared address of the 32 decoded instructions
   uint32_t stride;  // bytes of a row
-  uint32_t col;     // this lane's column
   uint32_t sink;    // offset of the sink row
+  uint32_t log_step;  // log entries from one instruction to the next (0: this lane's all go to one place)
 };
+// Of an item with so many parents: cells, then (below 32) the shared column.
+__device__ __forceinline__ uint32_t narrow_cells(uint32_t parents) {
+  return parents == 1u ? 8u : (parents == 2u ? 16u : 32u);
+}
 __device__ __forceinline__ NarrowRows narrow_rows(const void *base, uint32_t rcap, uint32_t lane, uint32_t parents) {
   NarrowRows R;
-  const uint32_t cells = parents == 1u ? 8u : (parents == 2u ? 16u : 32u);
+  const uint32_t cells = narrow_cells(parents);
   const uint32_t b = (uint32_t)__cvta_generic_to_shared(base);
   R.stride = cells < 32u ? (cells + 1u) * 8u : 256u;
-  R.col = min(lane, cells);
-  R.rf = b + R.col * 8u;
+  R.rf = b + min(lane, cells) * 8u;
   R.sink = rcap * 256u;
+  R.log_step = R.stride / 8u;
   R.prog = b + rcap * 256u + 256u;
   return R;
 }
@@ -205,10 +209,11 @@ __device__ __forceinline__ NarrowKinds narrow_kinds(uint32_t c) {
 __device__ __forceinline__ uint32_t uniform_u32(uint32_t v) { return __reduce_max_sync(FULL_MASK, v); }
 
 // Forward pass over `len` instructions (compute.wgsl:3633-3772).  Pushes the
-// operands of everything that is not linear on the log `lg` (16 bytes a
-// column and entry; null: no log) and the min/max branch ballots to `dg`
-// when they are set.  `nlog` is the number of log entries.  Returns the
-// output register's value.
+// operands of everything that is not linear on the log `lg` (this lane's
+// column of it, an entry of 16 bytes every R.log_step; null: no log) and the
+// min/max branch ballots to `dg` when they are set.  `nlog` is the number of
+// log entries (0 in a lane whose log_step is 0).  Returns the output
+// register's value.
 template <bool D>
 __device__ __noinline__ Iv narrow_forward(const uint2 *__restrict__ code, uint32_t len_, uint32_t out_reg,
                                           NarrowRows R, uint32_t lane, Iv x, Iv y, Iv z, Iv t, float4 *lg, uint2 *dg,
@@ -220,9 +225,8 @@ __device__ __noinline__ Iv narrow_forward(const uint2 *__restrict__ code, uint32
   row_st(R, R.stride, y);
   row_st(R, 2u * R.stride, z);
   row_st(R, 3u * R.stride, t);
-  const uint32_t cols = R.stride / 8u;
-  float4 *lp = lg + R.col;
-  const float4 *lp0 = lp;
+  const uint32_t cols = R.log_step;
+  float4 *lp = lg;
   row_st(R, R.sink, Iv{D ? 0.0f : -0.0f, -0.0f});
   auto linear_step = [&](const uint4 &w) {
     const uint32_t c = w.x;
@@ -303,7 +307,7 @@ __device__ __noinline__ Iv narrow_forward(const uint2 *__restrict__ code, uint32
       }
     }
   }
-  nlog = log_on ? (uint32_t)((lp - lp0) / cols) : 0u;
+  nlog = log_on && cols ? (uint32_t)((lp - lg) / cols) : 0u;
   return row_ld(R, out_reg * R.stride);
 }
 
@@ -340,10 +344,9 @@ __device__ __noinline__ void narrow_reverse(const uint2 *__restrict__ code, uint
   row_st(R, R.sink, iv(0.0f));
   row_st(R, out_reg * R.stride, iv(1.0f));
   // the log from its end, three entries ahead
-  const uint32_t cols = R.stride / 8u;
-  const float4 *lcol = lg + R.col;
+  const uint32_t cols = R.log_step;
   int lp = (int)uniform_u32(nlog);
-  auto entry = [&](int i) { return i < 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : lcol[(size_t)i * cols]; };
+  auto entry = [&](int i) { return i < 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : lg[(size_t)i * cols]; };
   float4 E0 = entry(lp - 1), E1 = entry(lp - 2), E2 = entry(lp - 3);
   float nonfinite = 0.0f;  // becomes NaN with the first infinite or NaN bound
   const bool all = !D || __any_sync(FULL_MASK, strict_);

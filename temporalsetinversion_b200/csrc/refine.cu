@@ -500,7 +500,7 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       }
       const long long q0 = clock64();
       uint32_t nlog = 0;
-      float4 *opl = any_deriv ? lg : nullptr;
+      float4 *opl = any_deriv ? lg + min(lane, narrow_cells(it.n)) : nullptr;  // this lane's column of the log
       field = narrow_forward<D>(TR.code, TR.len, TR.out_reg, R, lane, cx, cy, cz, targ, opl, dg, nlog);
       const long long q1 = clock64();
       bool bad = false;
