@@ -68,7 +68,10 @@ struct tsi_batch_graph {
   cudaGraphExec_t exec = nullptr;
   bool launched = false;
   std::vector<uint8_t> global;  // per request: wide cells in the global scratch
-  std::shared_ptr<unsigned char> wscratch;  // that scratch, which a later plan of the context may replace
+  // that scratch, and the rows its readback fills: the context may replace
+  // either later, while the captured launches and copies name these
+  std::shared_ptr<unsigned char> wscratch;
+  std::shared_ptr<ReadbackRows> rows;
 };
 
 namespace tsi_host {
@@ -399,43 +402,40 @@ tsi_status enqueue_invert(tsi_ctx *c, tsi_scene *const *scenes, const float *tim
 }
 
 tsi_status ensure_readback_rows(tsi_ctx *c, uint32_t n) {
-  if (n <= c->rb_rows) return TSI_OK;
+  if (c->rows && n <= c->rows->n) return TSI_OK;
   if (capturing(c)) return set_err(TSI_ERR_BUSY, "readback rows grown during graph capture");
   CK(cudaStreamSynchronize(c->stream));
-  cudaFreeHost(c->h_err);
-  cudaFreeHost(c->h_stats);
-  cudaFreeHost(c->h_live);
-  c->h_err = nullptr;
-  c->h_stats = nullptr;
-  c->h_live = nullptr;
-  c->rb_rows = 0;
+  auto r = std::make_shared<ReadbackRows>();
   const uint32_t rows = std::max(n, 64u);
-  CK(cudaMallocHost((void **)&c->h_err, rows * sizeof(uint32_t)));
-  CK(cudaMallocHost((void **)&c->h_stats, (size_t)rows * ST_COUNT * sizeof(unsigned long long)));
-  CK(cudaMallocHost((void **)&c->h_live, rows * sizeof(uint32_t)));
-  memset(c->h_live, 0, rows * sizeof(uint32_t));
-  memset(c->h_err, 0, rows * sizeof(uint32_t));
-  memset(c->h_stats, 0, (size_t)rows * ST_COUNT * sizeof(unsigned long long));
-  c->rb_rows = rows;
+  CK(cudaMallocHost((void **)&r->err, rows * sizeof(uint32_t)));
+  CK(cudaMallocHost((void **)&r->stats, (size_t)rows * ST_COUNT * sizeof(unsigned long long)));
+  CK(cudaMallocHost((void **)&r->live, rows * sizeof(uint32_t)));
+  memset(r->err, 0, rows * sizeof(uint32_t));
+  memset(r->stats, 0, (size_t)rows * ST_COUNT * sizeof(unsigned long long));
+  memset(r->live, 0, rows * sizeof(uint32_t));
+  r->n = rows;
+  c->rows = std::move(r);
   return TSI_OK;
 }
 
 // Error words and stats rows of the launch's n scenes into readback rows
 // row0 .. row0 + n - 1, and the list sizes of its steps.
 tsi_status enqueue_readback(tsi_ctx *c, uint32_t n, uint32_t row0 = 0) {
-  if (row0 + n > c->rb_rows) return set_err(TSI_ERR_INVALID_ARGUMENT, "readback rows not reserved");
-  CK(cudaMemcpyAsync(c->h_err + row0, c->d_error, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(c->h_stats + (size_t)row0 * ST_COUNT, c->d_stats, (size_t)n * ST_COUNT * sizeof(unsigned long long),
+  ReadbackRows &r = *c->rows;
+  if (row0 + n > r.n) return set_err(TSI_ERR_INVALID_ARGUMENT, "readback rows not reserved");
+  CK(cudaMemcpyAsync(r.err + row0, c->d_error, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(r.stats + (size_t)row0 * ST_COUNT, c->d_stats, (size_t)n * ST_COUNT * sizeof(unsigned long long),
                      cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(c->h_live + row0, c->d_live, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaMemcpyAsync(r.live + row0, c->d_live, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemcpyAsync(c->h_rb->item_count, c->d_item_count, sizeof(c->h_rb->item_count), cudaMemcpyDeviceToHost,
                      c->stream));
   return TSI_OK;
 }
 
-void fill_stats(const tsi_ctx *c, uint32_t row, const tsi_scene *s, tsi_stats *st, uint64_t voxels_live) {
+void fill_stats(const tsi_ctx *c, const ReadbackRows &r, uint32_t row, const tsi_scene *s, tsi_stats *st,
+                uint64_t voxels_live) {
   if (!st) return;
-  fill_stats_row(c->h_stats + (size_t)row * ST_COUNT, c->h_err[row], s, st, voxels_live);
+  fill_stats_row(r.stats + (size_t)row * ST_COUNT, r.err[row], s, st, voxels_live);
   uint64_t hw = 0;
   uint32_t levels = 0;
   for (uint32_t l = 0; l < TSI_STEP_RING; ++l) {
@@ -478,13 +478,13 @@ void fill_stats_row(const unsigned long long *r, uint32_t err, const tsi_scene *
 
 // tsi_stats summed over readback rows 0 .. n-1 (a batch or graph replay as
 // a whole); the error word is the or of the rows'.
-void fill_stats_sum(const tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, tsi_stats *st) {
+void fill_stats_sum(const tsi_ctx *c, const ReadbackRows &r, tsi_scene *const *scenes, uint32_t n, tsi_stats *st) {
   if (!st) return;
   tsi_stats acc;
   memset(&acc, 0, sizeof(acc));
   for (uint32_t i = 0; i < n; ++i) {
     tsi_stats one;
-    fill_stats(c, i, scenes ? scenes[i] : nullptr, &one, 0);
+    fill_stats(c, r, i, scenes ? scenes[i] : nullptr, &one, 0);
     uint64_t *a = &acc.parents_expanded;
     const uint64_t *b = &one.parents_expanded;
     for (size_t k = 0; k < (offsetof(tsi_stats, levels) - offsetof(tsi_stats, parents_expanded)) / sizeof(uint64_t); ++k)
@@ -496,9 +496,9 @@ void fill_stats_sum(const tsi_ctx *c, tsi_scene *const *scenes, uint32_t n, tsi_
   *st = acc;
 }
 
-uint32_t readback_error_or(const tsi_ctx *c, uint32_t n) {
+uint32_t readback_error_or(const ReadbackRows &r, uint32_t n) {
   uint32_t e = 0;
-  for (uint32_t i = 0; i < n; ++i) e |= c->h_err[i];
+  for (uint32_t i = 0; i < n; ++i) e |= r.err[i];
   return e;
 }
 
@@ -1039,9 +1039,7 @@ TSI_API void tsi_destroy(tsi_ctx *c) {
   cudaFree(c->d_visits);
   cudaFree(c->d_scratch);
   cudaFreeHost(c->h_rb);
-  cudaFreeHost(c->h_err);
-  cudaFreeHost(c->h_live);
-  cudaFreeHost(c->h_stats);
+  c->rows.reset();
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->launch_up) cudaEventDestroy(c->launch_up);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -1394,10 +1392,10 @@ TSI_API tsi_status tsi_scene_invert(tsi_scene *s, float time, float t0_or_nan, t
   float ms = 0.0f;
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   if (stats) {
-    fill_stats(c, 0, s, stats, (uint64_t)c->h_live[0] * 8u);
+    fill_stats(c, *c->rows, 0, s, stats, (uint64_t)c->rows->live[0] * 8u);
     stats->device_ms = ms;
   }
-  return status_from_error_bits(c->h_err[0]);
+  return status_from_error_bits(c->rows->err[0]);
 }
 
 TSI_API tsi_status tsi_scene_invert_async(tsi_scene *s, float time, float t0_or_nan) {
@@ -1423,7 +1421,7 @@ TSI_API tsi_status tsi_scene_invert_wait(tsi_scene *s, tsi_stats *stats) {
     SceneCounters ctr;
     const tsi_status st = read_counters(s, ctr);
     if (st != TSI_OK) return st;
-    fill_stats(c, 0, s, stats, (uint64_t)ctr.live_bricks * 8u);
+    fill_stats(c, *c->rows, 0, s, stats, (uint64_t)ctr.live_bricks * 8u);
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     stats->device_ms = ms;
@@ -2045,9 +2043,9 @@ TSI_API tsi_status tsi_batch_run(tsi_ctx *c, tsi_request *reqs, uint32_t n) {
   CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   uint32_t err = 0;
   for (uint32_t i = 0; i < n; ++i) {
-    err |= c->h_err[i];
+    err |= c->rows->err[i];
     if (reqs[i].stats) {
-      fill_stats(c, i, reqs[i].scene, reqs[i].stats, (uint64_t)c->h_live[i] * 8u);
+      fill_stats(c, *c->rows, i, reqs[i].scene, reqs[i].stats, (uint64_t)c->rows->live[i] * 8u);
       reqs[i].stats->device_ms = ms;
     }
   }
@@ -2166,6 +2164,7 @@ TSI_API tsi_status tsi_batch_graph_create(tsi_ctx *c, tsi_request *reqs, uint32_
   if (cudaEventRecordWithFlags(c->ev0, c->stream, cudaEventRecordExternal) != cudaSuccess)
     st = set_err(TSI_ERR_CUDA, "event record in capture");
   if (st == TSI_OK) st = batch_enqueue(c, g->reqs.data(), n);
+  g->rows = c->rows;
   if (st == TSI_OK && cudaEventRecordWithFlags(c->ev1, c->stream, cudaEventRecordExternal) != cudaSuccess)
     st = set_err(TSI_ERR_CUDA, "event record in capture");
   cudaGraph_t graph = nullptr;
@@ -2225,12 +2224,12 @@ TSI_API tsi_status tsi_batch_graph_wait(tsi_batch_graph *g, tsi_stats *stats) {
   if (stats) {
     std::vector<tsi_scene *> sc(n);
     for (uint32_t i = 0; i < n; ++i) sc[i] = g->reqs[i].scene;
-    fill_stats_sum(c, sc.data(), n, stats);
+    fill_stats_sum(c, *g->rows, sc.data(), n, stats);
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     stats->device_ms = ms;
   }
-  return status_from_error_bits(readback_error_or(c, n));
+  return status_from_error_bits(readback_error_or(*g->rows, n));
 }
 
 TSI_API void tsi_batch_graph_destroy(tsi_batch_graph *g) {

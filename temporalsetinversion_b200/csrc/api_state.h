@@ -38,6 +38,23 @@ struct TsiReadback {
   unsigned long long visits;
 };
 
+// Pinned host rows that the error words, the counters and the bricks in use of
+// a launch sequence's scenes are copied to.
+struct ReadbackRows {
+  uint32_t n = 0;
+  uint32_t *err = nullptr;
+  unsigned long long *stats = nullptr;  // [n][ST_COUNT]
+  uint32_t *live = nullptr;
+  ReadbackRows() = default;
+  ReadbackRows(const ReadbackRows &) = delete;
+  ReadbackRows &operator=(const ReadbackRows &) = delete;
+  ~ReadbackRows() {
+    cudaFreeHost(err);
+    cudaFreeHost(stats);
+    cudaFreeHost(live);
+  }
+};
+
 struct tsi_tape {
   tsi_ctx *ctx = nullptr;
   void *d_block = nullptr;  // the one allocation that holds the tape's arrays on the device
@@ -135,14 +152,13 @@ struct tsi_ctx {
   cudaEvent_t launch_up = nullptr;
   bool launch_up_pending = false;
   unsigned long long *d_stats = nullptr;        // [max_scenes][ST_COUNT]
-  uint32_t *d_live = nullptr, *h_live = nullptr;  // [max_scenes], [rb_rows]
+  uint32_t *d_live = nullptr;                     // [max_scenes]
   unsigned long long *d_level_stats = nullptr;  // [TSI_STEP_RING][ST_COUNT]
   unsigned long long *d_visits = nullptr;
   TsiReadback *h_rb = nullptr;
-  // per-scene rows read back after a launch sequence (pinned, rb_rows rows)
-  uint32_t *h_err = nullptr;
-  unsigned long long *h_stats = nullptr;
-  uint32_t rb_rows = 0;
+  // per-scene rows read back after a launch sequence (captured graphs keep
+  // the ones that their copies name); never null after tsi_create
+  std::shared_ptr<ReadbackRows> rows;
   // per-level profile of the last inversion (events when profiling is on)
   bool profile_levels = false;
   std::vector<cudaEvent_t> level_events;
@@ -194,7 +210,8 @@ tsi_status copy_image_out(tsi_scene *s, tsi_image *out, cudaStream_t st);
 // Grows the pinned per-scene readback rows to at least n.
 tsi_status ensure_readback_rows(tsi_ctx *c, uint32_t n);
 // tsi_stats of one scene from its readback row (and the launch's list sizes).
-void fill_stats(const tsi_ctx *c, uint32_t row, const tsi_scene *s, tsi_stats *st, uint64_t voxels_live);
+void fill_stats(const tsi_ctx *c, const ReadbackRows &r, uint32_t row, const tsi_scene *s, tsi_stats *st,
+                uint64_t voxels_live);
 // tsi_stats of one scene from a stats row (ST_COUNT counters) and error word.
 void fill_stats_row(const unsigned long long *row, uint32_t err, const tsi_scene *s, tsi_stats *st,
                     uint64_t voxels_live);

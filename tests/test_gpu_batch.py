@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import assert_cells_equal
-from temporalsetinversion_b200 import Scene, Tape, api, scenes
+from temporalsetinversion_b200 import Scene, Tape, _native as N, api, scenes
 
 
 def _make(device, specs):
@@ -96,6 +96,34 @@ def test_graph_survives_a_larger_scratch():
         g.close()
     finally:
         dev.close()
+
+
+@pytest.mark.gpu
+def test_graph_reads_its_own_rows_after_a_wider_batch():
+    """A graph's counters and error status after a batch of more scenes than
+    the context had readback rows for, which makes the context take others."""
+    from temporalsetinversion_b200 import Device
+
+    with Device() as dev:
+        p = api.default_params(localsubdiv=4, delta=0.02)
+        tape = Tape.from_llvm_ir(dev, scenes.spheres16(0))
+        a, b = Scene(dev, tape, p, 1 << 14), Scene(dev, tape, p, 1 << 14)
+        full = Scene(dev, tape, p, 64)  # a pool of a few bricks: the first frame exhausts it
+        good = api.BatchGraph(dev, [(a, 0.0, math.nan, None)])
+        bad = api.BatchGraph(dev, [(full, 0.0, math.nan, None)])
+        flat = api.default_params(localsubdiv=1)
+        api.run_batch(dev, [(Scene(dev, tape, flat, 1 << 10), 0.0, math.nan, None) for _ in range(130)])
+        for t in (0.0, 0.05):
+            good.launch([t])
+            st, want = good.wait(), b.invert(t)
+            assert st.cells_evaluated == want.cells_evaluated > 0 and st.error_flags == 0
+            assert_cells_equal(a.cells(), b.cells())
+        bad.launch([0.0])
+        with pytest.raises(N.TsiError) as e:
+            bad.wait()
+        assert e.value.status == 4  # TSI_ERR_OOM
+        good.close()
+        bad.close()
 
 
 @pytest.mark.gpu
