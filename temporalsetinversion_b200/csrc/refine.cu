@@ -60,6 +60,13 @@ extern __shared__ __align__(16) unsigned char tsi_dyn_smem[];
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// First word of the copy that a decided min/max (first word w) becomes: of
+// operand A, or else B, in register r.
+__device__ __forceinline__ uint32_t copy_word(uint32_t w, bool of_a, uint32_t d, uint32_t r) {
+  const uint32_t flag = of_a ? TSI_W0_FA(w) : TSI_W0_FB(w), raw = w & (of_a ? TSI_W0_RAW_A : TSI_W0_RAW_B);
+  return TSI_W0(H_COPY, flag, 0u, d, r) | (w & TSI_W0_ODD) | (raw ? TSI_W0_RAW_A : 0u);
+}
+
 // Backward liveness scan of one sibling group (g, enqueued siblings E) by the
 // whole warp: decided min/max become copies/constants, dead instructions
 // vanish.  The kept instructions are written in reverse order to `tmp`;
@@ -96,13 +103,13 @@ __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, 
       const uint2 dd = dg[m + __popc(mmb & ((1u << lane) - 1u))];
       const uint32_t ga = (dd.x >> (g * 8u)) & 0xffu, gb = (dd.y >> (g * 8u)) & 0xffu;
       if ((ga & E) == E) {
-        out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, d, a) | (w.x & TSI_W0_ODD) | deps_b, 0u);
+        out = make_uint2(copy_word(w.x, true, d, a) | deps_b, 0u);
         hk = H_COPY;
         use_b = false;
       } else if ((gb & E) == E) {
         use_a = false;
         if (TSI_H_IS_II(h)) {
-          out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, d, b) | (w.x & TSI_W0_ODD) | deps_a, 0u);
+          out = make_uint2(copy_word(w.x, false, d, b) | deps_a, 0u);
           hk = H_COPY;
         } else {
           out = make_uint2(TSI_W0(H_CONST, 0u, 0u, d, 0u) | deps_a, w.y);
@@ -127,8 +134,8 @@ __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, 
       keep |= on ? 1u << j : 0u;
     }
     // a copy of a register to itself does nothing, forward or reverse, but
-    // carry a directed reverse pass's test
-    if (!D) keep &= ~__ballot_sync(FULL_MASK, hk == H_COPY && TSI_W0_A(out.x) == d);
+    // carry a directed reverse pass's test and clamp an argument
+    if (!D) keep &= ~__ballot_sync(FULL_MASK, hk == H_COPY && TSI_W0_A(out.x) == d && !(out.x & TSI_W0_RAW_A));
     if ((keep >> lane) & 1u) {
       tmp[cnt + __popc(keep & ~((2u << lane) - 1u))] = out;
       kept_mm += TSI_H_IS_MINMAX(hk) ? 1u : 0u;
@@ -1109,11 +1116,11 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
               const uint32_t deps_a = TSI_W0_WITH_DEPS(TSI_W0_DEPS(w.x));
               const uint32_t deps_b = TSI_H_IS_II(h) ? TSI_W0_WITH_DEPS(TSI_W1_DEPS(w.y)) : 0u;
               if (d & 1u) {
-                out = make_uint2(TSI_W0(H_COPY, TSI_W0_FA(w.x), 0u, dd, TSI_W0_A(w.x)) | (w.x & TSI_W0_ODD) | deps_b, 0u);
+                out = make_uint2(copy_word(w.x, true, dd, TSI_W0_A(w.x)) | deps_b, 0u);
                 hk = H_COPY;
               } else if (d & 2u) {
                 if (TSI_H_IS_II(h)) {
-                  out = make_uint2(TSI_W0(H_COPY, TSI_W0_FB(w.x), 0u, dd, w.y & 255u) | (w.x & TSI_W0_ODD) | deps_a, 0u);
+                  out = make_uint2(copy_word(w.x, false, dd, w.y & 255u) | deps_a, 0u);
                   hk = H_COPY;
                 } else {
                   out = make_uint2(TSI_W0(H_CONST, 0u, 0u, dd, 0u) | deps_a, w.y);

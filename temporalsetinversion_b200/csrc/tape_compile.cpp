@@ -175,7 +175,8 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
     used[d] = (last_use[j] >= 0) ? 1 : 0;  // a never-read value frees at once
     if (d > maxreg) maxreg = d;
     const bool odd = (fa && users[a_slot] > 1u) || (fb && users[b_slot] > 1u);
-    out.code.push_back(TSI_W0(h, fa, fb, d, ra) | (odd ? TSI_W0_ODD : 0u));
+    out.code.push_back(TSI_W0(h, fa, fb, d, ra) | (odd ? TSI_W0_ODD : 0u) |
+                       (has_a && a_slot < 4u ? TSI_W0_RAW_A : 0u) | (has_b && b_slot < 4u ? TSI_W0_RAW_B : 0u));
     out.code.push_back(w1);
     if (TSI_H_IS_MINMAX(h)) out.n_minmax++;
     const uint32_t da = has_a ? deps[a_slot] : 0u, db = has_b ? deps[b_slot] : 0u;
@@ -455,7 +456,8 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
   // value v is the narrow tape's instruction v - 4
   auto same = [&](uint32_t v) -> uint32_t {
     const uint32_t w0 = pt.code[2 * size_t(v - 4u)], w1 = pt.code[2 * size_t(v - 4u) + 1];
-    const bool a = TSI_W0_DST(w0) == TSI_W0_A(w0), b = TSI_H_IS_II(TSI_W0_H(w0)) && TSI_W0_DST(w0) == (w1 & 255u);
+    const bool a = TSI_W0_DST(w0) == TSI_W0_A(w0) && !(w0 & TSI_W0_RAW_A);
+    const bool b = TSI_H_IS_II(TSI_W0_H(w0)) && TSI_W0_DST(w0) == (w1 & 255u) && !(w0 & TSI_W0_RAW_B);
     return (a ? WL_SAME_A : 0u) | (b ? WL_SAME_B : 0u);
   };
   std::vector<uint32_t> targets;

@@ -13,7 +13,10 @@
 //       bits  9..12  uploaded min/max: the arguments that operand A depends on;
 //                    copy or constant of a decided min/max: those that the
 //                    operand which lost depends on (x, y, z, t from bit 9)
-//       bits 13..15  reserved
+//       bits 13, 14  operand A, B is one of the four arguments: its bounds did
+//                    not pass through fix, so a copy of it (A) does something
+//                    even to the register it comes from
+//       bit  15      reserved
 //       bits 16..23  destination register
 //       bits 24..31  register A (larg, or rarg for the literal-left kinds)
 //   w1  register B in bits 0..7 (two-register handlers; of an uploaded min/max
@@ -44,6 +47,8 @@ enum tsi_handler {
 #define TSI_W0(h, fa, fb, dst, a) \
   ((uint32_t)(h) | ((uint32_t)(fa) << 6) | ((uint32_t)(fb) << 7) | ((uint32_t)(dst) << 16) | ((uint32_t)(a) << 24))
 #define TSI_W0_ODD (1u << 8)
+#define TSI_W0_RAW_A (1u << 13)
+#define TSI_W0_RAW_B (1u << 14)
 #define TSI_W0_DEPS(w) (((w) >> 9) & 15u)
 #define TSI_W1_DEPS(w) (((w) >> 8) & 15u)
 #define TSI_W0_WITH_DEPS(deps) ((uint32_t)(deps) << 9)

@@ -58,8 +58,9 @@ constexpr uint32_t kWideWarps = 8;
 struct WideTape;
 struct PackedTape;
 
-// Of a min/max in the liveness slots: its register is the operand's, so the
-// copy that it becomes when that operand is always chosen does nothing.
+// Of a min/max in the liveness slots: its register is the operand's, which is
+// no argument, so the copy that it becomes when that operand is always chosen
+// does nothing.
 constexpr uint32_t WL_SAME_A = 1u << 30, WL_SAME_B = 1u << 31;
 
 struct WideTapeDev {

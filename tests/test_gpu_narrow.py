@@ -167,3 +167,43 @@ def test_directed_infinite_sensitivities_match_full_tape(device, scene):
         else:
             for a, c in zip(cells, ref):
                 assert_cells_equal(a, c)
+
+
+def argument_tape(arg: str, kind: str) -> np.ndarray:
+    """Moving spheres, less a little of an argument beyond the clamp of `fix`
+    which a min/max that is always decided passes on: its last use, so the
+    copy that it becomes when pruned goes to the argument's own register."""
+    b = scenes.IRBuilder()
+    acc = None
+    for i in range(30):
+        c = [0.9 * np.cos(i), 0.9 * np.sin(2.0 * i), 0.9 * np.sin(i)]
+        d = [b.sub(v, float(ck)) for v, ck in zip((b.Y, b.Z), c)]
+        s = b.sub(b.sqrt(b.add(b.mul(d[0], d[0]), b.mul(d[1], d[1]))), 0.3 + 0.01 * i)
+        s = b.add(s, 0.0)
+        acc = s if acc is None else b.min(acc, s)
+    v = b.T if arg == "t" else b.X
+    m = b.min(v, 2.0e6) if kind == "literal" else b.max(b.min(b.mul(b.Y, 0.1), 3.0), v)
+    acc = b.sub(acc, b.mul(m, 2.0e-7))
+    return api.IR.new(b.text(acc)).gpu_instructions
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("threshold", [0xFFFFFFFF, 100])
+@pytest.mark.parametrize("kind", ["literal", "register"])
+@pytest.mark.parametrize("arg", ["t", "x"])
+def test_copies_of_arguments_beyond_the_clamp_are_kept(device, arg, kind, threshold):
+    """`fix` clamps what a min/max passes on; the four arguments are as given.
+    A pruned tape has to clamp the argument where the full tape does."""
+    tape = argument_tape(arg, kind)
+    assert len(tape) >= 260  # a bundled form
+    p = dict(localsubdiv=5, delta=0.02)
+    if arg == "x":
+        p.update(root_lo=(1.4e6, -2.0, -2.0), root_hi=(1.4e6 + 4.0, 2.0, 2.0))
+    p = api.default_params(**p)
+    t = Tape.upload(device, tape)
+    t.wide_threshold = threshold
+    gs, os_ = Scene(device, t, p), oracle.Scene(tape, p)
+    for time in ([1.4e6, 1.4e6 + 1.0] if arg == "t" else TIMES[:2]):
+        gs.invert(time)
+        os_.invert(time)
+        assert_cells_equal(gs.cells(), os_.cells())
