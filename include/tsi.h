@@ -295,7 +295,10 @@ TSI_API tsi_status tsi_scene_trace_wait(tsi_scene *scene);
 /* No counterpart in the reference (its workgroup shape is fixed at
  * compute.wgsl:3513).  Child cells whose pruned tape is at least the tape's
  * wide threshold are evaluated one cell per 256-thread block from the
- * tape's bundled SSA form; shorter ones one warp per 8-cell group.  Results
+ * tape's bundled SSA form; shorter ones one warp per 8-cell group.  To
+ * nearest, the threshold is multiplied on levels that have more such cells
+ * than the GPU has room for blocks, by how many times more, as long as the
+ * warps' own scratch holds their operand logs.  Results
  * are identical for every threshold; only the speed changes.  Tapes shorter
  * than 256 instructions, or whose wide working set would exceed 8 MiB per
  * cell, have no bundled form: they report UINT32_MAX (narrow only) and

@@ -190,6 +190,7 @@ WideDev wide_dev(const tsi_tape *t) {
   W.deep_level = t->wdeep_level;
   W.deep_min_len = has_wide ? t->wdeep_min_len : 0xffffffffu;
   W.ncontrib = t->wcontrib;
+  W.log_len = t->log_len;
   for (int q = 0; q < 4; ++q) {
     W.arg_gbase[q] = t->warg_gbase[q];
     W.arg_gcount[q] = t->warg_gcount[q];
@@ -229,7 +230,9 @@ void fill_launch(tsi_scene *s, uint32_t slot, float time, float t0_or_nan, bool 
   L.wide = wide_dev(s->tape);
   L.wide.prune_level = s->tape->wprune_level != 0xffffffffu ? s->tape->wprune_level : tree_levels(p) / 2u;
   L.wide.global = wide_global ? 1u : 0u;
-  L.wide.directed = p.rounding_mode == TSI_ROUND_DIRECTED ? 1u : 0u;
+  // (a warp's slice holds the log of the full tape for one cell at least)
+  L.wide.by_length =
+      p.rounding_mode == TSI_ROUND_DIRECTED || 2ull * s->tape->log_len > 32ull * s->ctx->slice_len ? 1u : 0u;
   R.code = s->tape->d_code;
   R.len = s->tape->len;
   R.nregs = s->tape->nregs;
@@ -1071,6 +1074,7 @@ static tsi_status upload_ir(tsi_ctx *c, const std::vector<IrInstr> &ins, tsi_tap
   t->fwd_cost = pt.fwd_cost;
   t->rev_cost = pt.rev_cost;
   t->strict = pt.strict;
+  t->log_len = pt.log_len;
   c->tapes.insert(t);
   // The tape's arrays on the device are parts of one allocation, filled by
   // one copy (each allocation and each copy cost more than the bytes: the

@@ -62,7 +62,8 @@ struct tsi_tape {
   uint32_t len = 0;  // instructions after the 4 ARG slots
   uint32_t count = 0, nregs = 0, out_reg = 0, n_minmax = 0;
   uint64_t fwd_cost = 0, rev_cost = 0;
-  bool strict = false;  // PackedTape::strict
+  bool strict = false;   // PackedTape::strict
+  uint32_t log_len = 0;  // PackedTape::log_len
   // bundled form for the wide path (absent when the tape is short)
   uint4 *d_wfwd = nullptr, *d_wrev = nullptr, *d_wlive = nullptr, *d_wrev16 = nullptr;
   uint4 *d_wfwd_slots = nullptr;

@@ -89,7 +89,8 @@ struct WideDev {
   uint32_t min_len;           // tapes at least this long go to the wide path
   uint32_t deep_level;        // children at this level or deeper use deep_min_len (TSI_NONE: never)
   uint32_t deep_min_len;
-  uint32_t directed;          // outward rounding (route_len)
+  uint32_t by_length;         // 1: the thresholds alone route an item (goes_wide)
+  uint32_t log_len;           // instructions of the full tape that are not linear to nearest (narrow_interp.cuh)
   uint32_t ncontrib;          // reverse contribution records per cell
   uint32_t prune_level;       // wide items at this octree level or deeper prune their group's tape
   uint32_t global;            // 1: the cell working set lives in the block's slice of

@@ -173,25 +173,6 @@ __device__ uint32_t alloc_brick(const SceneLaunch &S, uint32_t *error) {
 __device__ __forceinline__ uint32_t wide_min_len(const WideDev &W, uint32_t level) {
   return level >= W.deep_level ? W.deep_min_len : W.min_len;
 }
-// The tape length from which children of this step's groups take the wide
-// path: the threshold (where a block per cell and a warp per item take
-// equally long) times the waves of blocks that this step's long items need
-// for their eight cells each; the next step seldom has fewer.  A step of
-// long items finishes a wide item of 8 cells in 8/296 of a cell's time on a
-// B200's 296 blocks, but 2368 narrow items at once: by length alone, levels
-// of thousands of long items ran one block per cell.  Rotating swept scene
-// (64 primitives, localsubdiv 9) 8.0 to 2.7 ms an inversion, 1024 primitives
-// (localsubdiv 9) 3.7 to 3.3 ms, 256 primitives unchanged; half and twice
-// the multiplier measured 3.1 and 2.7 ms, 3.6 and 3.2 ms.  Directed, a
-// one-warp item costs two to four times as much an instruction (outward
-// rounding has no packed form, and its sines no short one) and the length
-// decides alone: rotating swept scenes of 44 and 64 primitives, localsubdiv 8,
-// three inversions 10.6 and 19.8 ms so, 15.3 and 23.0 with the waves.
-__device__ __forceinline__ uint32_t route_len(const LaunchParams &P, const WideDev &W, uint32_t step, uint32_t level) {
-  const uint32_t waves = W.directed ? 1u : max(1u, 8u * P.long_count[step & TSI_STEP_MASK] / gridDim.x);
-  return (uint32_t)min((unsigned long long)wide_min_len(W, level) * waves, 0xffffffffull);
-}
-
 __device__ __forceinline__ StepIdx step_idx(uint32_t step) {
   StepIdx si;
   si.cur = step & TSI_STEP_MASK;
@@ -199,6 +180,52 @@ __device__ __forceinline__ StepIdx step_idx(uint32_t step) {
   si.buf = step & 1u;
   si.nbuf = (step + 1u) & 1u;
   return si;
+}
+
+// Log entries of a cell on a tape of this length, at most.
+__device__ __forceinline__ uint32_t log_bound(const WideDev &W, uint32_t len) { return min(len, W.log_len); }
+// Whether the log of an item of n parents fits its warp's slice.
+__device__ __forceinline__ bool slice_holds(const LaunchParams &P, uint32_t n, uint32_t entries) {
+  return (n == 1u ? 9u : n == 2u ? 17u : 32u) * entries <= 32u * P.slice_len;
+}
+// Whether an item that the length alone sends wide may be a narrow one.
+__device__ __forceinline__ bool may_go_narrow(const LaunchParams &P, const WideDev &W, uint32_t level, uint32_t len) {
+  return !W.by_length && len >= wide_min_len(W, level) && slice_holds(P, 1u, log_bound(W, len));
+}
+
+// Whether children of this step's groups with a tape of this length take the
+// wide path: from the threshold on (where a block per cell and a warp per item
+// take equally long), but for levels with more long items than blocks.  There
+// the threshold is multiplied by the waves of blocks that this step's long
+// items need for their eight cells each; the next step seldom has fewer.  A
+// step of long items finishes a wide item of 8 cells in 8/296 of a cell's time
+// on a B200's 296 blocks, but 2368 narrow items at once: by length alone,
+// levels of thousands of long items ran one block per cell.  Rotating swept
+// scene (64 primitives, localsubdiv 9) 8.0 to 2.7 ms an inversion, 1024
+// primitives (localsubdiv 9) 3.7 to 3.3 ms, 256 primitives unchanged; half and
+// twice the multiplier measured 3.1 and 2.7 ms, 3.6 and 3.2 ms.
+//
+// An item that the length alone would send wide costs neither the log arena
+// nor the narrow list anything that others may need:
+//  - its log fits its warp's slice (the arena, 16 bytes per instruction and
+//    column, is what items below the threshold share), with fewer parents if
+//    need be, and where it has to run on a longer tape of its scene it takes
+//    the cells in turns (own_slice_passes);
+//  - half of the narrow list stays free of such items, and what finds it full
+//    goes wide after all (push_children).
+//
+// by_length: a tape whose log fits no slice, and outward rounding, where a
+// one-warp item costs two to four times as much an instruction (no packed
+// form, and its sines no short one): rotating swept scenes of 44 and 64
+// primitives, localsubdiv 8, three inversions 10.6 and 19.8 ms so, 15.3 and
+// 23.0 with the waves.
+__device__ __forceinline__ bool goes_wide(const LaunchParams &P, const WideDev &W, uint32_t step, uint32_t level,
+                                          uint32_t len) {
+  const uint32_t from = wide_min_len(W, level);
+  if (!may_go_narrow(P, W, level, len)) return len >= from;
+  const uint32_t waves = max(1u, 8u * P.long_count[step & TSI_STEP_MASK] / gridDim.x);
+  const uint32_t next = step_idx(step).next;
+  return len >= (unsigned long long)from * waves || *(const volatile uint32_t *)&P.item_count[next] > P.item_cap / 2u;
 }
 
 // Reserves n words of the code arena (a ring of code_cap words, a power of
@@ -229,59 +256,66 @@ __device__ __forceinline__ void find_valid(const LaunchParams &P, uint32_t &rec,
   }
 }
 
+// Wide items for the children `rest` (cells[0..7] of one parent), one per
+// child, its own children's brick allocated here; returns those that the wide
+// list has no room for.  One thread.
+__device__ __forceinline__ uint32_t push_wide(const LaunchParams &P, const SceneLaunch &S, uint32_t scene, uint32_t rec,
+                                           uint32_t step, uint32_t plevel, uint32_t rest, const uint32_t *cells,
+                                           unsigned long long *ws) {
+  const StepIdx si = step_idx(step);
+  const uint32_t n = __popc(rest);
+  const uint32_t pos = atomicAdd(&P.witem_count[si.next], n);
+  uint32_t j = 0;
+  while (rest && pos + j < P.witem_cap) {
+    const uint32_t bit = __ffs(rest) - 1u;
+    rest &= rest - 1u;
+    const uint32_t c = cells[bit];
+    uint32_t b = S.pool.child[c], fresh = 0;
+    if (b == TSI_NONE) {
+      b = alloc_brick(S, P.error + scene);
+      if (b != TSI_NONE) {
+        S.pool.child[c] = b;
+        fresh = 1;
+        atomicAdd(&ws[ST_BRICK_ALLOC], 1ull);
+      }
+    }
+    WorkItem wi;
+    wi.scene = scene;
+    wi.rec = rec;
+    wi.n = 1;
+    wi.level = plevel + 1;
+    wi.parent[0] = c;
+    wi.parent[1] = b;
+    wi.parent[2] = fresh;
+    wi.parent[3] = 0;
+    P.witems[si.nbuf][pos + j++] = wi;
+  }
+  return rest;
+}
+
 // Next-level work for the enqueued children (mask E) of one parent, whose
-// cells are cells[0..7]; one thread.  `wide`: one wide item per child, its
-// own children's brick allocated here; children beyond the wide list's
-// capacity, or all of them when not `wide`, go to the narrow list in items
-// of up to four.  Every reserved list slot below the capacity is written
-// (readers take min(count, capacity) entries); narrow-list overflow is
-// dropped and reported.
+// cells are cells[0..7]; one thread.  `wide`: wide items; children beyond the
+// wide list's capacity, or all of them when not `wide`, go to the narrow list
+// in items of up to four.  Every reserved list slot below the capacity is
+// written (readers take min(count, capacity) entries).  What the narrow list
+// has no room for goes wide if it may, else it is dropped and reported.
+// `either`: the log entries of a cell that may go either way, else 0.
 __device__ void push_children(const LaunchParams &P, const SceneLaunch &S, uint32_t scene, uint32_t rec,
-                              uint32_t step, uint32_t plevel, uint32_t E, const uint32_t *cells, bool wide,
+                              uint32_t step, uint32_t plevel, uint32_t E, const uint32_t *cells, bool wide, uint32_t either,
                               unsigned long long *ws) {
   const StepIdx si = step_idx(step);
   // a scene's items end at its last level: the launch steps of its frame
   // stop there, and in the continuous form later steps belong to others
   if (plevel + 1u >= S.levels) return;
-  uint32_t rest = E;
-  uint32_t *err = P.error + scene;
-  if (wide) {
-    const uint32_t n = __popc(E);
-    const uint32_t pos = atomicAdd(&P.witem_count[si.next], n);
-    uint32_t j = 0;
-    while (rest && pos + j < P.witem_cap) {
-      const uint32_t bit = __ffs(rest) - 1u;
-      rest &= rest - 1u;
-      const uint32_t c = cells[bit];
-      uint32_t b = S.pool.child[c], fresh = 0;
-      if (b == TSI_NONE) {
-        b = alloc_brick(S, err);
-        if (b != TSI_NONE) {
-          S.pool.child[c] = b;
-          fresh = 1;
-          atomicAdd(&ws[ST_BRICK_ALLOC], 1ull);
-        }
-      }
-      WorkItem wi;
-      wi.scene = scene;
-      wi.rec = rec;
-      wi.n = 1;
-      wi.level = plevel + 1;
-      wi.parent[0] = c;
-      wi.parent[1] = b;
-      wi.parent[2] = fresh;
-      wi.parent[3] = 0;
-      P.witems[si.nbuf][pos + j++] = wi;
-    }
-  }
+  uint32_t rest = wide ? push_wide(P, S, scene, rec, step, plevel, E, cells, ws) : E;
   if (rest == 0) return;
   // a narrow item takes up to 4 parents (32 cells, one per lane) at the leaf
   // level, where many short evaluations make throughput count, and fewer
   // above it, where more items in flight hide the interpreter's latency
-  const uint32_t per = (plevel + 2u >= S.levels) ? 4u : max(1u, min(4u, S.narrow_parents));
+  uint32_t per = (plevel + 2u >= S.levels) ? 4u : max(1u, min(4u, S.narrow_parents));
+  while (either && per > 1u && !slice_holds(P, per, either)) per >>= 1;
   const uint32_t nitems = (__popc(rest) + per - 1u) / per;
   const uint32_t pos = atomicAdd(&P.item_count[si.next], nitems);
-  if (pos + nitems > P.item_cap) atomicOr(err, EB_QUEUE_FULL);
   WorkItem *dst = P.items[si.nbuf];
   for (uint32_t j = 0; j < nitems && pos + j < P.item_cap; ++j) {
     WorkItem wi;
@@ -298,6 +332,8 @@ __device__ void push_children(const LaunchParams &P, const SceneLaunch &S, uint3
     for (uint32_t q = c; q < 4u; ++q) wi.parent[q] = wi.parent[0];
     dst[pos + j] = wi;
   }
+  if (rest && either) rest = push_wide(P, S, scene, rec, step, plevel, rest, cells, ws);
+  if (rest) atomicOr(P.error + scene, EB_QUEUE_FULL);
 }
 
 // push_children for the eight children of one wide item (cells base..base+7),
@@ -308,8 +344,8 @@ __device__ void push_children(const LaunchParams &P, const SceneLaunch &S, uint3
 // are not read: they are known to be empty.
 __device__ __forceinline__ void push_children_warp(const LaunchParams &P, const SceneLaunch &S, uint32_t scene,
                                                    uint32_t rec, uint32_t step, uint32_t plevel, uint32_t E,
-                                                   uint32_t base, bool fresh, bool wide, unsigned long long *ws,
-                                                   uint32_t lane) {
+                                                   uint32_t base, bool fresh, bool wide, uint32_t either,
+                                                   unsigned long long *ws, uint32_t lane) {
   const StepIdx si = step_idx(step);
   if (plevel + 1u >= S.levels) return;  // the scene's last level (push_children)
   uint32_t rest = E;
@@ -351,7 +387,7 @@ __device__ __forceinline__ void push_children_warp(const LaunchParams &P, const 
   if (lane == 0 && rest) {
     uint32_t cells[8];
     for (int q = 0; q < 8; ++q) cells[q] = base + q;
-    push_children(P, S, scene, rec, step, plevel, rest, cells, false, ws);
+    push_children(P, S, scene, rec, step, plevel, rest, cells, false, wide ? 0u : either, ws);
   }
 }
 
@@ -386,6 +422,48 @@ __device__ __forceinline__ bool item_scratch(const LaunchParams &P, uint32_t ste
   lg = P.log_overflow + off;
   dg = reinterpret_cast<uint2 *>(P.log_overflow + off + (unsigned long long)len * 32ull);
   return true;
+}
+
+// The sensitivities of an item's cells (to nearest) on a tape whose log is too
+// long for 32 columns of the warp's slice: some columns at a time, at least
+// one cell and the lanes' shared column, one forward and one reverse pass
+// each.  `log_len`: a bound of the tape's log entries.
+struct OwnSlice {
+  const uint2 *code;
+  uint32_t len, nregs, out_reg, log_len, slice_len, cells;
+  Iv x, y, z, t;
+  float4 *slice;
+  bool take;
+  Iv sens[4];  // out
+};
+static __device__ __noinline__ bool own_slice_passes(OwnSlice &a, NarrowRows R, uint32_t lane) {
+  const uint32_t cells = a.cells, per = min(cells, min(31u, 32u * a.slice_len / max(a.log_len, 1u) - 1u));
+  R.rf -= min(lane, cells) * 8u;
+  R.stride = (per + 1u) * 8u;
+  R.log_step = per + 1u;
+  bool bad = false;
+  for (uint32_t first = 0; first < cells; first += per) {
+    const uint32_t c = lane - first, col = min(c, per);  // lanes below `first` wrap around
+    NarrowRows Q = R;
+    Q.rf += col * 8u;
+    uint32_t n = 0;
+    Iv s[4];
+    bool b = false;
+    __syncwarp();  // the lanes' columns change
+    (void)narrow_forward<false>(a.code, a.len, a.out_reg, Q, lane, a.x, a.y, a.z, a.t, a.slice + col, nullptr, n);
+    narrow_reverse<false>(a.code, a.len, a.nregs, a.out_reg, Q, lane, a.slice + col, n, a.take && c < per, true, s, b);
+    if (c < per) {
+      for (int q = 0; q < 4; ++q) a.sens[q] = s[q];
+      bad = b;
+    }
+  }
+  __syncwarp();
+  return bad;
+}
+// Whether an item of n parents can prune this tape within its warp's slices:
+// the decisions and the kept instructions of a group per parent.
+__device__ __forceinline__ bool slice_prunes(const LaunchParams &P, const TapeRec &TR, uint32_t n) {
+  return TR.n_minmax <= P.slice_len && (unsigned long long)n * TR.len <= 64ull * P.slice_len;
 }
 
 template <bool D>
@@ -483,6 +561,9 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
   bool want_prune = false;
   float4 *lg = nullptr;
   uint2 *dg = nullptr;
+  // whether a full level turned the item away from the wide path (or it found
+  // the wide list full): it then leaves the log arena alone
+  auto leaves_arena = [&]() { return !D && may_go_narrow(P, S.wide, it.level, P.recs[it.rec].len); };
 
   if (b_eval) {
     // ---- the most pruned tape valid for every evaluated cell
@@ -491,7 +572,9 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
     TR = P.recs[rec];
     if (!(TR.c_level == it.level && TR.c_lo <= tl && th <= TR.c_hi)) find_valid(P, rec, TR, tl, th);
     for (int attempt = 0; attempt < 2; ++attempt) {
-      want_prune = (flags & SF_PRUNING) && TR.len >= TSI_PRUNE_MIN_LEN && TR.nregs <= TSI_PRUNE_MAX_REGS;
+      const bool own_slice = leaves_arena(), in_turns = own_slice && !slice_holds(P, it.n, log_bound(S.wide, TR.len));
+      want_prune = (flags & SF_PRUNING) && TR.len >= TSI_PRUNE_MIN_LEN && TR.nregs <= TSI_PRUNE_MAX_REGS &&
+                   (!own_slice || slice_prunes(P, TR, it.n));
       if (lane == 0 && attempt == 0) {
         if (TR.len >= S.wide.min_len) ws[ST_NARROW_LONG] += 1;
         ws[ST_NARROW_LEN_MAX] = max(ws[ST_NARROW_LEN_MAX], (unsigned long long)TR.len);
@@ -499,19 +582,24 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       lg = nullptr;
       dg = nullptr;
       if (any_deriv || want_prune) {
-        float4 *lgs = nullptr;
-        uint2 *dgs = nullptr;
-        if (!item_scratch(P, step, it.scene, TR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
+        float4 *lgs = slice_log;
+        uint2 *dgs = want_prune ? slice_dec : nullptr;
+        if (!own_slice && !item_scratch(P, step, it.scene, TR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
         lg = lgs;
         dg = dgs;
       }
       const long long q0 = clock64();
       uint32_t nlog = 0;
-      float4 *opl = any_deriv ? lg + min(lane, narrow_cells(it.n)) : nullptr;  // this lane's column of the log
-      field = narrow_forward<D>(TR.code, TR.len, TR.out_reg, R, lane, cx, cy, cz, targ, opl, dg, nlog);
-      const long long q1 = clock64();
       bool bad = false;
-      if (any_deriv)
+      float4 *opl = any_deriv ? lg + min(lane, narrow_cells(it.n)) : nullptr;  // this lane's column of the log
+      field = narrow_forward<D>(TR.code, TR.len, TR.out_reg, R, lane, cx, cy, cz, targ, in_turns ? nullptr : opl, dg, nlog);
+      const long long q1 = clock64();
+      if (any_deriv && in_turns) {
+        OwnSlice o{TR.code, TR.len, TR.nregs, TR.out_reg, log_bound(S.wide, TR.len), P.slice_len, narrow_cells(it.n),
+                   cx, cy, cz, targ, lg, take_deriv, {sens[0], sens[1], sens[2], sens[3]}};
+        bad = own_slice_passes(o, R, lane);
+        for (int q = 0; q < 4; ++q) sens[q] = o.sens[q];
+      } else if (any_deriv)
         narrow_reverse<D>(TR.code, TR.len, TR.nregs, TR.out_reg, R, lane, opl, nlog, take_deriv, (flags & SF_STRICT) != 0, sens,
                           bad);
       if (lane == 0 && attempt == 0) {
@@ -652,7 +740,8 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       uint32_t wrec = rec;
       TapeRec WR;
       find_valid(P, wrec, WR, wl, wh);
-      if (WR.len >= route_len(P, S.wide, step, it.level + 1u)) {
+      const bool long_tape = goes_wide(P, S.wide, step, it.level + 1u, WR.len), own_slice = leaves_arena();
+      if (long_tape) {
         // A long tape: no pass over it on one warp.  A group with a widened
         // child hands its children, with that tape's record, to the wide
         // path; the other groups prune from the first pass's decisions.
@@ -664,12 +753,13 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       } else {
         prec = wrec;
         PR = WR;
-        want_prune = (flags & SF_PRUNING) && PR.len >= TSI_PRUNE_MIN_LEN && PR.nregs <= TSI_PRUNE_MAX_REGS;
+        want_prune = (flags & SF_PRUNING) && PR.len >= TSI_PRUNE_MIN_LEN && PR.nregs <= TSI_PRUNE_MAX_REGS &&
+                     (!own_slice || slice_prunes(P, PR, it.n));
       }
-      if (want_prune && WR.len < route_len(P, S.wide, step, it.level + 1u)) {
-        float4 *lgs;
-        uint2 *dgs;
-        if (!item_scratch(P, step, it.scene, PR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
+      if (want_prune && !long_tape) {
+        float4 *lgs = slice_log;
+        uint2 *dgs = slice_dec;
+        if (!own_slice && !item_scratch(P, step, it.scene, PR.len, lane, slice_log, slice_dec, lgs, dgs)) return;
         lg = lgs;
         dg = dgs;
         const Iv tw = enq ? Iv{nl, nh} : targ;
@@ -774,8 +864,9 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
     const uint32_t next_len = (new_rec == prec) ? PR.len : ((new_rec == rec) ? TR.len : cnt);
     if (k == 0 && E != 0) {
       if (next_len >= wide_min_len(S.wide, it.level + 1u)) atomicAdd(&P.long_count[si.next], (uint32_t)__popc(E));
-      push_children(P, S, it.scene, new_rec, step, it.level, E, cb, next_len >= route_len(P, S.wide, step, it.level + 1u),
-                    ws);
+      const bool wide = goes_wide(P, S.wide, step, it.level + 1u, next_len);
+      const bool either = !wide && may_go_narrow(P, S.wide, it.level + 1u, next_len);
+      push_children(P, S, it.scene, new_rec, step, it.level, E, cb, wide, either ? log_bound(S.wide, next_len) : 0u, ws);
     }
   }
 
@@ -1069,7 +1160,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
       // wide path evaluates the full tape), or may: children the full wide
       // list turns away run narrow on this record
       const bool wide_room = *(const volatile uint32_t *)&P.witem_count[si.next] + 8u <= P.witem_cap;
-      if (total < n_narrow && (total < route_len(P, W, step, it.level + 1u) || !wide_room)) {
+      if (total < n_narrow && (!goes_wide(P, W, step, it.level + 1u, total) || !wide_room)) {
         const unsigned long long off = code_alloc(P, total);
         if (off != ~0ull) {
           const uint32_t ri = rec_alloc(P);
@@ -1169,7 +1260,8 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
     const uint32_t len = (new_rec == S.root_rec) ? root.len : sh.cnt;
     if (tid == 0 && len >= wide_min_len(W, it.level + 1u)) atomicAdd(&P.long_count[si.next], (uint32_t)__popc(E));
     push_children_warp(P, S, it.scene, new_rec, step, it.level, E, it.parent[1], it.parent[2] != 0u,
-                       len >= route_len(P, W, step, it.level + 1u), ws, tid);
+                       goes_wide(P, W, step, it.level + 1u, len),
+                       may_go_narrow(P, W, it.level + 1u, len) ? log_bound(W, len) : 0u, ws, tid);
   }
   if (tid == 0) {
     const long long f3 = clock64();

@@ -74,6 +74,16 @@ uint32_t handler_of(uint32_t op, uint32_t top) {
 
 }  // namespace
 
+// Whether the narrow interpreter takes an instruction as linear, to nearest
+// (narrow_interp.cuh, decode_forward).
+static bool linear_handler(uint32_t h, float lit) {
+  switch (h) {
+    case H_ADD_II: case H_SUB_II: case H_ADD_IF: case H_SUB_IF: case H_SUB_FI: case H_NEG: case H_COPY: return true;
+    case H_MUL_IF: return std::fabs(lit) <= 1000000.0f;
+    default: return false;
+  }
+}
+
 // A bound of log2 |value| from those of the operands; NaN for handlers whose
 // value or reverse rule is infinite on ordinary operands.
 static double magnitude(uint32_t h, double a, double b, float lit) {
@@ -179,6 +189,7 @@ bool compile_tape(const std::vector<IrInstr> &ins, PackedTape &out, tsi_status &
                        (has_a && a_slot < 4u ? TSI_W0_RAW_A : 0u) | (has_b && b_slot < 4u ? TSI_W0_RAW_B : 0u));
     out.code.push_back(w1);
     if (TSI_H_IS_MINMAX(h)) out.n_minmax++;
+    if (odd || !linear_handler(h, lit)) out.log_len++;
     const uint32_t da = has_a ? deps[a_slot] : 0u, db = has_b ? deps[b_slot] : 0u;
     deps[j] = uint8_t(da | db);
     out.deps.push_back(uint8_t(da | (db << 4)));

@@ -21,6 +21,7 @@ struct PackedTape {
   // that the skip rule (compute.wgsl:3800-3806) does not keep from it, for
   // arguments up to 2^20.
   bool strict = false;
+  uint32_t log_len = 0;       // instructions whose operands the narrow interpreter logs, to nearest
   std::vector<uint8_t> deps;  // per instruction: the arguments A depends on, B's in the upper four bits
   std::vector<uint32_t> slot_reg;  // register of every SSA slot (debug, tests)
 };
