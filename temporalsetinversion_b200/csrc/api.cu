@@ -571,12 +571,18 @@ void make_camera(const tsi_params &p, const tsi_uniforms &u, TraceParams &T) {
   T.rendermode = u.rendermode;
   T.normal_viz = p.normal_viz ? 1u : 0u;
   T.darken = p.octree_darken_factor;
+  // The extents of the root and of the smallest cells are ordinary, and the
+  // latter at least eight steps of the numbers at the root's bounds: a level's
+  // bounds round to a step, which adds up to two steps over the levels, so
+  // that extents stay within a quarter of the nominal ones.  (Far from the
+  // origin boxes may round to no extent at all.)
   T.plain_boxes = 1u;
-  for (int a = 0; a < 3; ++a) {  // extents of the root and of the smallest cells
-    const float e = p.root_hi[a] - p.root_lo[a];
-    if (!(e <= 16777216.0f) || !(ldexpf(e, -(int)tree_levels(p) - 1) >= 5.9604645e-08f) ||
-        !(fabsf(p.root_lo[a]) <= 16777216.0f))
-      T.plain_boxes = 0u;
+  const int levels = (int)tree_levels(p);
+  for (int a = 0; a < 3; ++a) {
+    const float e = p.root_hi[a] - p.root_lo[a], far = std::max(fabsf(p.root_lo[a]), fabsf(p.root_hi[a]));
+    const float least = ldexpf(e, -levels);
+    if (!(e <= 16777216.0f) || !(least >= 1.1920929e-07f) || !(far <= 16777216.0f) || !(least >= far * 9.5367432e-07f))
+      T.plain_boxes = 0u;  // (2^24, 2^-23, 2^-20 of a number: eight of its steps or more)
   }
 }
 

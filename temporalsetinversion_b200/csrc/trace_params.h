@@ -18,7 +18,7 @@ struct TraceParams {
   float rendermode;
   uint32_t normal_viz;
   float darken;       // octree_darken_factor
-  uint32_t plain_boxes;  // every node's extents lie in [2^-24, 2^24] (trace_walk.cuh's fast walk)
+  uint32_t plain_boxes;  // every node's extents, as rounded, lie in [2^-24, 2^24] (walk_plain, trace_walk.cuh)
   VoxelPoolDev pool;
   // fast normals: the scene's full tape, evaluated at points (nullptr: off)
   const uint2 *code;

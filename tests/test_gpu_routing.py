@@ -56,10 +56,10 @@ def test_unpruned_long_tapes_need_no_log(kind):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("parents", [1, 4])
-@pytest.mark.parametrize("n,localsubdiv", [(64, 9), (330, 7)])
+@pytest.mark.parametrize("n,localsubdiv", [(64, 9), (330, 7), (600, 7)])
 def test_second_runs_on_the_full_tape_need_no_log(n, localsubdiv, parents):
     """Cells of crowded levels with infinite sensitivities, on full tapes of
-    1191 and of 6 thousand instructions, and the same arena.  (The threshold
+    1191, 6 and 11 thousand instructions, and the same arena.  (The threshold
     is below every pruned tape's length: no item is a short one.)"""
     tape = steep(n)
     with Device(log_arena_bytes=1 << 16) as dev:

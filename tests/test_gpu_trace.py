@@ -129,3 +129,42 @@ def test_pipelined_frames_match_sequential(device):
         assert np.array_equal(depth.reshape(want["depth"].shape), want["depth"]), f
         assert np.array_equal(normal.reshape(want["normal"].shape), want["normal"]), f
 
+
+
+def _steps(lo: float, n: int) -> float:
+    return n * float(np.spacing(np.float32(abs(lo))))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lo,extent", [
+    (0.0, 1.0), (0.0, 2.0 ** -18), (0.0, 2.0 ** -19), (1.0e5, _steps(1.0e5, 4)), (1.0e5, _steps(1.0e5, 6)),
+    (-1.0e5, _steps(1.0e5, 12)), (1.0e5, _steps(1.0e5, 100)), (1.0e5, _steps(1.0e5, 512))])
+def test_walk_at_the_limits_of_ordinary_rays_and_boxes(device, lo, extent):
+    """Rays along a diagonal (steps on two and three axes at once) and within
+    1e-9 of an axis, boxes of extents around 2^-24, and boxes some steps of
+    the numbers at their bounds wide: far from the origin the smallest ones
+    round to no extent at all."""
+    c = lo + 0.5 * extent
+    b = scenes.IRBuilder()
+    d = [b.mul(b.sub(b.X, c), 1.0 / extent), b.sub(b.Y, 0.5), b.sub(b.Z, 0.5)]
+    s = b.add(b.add(b.mul(d[0], d[0]), b.mul(d[1], d[1])), b.mul(d[2], d[2]))
+    tape = api.IR.new(b.text(b.sub(b.sqrt(s), 0.3))).gpu_instructions
+    p = api.default_params(localsubdiv=8, root_lo=(lo, 0.0, 0.0), root_hi=(lo + extent, 1.0, 1.0))
+    gs, os_ = Scene(device, Tape.upload(device, tape), p), oracle.Scene(tape, p)
+    gs.invert(0.0)
+    os_.invert(0.0)
+    hits = 0
+    for eye in ((2.0, 2.0, 2.0), (-2.0, 0.4, 0.6), (3.0, 0.9, 0.2), (1e-9, 0.0, 1.0), (1.0, 1e-7, 1e-9)):
+        at = (c + eye[0], 0.5 + eye[1], 0.5 + eye[2])
+        u = api.make_uniforms(scenes.camera_look_at(at, (c, 0.5, 0.5)), (33, 33), 0.0)
+        g, o = gs.trace(u), os_.trace(u)
+        hit = o["depth"] >= 0
+        hits += int(hit.sum())
+        # (a ray that misses is darkened at every step: what the conversion of
+        # an infinity to an integer gives in a box without an extent decides
+        # how many it makes, and that differs from the oracle's)
+        bare = abs(lo) > 0 and extent < _steps(lo, 32)
+        for k in ("depth", "normal", "rgba"):
+            eq = g[k].view(np.uint32) == o[k].view(np.uint32)
+            assert eq[hit].all() if bare and k == "rgba" else eq.all(), (k, eye)
+    assert hits >= 10
