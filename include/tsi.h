@@ -577,7 +577,9 @@ TSI_API tsi_status tsi_compile_wide_gpu_instructions(const tsi_gpu_instruction *
                                                      uint32_t *n_bundles);
 /* Elementwise device f32 math, for the math tests: which = 0 sin(a),
  * 1 exp(a), 2 log(a), 3 atan2(a, b), 4 powi(a, (int)b), 5 min(a, b),
- * 6 max(a, b) (minimumNumber / maximumNumber), 7 fminf, 8 fmaxf. */
+ * 6 max(a, b) (minimumNumber / maximumNumber), 7 fminf, 8 fmaxf; the forms
+ * without branches for operands well inside the normal range: 9 1 / a,
+ * 10 a / b, 11 sqrt(a), 12 floor(a / (pi/2)). */
 TSI_API tsi_status tsi_debug_math(tsi_ctx *ctx, int32_t which, uint32_t n, const float *a, const float *b,
                                   float *out);
 /* Per-level profile of the context's last inversion: device ms of each

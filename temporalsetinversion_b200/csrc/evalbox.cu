@@ -106,6 +106,10 @@ __global__ void math_kernel(int which, uint32_t n, const float *a, const float *
     case 6: r = fm_max(a[i], b[i]); break;
     case 7: r = fminf(a[i], b[i]); break;
     case 8: r = fmaxf(a[i], b[i]); break;
+    case 9: r = fm_rcp_in(a[i]); break;
+    case 10: r = fm_div_in(a[i], b[i], fm_rcp_in(b[i])); break;
+    case 11: r = fm_sqrt_in(a[i]); break;
+    case 12: r = IA<false>::quadrant(a[i]); break;
     default: r = 0.0f; break;
   }
   out[i] = r;

@@ -83,9 +83,11 @@ TSI_DEV F2 f2_mul_alone(F2 a, F2 b) {
 // for operands and results well inside the normal range (the callers check):
 // the hardware's approximation and one residual step each, Markstein's
 // scheme ("Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990).  Compared with __frcp_rn and __fsqrt_rn for every
-// mantissa and exponents -60..60 and -80..80, the quotient with __fdiv_rn for
-// 8.6 thousand million pairs of exponents -20..20: no difference.
+// processor", 1990).  tests/test_gpu_short_math.py compares them with IEEE
+// operations: reciprocals and roots for every mantissa at the ends and in the
+// middle of the callers' exponents, quotients of random pairs and next to
+// midpoints.  (A quotient of -0 comes out as +0; the tracer, the only one to
+// divide so, takes its floor and the difference from that, the same of both.)
 TSI_DEV float fm_rcp_in(float d) {
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));

@@ -365,8 +365,9 @@ struct IA {
   }
   // floor(x / (pi/2 as f32)) for |x| < 1e7, as floor(__fdiv_rn(x, kHALFPI))
   // gives it: the quotient by the reciprocal, corrected once by its exact
-  // residual, equals the correctly rounded one for every f32 from 0.5 to 2^25
-  // (checked exhaustively); below 0.5 the floor is that of x itself.
+  // residual; below 0.5 the floor is that of x itself.  (Compared at and next
+  // to every multiple of pi/2, where alone the floor could differ:
+  // tests/test_gpu_short_math.py.)
   static TSI_DEV float quadrant(float x) {
     const float rc = 0.6366197466850281f;  // 1 / kHALFPI rounded to f32
     const float q = __fmul_rn(x, rc);
