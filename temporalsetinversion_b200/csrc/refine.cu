@@ -227,6 +227,12 @@ __device__ __forceinline__ bool goes_wide(const LaunchParams &P, const WideDev &
   const uint32_t next = step_idx(step).next;
   return len >= (unsigned long long)from * waves || *(const volatile uint32_t *)&P.item_count[next] > P.item_cap / 2u;
 }
+// The same for a warp that goes on together: lane 0's answer, for the list may
+// grow between the reads of two lanes.
+__device__ __forceinline__ bool warp_goes_wide(const LaunchParams &P, const WideDev &W, uint32_t step, uint32_t level,
+                                               uint32_t len) {
+  return __shfl_sync(FULL_MASK, goes_wide(P, W, step, level, len) ? 1u : 0u, 0) != 0u;
+}
 
 // Reserves n words of the code arena (a ring of code_cap words, a power of
 // two); returns the word offset, or ~0 when the ring has no room left above
@@ -740,7 +746,7 @@ __device__ __noinline__ void process_item(const LaunchParams &P, const WorkItem 
       uint32_t wrec = rec;
       TapeRec WR;
       find_valid(P, wrec, WR, wl, wh);
-      const bool long_tape = goes_wide(P, S.wide, step, it.level + 1u, WR.len), own_slice = leaves_arena();
+      const bool long_tape = warp_goes_wide(P, S.wide, step, it.level + 1u, WR.len), own_slice = leaves_arena();
       if (long_tape) {
         // A long tape: no pass over it on one warp.  A group with a widened
         // child hands its children, with that tape's record, to the wide
@@ -1260,7 +1266,7 @@ __device__ __forceinline__ void finish_group(const LaunchParams &P, const WorkIt
     const uint32_t len = (new_rec == S.root_rec) ? root.len : sh.cnt;
     if (tid == 0 && len >= wide_min_len(W, it.level + 1u)) atomicAdd(&P.long_count[si.next], (uint32_t)__popc(E));
     push_children_warp(P, S, it.scene, new_rec, step, it.level, E, it.parent[1], it.parent[2] != 0u,
-                       goes_wide(P, W, step, it.level + 1u, len),
+                       warp_goes_wide(P, W, step, it.level + 1u, len),
                        may_go_narrow(P, W, it.level + 1u, len) ? log_bound(W, len) : 0u, ws, tid);
   }
   if (tid == 0) {
