@@ -3,10 +3,10 @@
 
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <iterator>
 #include <limits>
 #include <map>
-#include <set>
 #include <utility>
 #include <cstring>
 
@@ -230,11 +230,21 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   auto handler = [&](uint32_t j) { return TSI_W0_H(narrow.code[2 * (j - 4)]); };
   // users of every value, in program order (an instruction reading one value
   // through both operands is one user)
-  std::vector<std::vector<uint32_t>> users(n);
+  std::vector<uint32_t> first_user(size_t(n) + 1, 0), user;  // value v's: user[first_user[v] .. first_user[v + 1])
   for (uint32_t j = 4; j < n; ++j) {
-    if (opa[j] != TSI_NONE) users[opa[j]].push_back(j);
-    if (opb[j] != TSI_NONE && opb[j] != opa[j]) users[opb[j]].push_back(j);
+    if (opa[j] != TSI_NONE) ++first_user[opa[j] + 1];
+    if (opb[j] != TSI_NONE && opb[j] != opa[j]) ++first_user[opb[j] + 1];
   }
+  for (uint32_t v = 0; v < n; ++v) first_user[v + 1] += first_user[v];
+  user.resize(first_user[n]);
+  {
+    std::vector<uint32_t> at(first_user.begin(), first_user.end() - 1);
+    for (uint32_t j = 4; j < n; ++j) {
+      if (opa[j] != TSI_NONE) user[at[opa[j]]++] = j;
+      if (opb[j] != TSI_NONE && opb[j] != opa[j]) user[at[opb[j]]++] = j;
+    }
+  }
+  auto users = [&](uint32_t v) { return first_user[v + 1] - first_user[v]; };
   // The reverse pass accumulates a value's sensitivity user by user, in
   // reverse program order, and that order fixes the rounding.  A value with
   // one user receives it directly; a value with several gets one
@@ -244,8 +254,8 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   // users found here.
   for (uint32_t j = 4; j < n; ++j) {
     const uint32_t w0 = narrow.code[2 * (j - 4)];
-    if ((TSI_W0_FA(w0) && opa[j] != TSI_NONE && users[opa[j]].size() != 1) ||
-        (TSI_W0_FB(w0) && opb[j] != TSI_NONE && users[opb[j]].size() != 1)) {
+    if ((TSI_W0_FA(w0) && opa[j] != TSI_NONE && users(opa[j]) != 1) ||
+        (TSI_W0_FB(w0) && opb[j] != TSI_NONE && users(opb[j]) != 1)) {
       status = TSI_ERR_INVALID_ARGUMENT;
       why = "single-use flag on a value with several users";
       return false;
@@ -254,10 +264,10 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   std::vector<uint32_t> gbase(n, TSI_NONE), rec_a(n, TSI_NONE), rec_b(n, TSI_NONE);
   uint32_t ncontrib = 0;
   for (uint32_t v = 0; v < n; ++v) {
-    if (users[v].size() < 2) continue;
+    if (users(v) < 2) continue;
     gbase[v] = ncontrib;
-    for (size_t u = users[v].size(); u-- > 0;) {  // last user first
-      const uint32_t j = users[v][u];
+    for (uint32_t u = first_user[v + 1]; u-- > first_user[v];) {  // last user first
+      const uint32_t j = user[u];
       if (opa[j] == v) rec_a[j] = ncontrib;
       if (opb[j] == v) rec_b[j] = ncontrib;
       ++ncontrib;
@@ -287,7 +297,7 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   std::vector<uint32_t> prio(n, 0);
   for (uint32_t j = n; j-- > 4;) {
     uint32_t p = 0;
-    for (uint32_t u : users[j]) p = std::max(p, prio[u]);
+    for (uint32_t u = first_user[j]; u < first_user[j + 1]; ++u) p = std::max(p, prio[user[u]]);
     prio[j] = p + 1u;
   }
   std::vector<uint32_t> indeg(n, 0);
@@ -295,10 +305,16 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
     if (opa[j] != TSI_NONE && opa[j] >= 4) ++indeg[j];
     if (opb[j] != TSI_NONE && opb[j] >= 4 && opb[j] != opa[j]) ++indeg[j];
   }
-  using Key = std::pair<uint32_t, uint32_t>;  // (~priority, instruction): highest priority, then oldest, first
-  std::vector<std::set<Key>> ready(64);
+  // heaps of ~priority << 32 | instruction: the least, with the highest
+  // priority and then the oldest, in front
+  std::vector<std::vector<uint64_t>> ready(64);
+  auto insert = [&](uint32_t j) {
+    std::vector<uint64_t> &r = ready[handler(j)];
+    r.push_back(uint64_t(~prio[j]) << 32 | j);
+    std::push_heap(r.begin(), r.end(), std::greater<uint64_t>());
+  };
   for (uint32_t j = 4; j < n; ++j)
-    if (indeg[j] == 0) ready[handler(j)].insert(Key(~prio[j], j));
+    if (indeg[j] == 0) insert(j);
   std::vector<std::vector<std::vector<uint32_t>>> bundles;  // bundle -> groups -> instructions
   uint32_t scheduled = 0;
   std::vector<uint32_t> next;
@@ -311,16 +327,16 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
     bool inline_ready = false;
     for (uint32_t h = 0; h < 64; ++h)
       if (!ready[h].empty()) {
-        cp = std::max(cp, ~ready[h].begin()->first);
+        cp = std::max(cp, ~uint32_t(ready[h].front() >> 32));
         inline_ready = inline_ready || inline_handler(h);
       }
     auto eligible = [&](uint32_t h) {
-      return inline_handler(h) || !inline_ready || ~ready[h].begin()->first >= cp;
+      return inline_handler(h) || !inline_ready || ~uint32_t(ready[h].front() >> 32) >= cp;
     };
     while (groups.size() < groups_per_bundle) {
       uint32_t hb = 64;
       for (uint32_t h = 0; h < 64; ++h)
-        if (!ready[h].empty() && eligible(h) && (hb == 64 || *ready[h].begin() < *ready[hb].begin())) hb = h;
+        if (!ready[h].empty() && eligible(h) && (hb == 64 || ready[h].front() < ready[hb].front())) hb = h;
       if (hb == 64) break;
       // a group of an out-of-line handler (elementary functions, divisions:
       // a step of them costs several steps of the others) takes every ready
@@ -329,8 +345,9 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
       do {
         std::vector<uint32_t> g;
         while (g.size() < 32u && !ready[hb].empty()) {
-          g.push_back(ready[hb].begin()->second);
-          ready[hb].erase(ready[hb].begin());
+          g.push_back(uint32_t(ready[hb].front()));
+          std::pop_heap(ready[hb].begin(), ready[hb].end(), std::greater<uint64_t>());
+          ready[hb].pop_back();
         }
         groups.push_back(std::move(g));
       } while (!inline_handler(hb) && !ready[hb].empty() && groups.size() < groups_per_bundle);
@@ -344,10 +361,10 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
     for (const auto &g : groups)
       for (uint32_t j : g) {
         ++scheduled;
-        for (uint32_t u : users[j])
-          if (--indeg[u] == 0) next.push_back(u);
+        for (uint32_t u = first_user[j]; u < first_user[j + 1]; ++u)
+          if (--indeg[user[u]] == 0) next.push_back(user[u]);
       }
-    for (uint32_t u : next) ready[handler(u)].insert(Key(~prio[u], u));
+    for (uint32_t u : next) insert(u);
     bundles.push_back(std::move(groups));
   }
   const uint32_t nb = uint32_t(bundles.size());
@@ -395,7 +412,7 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
       S[8] = rec_a[j];
       S[9] = rec_b[j];
       S[10] = gbase[j];
-      S[11] = gbase[j] == TSI_NONE ? 0u : uint32_t(users[j].size());
+      S[11] = gbase[j] == TSI_NONE ? 0u : users(j);
     }
     out.bundles[2 * k] = off;
     out.bundles[2 * k + 1] = count;
@@ -403,7 +420,7 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
   }
   for (uint32_t a = 0; a < 4; ++a) {
     out.arg_gbase[a] = gbase[a];
-    out.arg_gcount[a] = gbase[a] == TSI_NONE ? 0u : uint32_t(users[a].size());
+    out.arg_gcount[a] = gbase[a] == TSI_NONE ? 0u : users(a);
   }
   out.ncontrib = ncontrib;
   out.nvalues = n;
@@ -414,22 +431,25 @@ bool compile_wide(const std::vector<IrInstr> &ins, const PackedTape &narrow, Wid
 // Slots of the sensitivities in the order of the reverse pass (wide_tape.h):
 // first fit, but for single slots, which are taken again last in, first out.
 struct SlotPool {
-  std::map<uint32_t, uint32_t> gaps{{0u, 0xffffffffu}};  // first slot, length
+  std::map<uint32_t, uint32_t> gaps;  // first slot, length
   std::vector<uint32_t> ones;
-  uint32_t top = 0;
+  uint32_t tail = 0, top = 0;  // from tail on nothing is taken, from top on nothing ever was
   uint32_t take(uint32_t n) {
     if (n == 1u && !ones.empty()) {
       const uint32_t at = ones.back();
       ones.pop_back();
       return at;
     }
-    auto it = gaps.begin();
-    while (it->second < n) ++it;
-    const uint32_t at = it->first, left = it->second - n;
-    gaps.erase(it);
-    if (left) gaps.emplace(at + n, left);
-    top = std::max(top, at + n);
-    return at;
+    for (auto it = gaps.begin(); it != gaps.end(); ++it) {
+      if (it->second < n) continue;
+      const uint32_t at = it->first, left = it->second - n;
+      gaps.erase(it);
+      if (left) gaps.emplace(at + n, left);
+      return at;
+    }
+    tail += n;
+    top = std::max(top, tail);
+    return tail - n;
   }
   void give(uint32_t at, uint32_t n) {
     if (n == 1u) {
@@ -444,11 +464,13 @@ struct SlotPool {
     if (next != gaps.begin()) {
       auto prev = std::prev(next);
       if (prev->first + prev->second == at) {
-        prev->second += n;
-        return;
+        at = prev->first;
+        n += prev->second;
+        gaps.erase(prev);
       }
     }
-    gaps.emplace(at, n);
+    if (at + n == tail) tail = at;
+    else gaps.emplace(at, n);
   }
 };
 
@@ -473,10 +495,8 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
   };
   std::vector<uint32_t> targets;
   auto push4 = [](std::vector<uint32_t> &v, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    v.push_back(a);
-    v.push_back(b);
-    v.push_back(c);
-    v.push_back(d);
+    const uint32_t q[4] = {a, b, c, d};
+    v.insert(v.end(), q, q + 4);
   };
   const uint32_t minus0 = 0x80000000u;
   // ---- the sensitivities' slots: per value its place or its records' first
@@ -547,6 +567,16 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
     if (out.fslots > 65536u) fplace.clear();
   }
   const bool small = nv2 <= 65536u && out.gslots <= 65536u;  // (a value's records are as many as its users)
+  {  // the arrays' final sizes, or a little more
+    size_t padded = 32;  // and a slot past a warp's last group
+    for (uint32_t k = 0; k < wt.nbundles; ++k) padded += (wt.bundles[2 * k + 1] + 31u) & ~31u;
+    out.fwd.reserve(padded * 4u);
+    if (!fplace.empty()) out.fwd_slots.reserve(padded * 4u);
+    out.rev.reserve(padded * 8u);
+    targets.reserve(padded * 4u);
+    if (small) out.rev16.reserve(padded * 4u);
+    out.live.reserve(padded * 4u);
+  }
   // One group (warp g of bundle k) of the forward or reverse streams; its
   // kind.
   auto emit = [&](uint32_t k, uint32_t g, bool reverse) -> uint32_t {
@@ -570,59 +600,75 @@ void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out) {
       case H_MIN_II: case H_MIN_IF: kind = WK_MM; break;
       default: break;
     }
+    const bool has_a = h != H_CONST;  // (B: ii)
+    // 32 more slots at an array's end
+    auto grow = [](std::vector<uint32_t> &v) {
+      v.resize(v.size() + 128u);
+      return &v[v.size() - 128u];
+    };
+    auto put = [](uint32_t *&at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+      at[0] = a;
+      at[1] = b;
+      at[2] = c;
+      at[3] = d;
+      at += 4;
+    };
+    if (!reverse) {
+      uint32_t c = base, flip = 0u;
+      switch (h) {
+        case H_ADD_II: case H_COPY: c |= WC_ZERO; break;
+        case H_SUB_II: c |= WC_ZERO | WC_NEG | WC_SWAP; break;
+        case H_SUB_IF: flip = minus0; break;
+        case H_SUB_FI: c |= WC_NEG | WC_SWAP; break;
+        case H_NEG: c |= WC_NEG | WC_SWAP | WC_ZERO; break;
+        default: break;
+      }
+      uint32_t *f = grow(out.fwd), *fs = fplace.empty() ? nullptr : grow(out.fwd_slots);
+      for (uint32_t s = 0; s < 32u; ++s) {
+        const uint32_t *S = s < left ? &wt.slots[size_t(first + s) * 12] : nullptr;
+        const bool pad = !S || (S[0] & 63u) == TSI_H_PAD;
+        uint32_t x = pad || !has_a ? zero : S[6], y = pad || !ii ? zero : S[7], w = pad || ii ? 0u : S[3];
+        const uint32_t d = pad ? dummy : S[4];
+        // the ordinal or the handler travels where the literal or B does not
+        if (kind == WK_MM || kind == WK_OTHER) (ii ? w : y) = kind == WK_OTHER ? h : pad ? n_minmax : S[5];
+        if (h == H_SUB_II) std::swap(x, y);
+        w = (c & WC_ZERO) ? minus0 : w ^ flip;
+        put(f, c | (d << WC_DST_SHIFT), x, y, w);
+        if (fs) put(fs, c | (d << WC_DST_SHIFT), fplace[x] | (fplace[d] << 16), ii ? fplace[y] : y, w);
+      }
+      return kind;
+    }
+    uint32_t *r = grow(out.rev), *t = grow(targets), *r16 = small ? grow(out.rev16) : nullptr;
     for (uint32_t s = 0; s < 32u; ++s) {
       const uint32_t *S = s < left ? &wt.slots[size_t(first + s) * 12] : nullptr;
       const bool pad = !S || (S[0] & 63u) == TSI_H_PAD;
-      const uint32_t a = pad || S[6] == TSI_NONE ? zero : S[6];
-      const uint32_t b = pad || S[7] == TSI_NONE ? zero : S[7];
-      const uint32_t mmo = pad || S[5] == TSI_NONE ? n_minmax : S[5];
-      const uint32_t lit = pad || ii ? 0u : S[3];
-      uint32_t c = base, x = a, y = ii ? b : zero, w = lit;
-      if (kind == WK_OTHER && !reverse) {  // the handler travels where the literal or B does not
-        if (ii) w = h;
-        else y = h;
-      }
-      if (!reverse) {
-        if (kind == WK_MM) {
-          if (ii) w = mmo;
-          else y = mmo;
-        }
-        switch (h) {
-          case H_ADD_II: case H_COPY: c |= WC_ZERO; w = minus0; break;
-          case H_SUB_II: c |= WC_ZERO | WC_NEG | WC_SWAP; x = b; y = a; w = minus0; break;
-          case H_SUB_IF: w = lit ^ minus0; break;
-          case H_SUB_FI: c |= WC_NEG | WC_SWAP; break;
-          case H_NEG: c |= WC_NEG | WC_SWAP | WC_ZERO; w = minus0; break;
-          default: break;
-        }
-        push4(out.fwd, c | ((pad ? dummy : S[4]) << WC_DST_SHIFT), x, y, w);
-        if (!fplace.empty())
-          push4(out.fwd_slots, c | ((pad ? dummy : S[4]) << WC_DST_SHIFT),
-                fplace[x] | (fplace[pad ? dummy : S[4]] << 16), ii ? fplace[y] : y, w);
-        continue;
-      }
+      const uint32_t x = pad || !has_a ? zero : S[6], y = pad || !ii ? zero : S[7], w = pad || ii ? 0u : S[3];
+      uint32_t c = base;
       if (h == H_SUB_II) c |= WC_NEG2;
       if (h == H_SUB_FI || h == H_NEG) c |= WC_NEG;
-      const uint32_t fa = pad ? 0u : (S[0] >> 6) & 1u, fb = pad ? 0u : (S[0] >> 7) & 1u;
-      if (fa && (!ii || fb)) c |= WC_SKIP;
       uint32_t ta = dummy, tb = dummy, src = zero, n = 0;
       uint32_t ga = 1u, gb = 1u, gs = 0u;  // the same in the 16-bit form's slots
       if (!pad) {
-        if (S[6] != TSI_NONE) ta = S[8] != TSI_NONE ? nv2 + S[8] : S[6];
-        if (S[7] != TSI_NONE) tb = S[9] != TSI_NONE ? nv2 + S[9] : S[7];
+        const uint32_t fa = (S[0] >> 6) & 1u, fb = (S[0] >> 7) & 1u;
+        if (fa && (!ii || fb)) c |= WC_SKIP;
+        auto target = [&](uint32_t v, uint32_t rec, uint32_t &to, uint32_t &place16) {
+          const bool one = rec == TSI_NONE;
+          to = one ? v : nv2 + rec;
+          place16 = place[v] + (one ? 0u : rec - first_rec[v]);
+        };
+        if (has_a) target(S[6], S[8], ta, ga);
+        if (ii) target(S[7], S[9], tb, gb);
         // a value nobody reads has sensitivity zero, the field one
         n = S[11];
         src = n ? nv2 + S[10] : (used[S[4]] || S[4] == nv - 1u ? S[4] : zero);
-        if (S[6] != TSI_NONE) ga = place[S[6]] + (S[8] != TSI_NONE ? S[8] - first_rec[S[6]] : 0u);
-        if (S[7] != TSI_NONE) gb = place[S[7]] + (S[9] != TSI_NONE ? S[9] - first_rec[S[7]] : 0u);
         if (src != zero) gs = place[S[4]];
         gather = gather || n != 0u;
       }
-      push4(out.rev, c | (h << 8), x, y, w);
-      push4(targets, ta, tb, src, n);
-      if (small) push4(out.rev16, x | (gs << 16), ga | (gb << 16), ii ? y : w, c | (h << 8) | (n << 16));
+      put(r, c | (h << 8), x, y, w);
+      put(t, ta, tb, src, n);
+      if (r16) put(r16, x | (gs << 16), ga | (gb << 16), ii ? y : w, c | (h << 8) | (n << 16));
     }
-    return kind | (reverse && gather ? WK_GATHER : 0u);
+    return kind | (gather ? WK_GATHER : 0u);
   };
   for (uint32_t dir = 0; dir < 2u; ++dir) {
     const bool reverse = dir == 1u;
