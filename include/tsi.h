@@ -297,12 +297,12 @@ TSI_API tsi_status tsi_scene_trace_wait(tsi_scene *scene);
  * wide threshold are evaluated one cell per 256-thread block from the
  * tape's bundled SSA form; shorter ones one warp per 8-cell group.  To
  * nearest, the threshold is multiplied on levels that have more such cells
- * than the GPU has room for blocks, by how many times more, as long as the
- * warps' own scratch holds their operand logs.  Results
- * are identical for every threshold; only the speed changes.  Tapes shorter
- * than 256 instructions, or whose wide working set would exceed 8 MiB per
- * cell, have no bundled form: they report UINT32_MAX (narrow only) and
- * ignore a new value. */
+ * (of all scenes that run together) than the GPU has room for blocks, by how
+ * many times more, as long as the warps' own scratch holds their operand
+ * logs.  Results are identical for every threshold; only the speed changes.
+ * Tapes shorter than 256 instructions, or whose wide working set would exceed
+ * 8 MiB per cell, have no bundled form: they report UINT32_MAX (narrow only)
+ * and ignore a new value. */
 TSI_API uint32_t tsi_tape_wide_threshold(const tsi_tape *tape);
 TSI_API tsi_status tsi_tape_set_wide_threshold(tsi_tape *tape, uint32_t min_len);
 // A second wide threshold for children at octree level `level` or deeper
@@ -533,14 +533,16 @@ TSI_API void tsi_server_destroy(tsi_server *s);
  * routine: its scratch is a static device array of TSI_STATIC_SCRATCH_BYTES
  * per device (held by every GPU that loads the library until the process
  * exits), and n x (8 x registers + 16 x tape length) bytes must fit in it,
- * else TSI_ERR_BUFFER_TOO_SMALL (split the call).  Nothing in the array needs
- * to start at zero: each launch writes every log entry before reading it.  The first call on a device looks up the array's device
- * address (cudaGetSymbolAddress) and loads the evaluation kernels, so make it
- * before any stream capture.  The call makes the tape's device current and
- * puts the caller's current device back before it returns.  All calls share
- * the one array per device: calls that can overlap on the GPU (different
- * streams, or different contexts on the same device) race on it and must be
- * ordered by the caller. */
+ * else TSI_ERR_BUFFER_TOO_SMALL (split the call).  (The kernels keep the
+ * registers in shared memory; the limit counts them all the same, so that a
+ * call fits or not as it always did.)  Nothing in the array needs to start at
+ * zero: what a launch reads of it, it wrote before.  The first call on a
+ * device looks up the array's device address (cudaGetSymbolAddress) and loads
+ * the evaluation kernels, so make it before any stream capture.  The call
+ * makes the tape's device current and puts the caller's current device back
+ * before it returns.  All calls share the one array per device: calls that
+ * can overlap on the GPU (different streams, or different contexts on the
+ * same device) race on it and must be ordered by the caller. */
 #define TSI_STATIC_SCRATCH_BYTES (16u << 20)
 TSI_API tsi_status tsi_tape_eval_boxes_static(const tsi_tape *tape, uint32_t n, const float *boxes_dev,
                                               int32_t rounding_mode, int32_t reverse, float *out_dev,

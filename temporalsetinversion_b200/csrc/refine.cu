@@ -74,7 +74,9 @@ __device__ __forceinline__ uint32_t copy_word(uint32_t w, bool of_a, uint32_t d,
 // (decision, operand and destination masks); what is left of the serial scan
 // is three logic operations an instruction on the 64-bit mask of live
 // registers, on masks read back by broadcast loads.  (One lane decoding and
-// scanning took 300 cycles an instruction, this takes 35.)
+// scanning took 300 cycles an instruction.  By the level counters the scans of
+// the 64 and 256-primitive animations take 60 cycles per instruction of their
+// items' forward passes, which take 320 to 340.)
 template <bool D>
 __device__ __forceinline__ uint32_t prune_group(const uint2 *__restrict__ code, uint32_t len_, uint32_t n_minmax_,
                                                 uint32_t out_reg, const uint2 *dg, uint32_t g, uint32_t E, uint2 *tmp,

@@ -78,7 +78,12 @@ struct WideTapeDev {
   // of rev16: the sensitivities' slots, the arguments' (first) ones, the field's
   uint32_t gslots = 0, g_arg[4] = {0, 0, 0, 0}, g_field = 0;
 };
-// Tapes of at least this many values get fwd_slots.
+// Tapes of at least this many values get fwd_slots: with 17 bytes a value and
+// what its decisions take, cells of some 6500 values and more leave the 111 KB
+// that a cell has in shared memory with two blocks an SM, and shorter tapes
+// would carry the slots, a fifth more bytes, for nothing.  Where a
+// smaller budget or wider register files send a shorter tape's cells to the
+// global scratch, they take the form that reads its operands there.
 constexpr uint32_t kForwardSlotsMin = 6144;
 void decode_wide(const WideTape &wt, const PackedTape &pt, WideTapeDev &out);
 }  // namespace tsi
