@@ -168,3 +168,30 @@ def test_walk_at_the_limits_of_ordinary_rays_and_boxes(device, lo, extent):
             eq = g[k].view(np.uint32) == o[k].view(np.uint32)
             assert eq[hit].all() if bare and k == "rgba" else eq.all(), (k, eye)
     assert hits >= 10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("localsubdiv,reaches", [(14, True), (15, False)])
+def test_a_ray_of_five_thousand_nodes(device, localsubdiv, reaches):
+    """A ray along a sheet thinner than a leaf, between 2048 leaves and twice as
+    many, to a ball at its end: the walk stops after 5000 nodes (visits of a
+    node and returns to its parent), there as in the oracle."""
+    b = scenes.IRBuilder()
+    sheet = b.sub(b.abs(b.sub(b.Z, 0.5003)), 1e-5)
+    strip = b.sub(b.abs(b.sub(b.X, b.Y)), 0.001)
+    d = [b.sub(b.X, 0.97), b.sub(b.Y, 0.97), b.sub(b.Z, 0.5)]
+    s = b.add(b.add(b.mul(d[0], d[0]), b.mul(d[1], d[1])), b.mul(d[2], d[2]))
+    f = b.min(b.max(sheet, strip), b.sub(b.sqrt(s), 0.05))
+    tape = api.IR.new(b.text(f)).gpu_instructions
+    p = api.default_params(localsubdiv=localsubdiv, root_lo=(0.0, 0.0, 0.0), root_hi=(1.0, 1.0, 1.0))
+    gs, os_ = Scene(device, Tape.upload(device, tape), p), oracle.Scene(tape, p)
+    gs.invert(0.0)
+    os_.invert(0.0)
+    view = scenes.camera_look_at((-0.1, -0.1003, 0.5003), (0.97, 0.97, 0.50035))
+    for res in ((1, 1), (5, 5)):
+        u = api.make_uniforms(view, res, 0.0)
+        g, o = gs.trace(u), os_.trace(u)
+        for k in ("depth", "normal", "rgba"):
+            assert np.array_equal(g[k].view(np.uint32), o[k].view(np.uint32)), (k, res)
+        if res == (1, 1):
+            assert (float(o["depth"][0, 0]) >= 0) == reaches and o["visits"] > 3500
